@@ -24,6 +24,7 @@
 #include "kma_structs.h"
 #include "kma_structs.cuh"
 #include "kma_backend.cuh"
+#include "kma_tree_check.cuh"
 
 #define GR_LINK_REQ 16u /* the reference's clGraph_link size */
 
@@ -192,34 +193,6 @@ __global__ void k_gr_export(gr_dev<B> g, uint64_t nodes, uint32_t *keys, long lo
 	offs[i] = gr_block_off(g.h, nd);
 }
 
-/* in-order walk with an explicit stack: strictly increasing keys? */
-__global__ void k_gr_sorted(const kma_cltree *t, unsigned long long *stack, uint64_t cap, unsigned long long *out)
-{
-	uint64_t sp = 0, count = 0;
-	long long prev = -1;
-	uint32_t sorted = 1;
-	unsigned long long cur = t->root;
-	while (cur || sp) {
-		while (cur) {
-			if (sp >= cap) {
-				out[0] = 2; /* deeper than the stack: not checked */
-				return;
-			}
-			stack[sp++] = cur;
-			cur = ((const kma_cltree_node *)cur)->left;
-		}
-		cur = stack[--sp];
-		const kma_cltree_node *nd = (const kma_cltree_node *)cur;
-		if ((long long)nd->key <= prev)
-			sorted = 0;
-		prev = nd->key;
-		count++;
-		cur = nd->right;
-	}
-	out[0] = sorted;
-	out[1] = count;
-}
-
 /* teardown: every node frees its links, then itself */
 template <class B>
 __global__ void k_gr_free(gr_dev<B> g, uint64_t nodes)
@@ -260,9 +233,13 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	uint64_t cap = 2 * n;
 	void *mem = NULL;
 	size_t o_tree = 0, o_reg = 256, o_nreg = o_reg + cap * 8, o_acc = o_nreg + 8, o_err = o_acc + 16,
-	       o_sums = (o_err + 8 + 255) & ~(size_t)255, o_cnt = o_sums + 64, o_start = o_cnt + cap * 8,
+	       o_sums = (o_err + 8 + 255) & ~(size_t)255, o_tc = o_sums + 64, o_cnt = o_tc + 128, o_start = o_cnt + cap * 8,
 	       o_sinks = o_start + (cap + 1) * 8, o_keys = o_sinks + n * 4, o_offs = (o_keys + cap * 4 + 7) & ~(size_t)7,
-	       o_edges = o_offs + cap * 8, o_stack = o_edges + n * 8, total = o_stack + (size_t)(1 << 20) * 8;
+	       o_edges = o_offs + cap * 8, total = o_edges + n * 8;
+	/* the tree check's work list (16 bytes a node, at most cap nodes) lies over
+	 * the export arrays, which are written after it (44 n + 8 bytes, of which
+	 * it needs 16 cap = 32 n behind a 16-byte boundary) */
+	const size_t o_list = (o_start + 15) & ~(size_t)15;
 	if (cudaMalloc(&mem, total) != cudaSuccess) {
 		cudaGetLastError();
 		return KMA_ENOMEM;
@@ -302,17 +279,22 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	if (rc == KMA_OK && nodes) {
 		unsigned long long *cnt = (unsigned long long *)(m + o_cnt);
 		k_gr_walk<B><<<gb, 256>>>(g, nodes, keys_out ? cnt : NULL, NULL, NULL, sums);
-		k_gr_sorted<<<1, 1>>>(g.tree, (unsigned long long *)(m + o_stack), 1 << 20, sums + 4);
-		if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+		if (cudaGetLastError() != cudaSuccess)
 			rc = KMA_ECUDA;
-		unsigned long long sm[6];
-		if (rc == KMA_OK && cudaMemcpy(sm, sums, sizeof(sm), cudaMemcpyDeviceToHost) != cudaSuccess)
+		unsigned long long *tc = (unsigned long long *)(m + o_tc);
+		if (rc == KMA_OK)
+			rc = tree_check(g.tree, m + o_list, nodes, tc, device, NULL);
+		if (rc == KMA_OK && cudaDeviceSynchronize() != cudaSuccess)
+			rc = KMA_ECUDA;
+		unsigned long long sm[3], tcw[KMA_TC_WORDS];
+		if (rc == KMA_OK && (cudaMemcpy(sm, sums, sizeof(sm), cudaMemcpyDeviceToHost) != cudaSuccess ||
+				     cudaMemcpy(tcw, tc, sizeof(tcw), cudaMemcpyDeviceToHost) != cudaSuccess))
 			rc = KMA_ECUDA;
 		if (rc == KMA_OK) {
 			st->links = sm[0];
 			st->edge_xor = sm[1];
 			st->edge_sum = sm[2];
-			st->sorted = (uint32_t)sm[4];
+			st->sorted = tcw[KMA_TC_UNSORTED] == 0 && tcw[KMA_TC_OVERFLOW] == 0;
 		}
 		if (rc == KMA_OK && keys_out) {
 			/* export: nodes in key order, links in queue order */

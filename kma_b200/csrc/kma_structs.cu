@@ -14,6 +14,7 @@
 #include "kma_structs.h"
 #include "kma_structs.cuh"
 #include "kma_backend.cuh"
+#include "kma_tree_check.cuh"
 
 struct kma_clqueue_s {
 	int device;
@@ -746,8 +747,9 @@ extern "C" int kma_cltree_destroy(kma_cltree_t t)
 extern "C" struct kma_cltree *kma_cltree_device_ptr(kma_cltree_t t) { return t ? t->dt : NULL; }
 
 namespace {
-/* In-order walk of the live keys with an explicit stack of `cap` entries;
- * writes up to cap keys (when keys != NULL) and the summary. */
+/* In-order walk of the live keys with an explicit stack of `cap` entries,
+ * for the replay, which lists the keys: writes up to cap of them and the
+ * summary. */
 __global__ void k_tree_walk(const kma_cltree *t, unsigned long long *stack, uint64_t cap, uint32_t *keys,
 		unsigned long long *summary /* count, xor, sum, sorted, overflow */)
 {
@@ -775,7 +777,7 @@ __global__ void k_tree_walk(const kma_cltree *t, unsigned long long *stack, uint
 			if ((long long)nd->key <= prev)
 				sorted = 0;
 			prev = nd->key;
-			if (keys && count < cap)
+			if (count < cap)
 				keys[count] = nd->key;
 			count++;
 			x ^= nd->key;
@@ -1467,9 +1469,9 @@ extern "C" int kma_c3_tree_run(const uint8_t *kinds, const uint32_t *keys, uint6
 		uint32_t *dord = b.alloc<uint32_t>(n_ops * 4);
 		uint64_t *doffs = b.alloc<uint64_t>(((size_t)threads + 1) * 8);
 		int8_t *dres = b.alloc<int8_t>(n_ops);
-		unsigned long long *stack = b.alloc<unsigned long long>(n_ops * 8);
-		unsigned long long *summ = b.alloc<unsigned long long>(5 * 8);
-		if (!pool || !dk || !dkeys || !dord || !doffs || !dres || !stack || !summ)
+		ulonglong2 *list = b.alloc<ulonglong2>(n_ops * sizeof(ulonglong2));
+		unsigned long long *summ = b.alloc<unsigned long long>(KMA_TC_WORDS * 8);
+		if (!pool || !dk || !dkeys || !dord || !doffs || !dres || !list || !summ)
 			rc = KMA_ENOMEM;
 		if (rc == KMA_OK &&
 		    (cudaMemcpy(dk, kinds, n_ops, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -1484,23 +1486,26 @@ extern "C" int kma_c3_tree_run(const uint8_t *kinds, const uint32_t *keys, uint6
 			cudaEventRecord(e0);
 			k_c3_tree<<<(threads + 255) / 256, 256>>>(t->dt, pool, dk, dkeys, dord, doffs, threads, dres);
 			cudaEventRecord(e1);
-			k_tree_walk<<<1, 1>>>(t->dt, stack, n_ops, NULL, summ);
-			if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+			if (cudaGetLastError() != cudaSuccess)
+				rc = KMA_ECUDA;
+			if (rc == KMA_OK)
+				rc = tree_check(t->dt, list, n_ops, summ, t->device, NULL);
+			if (rc == KMA_OK && cudaDeviceSynchronize() != cudaSuccess)
 				rc = KMA_ECUDA;
 			cudaEventElapsedTime(&st->ms, e0, e1);
 			cudaEventDestroy(e0);
 			cudaEventDestroy(e1);
 		}
-		unsigned long long s[5];
+		unsigned long long s[KMA_TC_WORDS];
 		if (rc == KMA_OK && (cudaMemcpy(s, summ, sizeof(s), cudaMemcpyDeviceToHost) != cudaSuccess ||
 				     cudaMemcpy(results, dres, n_ops, cudaMemcpyDeviceToHost) != cudaSuccess))
 			rc = KMA_ECUDA;
 		if (rc == KMA_OK) {
-			st->live_keys = s[0];
-			st->keys_xor = s[1];
-			st->keys_sum = s[2];
-			st->sorted = (uint32_t)s[3];
-			st->err = s[4] ? 1u : 0u;
+			st->live_keys = s[KMA_TC_LIVE];
+			st->keys_xor = s[KMA_TC_XOR];
+			st->keys_sum = s[KMA_TC_SUM];
+			st->sorted = s[KMA_TC_UNSORTED] == 0;
+			st->err = s[KMA_TC_OVERFLOW] ? 1u : 0u;
 		}
 	}
 	kma_cltree_destroy(t);

@@ -330,3 +330,46 @@ def test_gpu_c3_tree_equals_sequential_replay():
     for k in mkeys:
         x ^= int(k)
     assert st["keys_xor"] == x
+
+
+def _balanced(lo, hi):
+    """Keys lo..hi in the level order of a balanced tree: inserted so, each level is full."""
+    out, level = [], [(lo, hi)]
+    while level:
+        nxt = []
+        for a, b in level:
+            if a <= b:
+                m = (a + b) // 2
+                out.append(m)
+                nxt += [(a, m - 1), (m + 1, b)]
+        level = nxt
+    return out
+
+
+TREE_SHAPES = {
+    "empty": [],
+    "one": [0],
+    "up": [*range(700), 0xFFFFFFFF],
+    "down": [*range(0xFFFFFFFF, 0xFFFFFFFF - 700, -1), 0],
+    "levels_to_512": _balanced(1, 1023),   # the widest level one block takes
+    "levels_to_1024": _balanced(1, 2047),  # one that all blocks share
+    # wide levels, then a chain below the last key, then nothing wide again
+    "wide_then_chain": _balanced(1, 5000) + [*range(5001, 5600)],
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", TREE_SHAPES)
+def test_gpu_tree_check_over_shapes(shape):
+    """The check of the whole tree counts every live key once, whatever the
+    widths of the levels (one thread inserts, so the order sets the shape)."""
+    from kma_b200 import structs
+    ins = TREE_SHAPES[shape]
+    gone = ins[::3]
+    kinds = np.array([0] * len(ins) + [2] * len(gone) + [1], np.uint8)
+    keys = np.array(ins + gone + [3], np.uint32)
+    _, st = structs.c3_tree(kinds, keys, threads=1)
+    want = np.array(sorted(set(ins) - set(gone)), np.uint64)
+    assert (st["sorted"], st["err"], st["live_keys"]) == (1, 0, len(want))
+    assert st["keys_sum"] == int(want.sum())
+    assert st["keys_xor"] == int(np.bitwise_xor.reduce(want)) if len(want) else st["keys_xor"] == 0
