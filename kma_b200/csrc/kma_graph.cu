@@ -6,8 +6,8 @@
  * endpoints (tree get; else malloc a node, init its links queue, tree add;
  * free the node again when another thread added the key first) and
  * enqueue a freshly malloc'd link on the source's queue.  Every inserted
- * node is also recorded in a registry array, so the walk and the teardown
- * run one thread per node.
+ * node and every link is also recorded in a registry array: the teardown
+ * frees them from there, and the walk starts in the middle of long queues.
  *
  * Every kernel is a template on the heap backend (kma_backend.cuh), as the
  * reference's driver builds the same tb_clTree.cl over kma.cl or pma.cl
@@ -68,6 +68,7 @@ struct gr_dev {
 	typename B::heap *h;
 	kma_cltree *tree;
 	gr_node **reg;               /* [cap] inserted nodes */
+	unsigned long long *link;    /* [n] edge i's link item, 0 when it has none */
 	unsigned long long *nreg;
 	unsigned long long *acc;     /* lost_adds, nulls */
 	uint32_t *qerr;
@@ -113,14 +114,14 @@ __global__ void k_gr_build(gr_dev<B> g, const uint32_t *edges, uint64_t n)
 	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
 		gr_node *src = gr_ensure(g, edges[2 * i], lost, nulls);
 		gr_node *snk = gr_ensure(g, edges[2 * i + 1], lost, nulls);
-		if (!src || !snk)
-			continue;
-		void *b = B::alloc(g.h, GR_LINK_REQ);
+		void *b = src && snk ? B::alloc(g.h, GR_LINK_REQ) : nullptr;
 		if (!b) {
-			nulls++;
+			nulls += src && snk;
+			g.link[i] = 0;
 			continue;
 		}
 		unsigned char *item = reinterpret_cast<unsigned char *>(((uintptr_t)b + 7) & ~(uintptr_t)7);
+		g.link[i] = (unsigned long long)item;
 		*reinterpret_cast<uint32_t *>(item + 8) = (uint32_t)(((unsigned char *)snk - B::base(g.h)) >> 3);
 		__threadfence();
 		kma_clqueue_enqueue(&src->links, reinterpret_cast<kma_clqueue_item *>(item), g.qerr);
@@ -131,44 +132,212 @@ __global__ void k_gr_build(gr_dev<B> g, const uint32_t *edges, uint64_t n)
 		atomicAdd(&g.acc[1], nulls);
 }
 
-template <class B>
-__device__ __forceinline__ uint32_t gr_sink_key(const gr_dev<B> &g, const kma_clqueue_item *it)
+/*
+ * The walk of every node's queue.  A queue is a linked list, one dependent
+ * load per link, and with skewed edges one queue holds a large share of all
+ * links: one thread per node took 30 ms for 2^20 Zipf(1.1) edges, all but a
+ * little of it on the hottest node.  So the lists are cut (Helman and JaJa's
+ * list ranking): every link whose address hashes to 0 mod `spacing` starts a
+ * segment, and its thread walks to the next such link or the queue's end;
+ * then a node's thread walks to its first segment and goes on from segment to
+ * segment.  Both parts are chains of dependent loads, the first of about
+ * spacing * ln(segments) links, the second of (links / spacing) segments, and
+ * spacing = sqrt(n) / 8 keeps both below a millisecond (1.4 ms in all where
+ * it took 30; spacing 128).
+ *
+ * While the walk runs, a segment's first link holds the segment's number in
+ * place of its sink, which the segment keeps.
+ */
+struct gr_seg {
+	unsigned long long item; /* its first link */
+	uint32_t sink8;          /* that link's sink, as a link holds it */
+	uint32_t key;            /* the source of that link's edge */
+	uint32_t len, next;      /* links; the segment behind it, or GR_NO_SEG */
+	unsigned long long x, s; /* edge hashes */
+	unsigned long long pos;  /* where its sinks go, or ~0 when no queue leads to it */
+};
+#define GR_NO_SEG 0xffffffffu
+
+struct gr_cut {
+	gr_seg *seg;
+	unsigned int *nseg; /* may count past cap: the links past it stay ordinary */
+	uint32_t cap, mask; /* mask: spacing - 1 */
+	uint32_t n;         /* no queue is longer */
+};
+
+__device__ __forceinline__ uint32_t *gr_sink_word(unsigned long long item)
 {
-	uint32_t off8 = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const unsigned char *>(it) + 8);
-	const gr_node *s = reinterpret_cast<const gr_node *>(B::base(g.h) + ((size_t)off8 << 3));
-	return s->tree.key;
+	return reinterpret_cast<uint32_t *>(item + 8);
 }
 
-/* per node: links in queue order -> count, edge hashes; optionally the
- * sinks at out[start[i] ...] */
-template <class B>
-__global__ void k_gr_walk(gr_dev<B> g, uint64_t nodes, unsigned long long *counts, const uint64_t *start,
-		uint32_t *sinks, unsigned long long *sums /* links, xor, sum */)
+__device__ __forceinline__ bool gr_hits(const gr_cut &c, unsigned long long item)
 {
-	uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	unsigned long long c = 0, x = 0, s = 0;
-	if (i < nodes) {
-		const gr_node *nd = g.reg[i];
-		uint32_t key = nd->tree.key;
-		for (const kma_clqueue_item *it = kma_clqueue_first(&nd->links); it && c < (1ull << 31);
-		     it = kma_clqueue_next(it)) {
-			uint32_t sk = gr_sink_key(g, it);
-			if (sinks)
-				sinks[start[i] + c] = sk;
-			uint64_t m = gr_mix(key, sk);
+	return ((uint32_t)((item >> 3) * 0x9E3779B97F4A7C15ull >> 32) & c.mask) == 0;
+}
+
+/* The segment that starts at `item` (whose sink word is w), or GR_NO_SEG.
+ * Only the segment's own record decides: w is a sink, and may be any number,
+ * in a link that hits but found the records full. */
+__device__ __forceinline__ uint32_t gr_seg_at(const gr_cut &c, uint32_t nseg, unsigned long long item, uint32_t w)
+{
+	return gr_hits(c, item) && w < nseg && c.seg[w].item == item ? w : GR_NO_SEG;
+}
+__device__ __forceinline__ uint32_t gr_nseg(const gr_cut &c)
+{
+	const uint32_t m = *c.nseg;
+	return m < c.cap ? m : c.cap;
+}
+
+template <class B>
+__global__ void k_gr_cut(gr_dev<B> g, const uint32_t *edges, uint64_t n, gr_cut c)
+{
+	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+		const unsigned long long item = g.link[i];
+		if (!item || !gr_hits(c, item))
+			continue;
+		const uint32_t s = atomicAdd(c.nseg, 1u);
+		if (s >= c.cap)
+			continue;
+		gr_seg &r = c.seg[s];
+		r.item = item;
+		r.sink8 = *gr_sink_word(item);
+		r.key = edges[2 * i];
+		r.pos = ~0ull;
+		*gr_sink_word(item) = s;
+	}
+}
+
+/* Put the sinks back into the segments' first links. */
+__global__ void k_gr_uncut(gr_cut c)
+{
+	const uint32_t nseg = gr_nseg(c), stride = gridDim.x * blockDim.x;
+	for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += stride)
+		*gr_sink_word(c.seg[s].item) = c.seg[s].sink8;
+}
+
+template <class B>
+__device__ __forceinline__ uint32_t gr_key_at(const gr_dev<B> &g, uint32_t off8)
+{
+	return reinterpret_cast<const gr_node *>(B::base(g.h) + ((size_t)off8 << 3))->tree.key;
+}
+
+/* Walk from `item` (0: nothing) to the next segment or the end of the queue;
+ * first: item's own sink, when item starts a segment.  Visits the sink keys
+ * in order; returns how many, *next: the segment it ended at.  A sink's key
+ * is handed on one step late, so that its load runs beside the next link's. */
+template <class B, class F>
+__device__ __forceinline__ uint32_t gr_run(const gr_dev<B> &g, const gr_cut &c, uint32_t nseg, unsigned long long item,
+		bool starts, uint32_t first, uint32_t *next, F visit)
+{
+	uint32_t len = 0, key = 0;
+	*next = GR_NO_SEG;
+	while (item && len < c.n) {
+		uint32_t w = *gr_sink_word(item);
+		const unsigned long long after = kma_detail::clq_next<kma_detail::clq_link_head>(item);
+		if (starts && len == 0) {
+			w = first;
+		} else {
+			const uint32_t s = gr_seg_at(c, nseg, item, w);
+			if (s != GR_NO_SEG) {
+				*next = s;
+				break;
+			}
+		}
+		const uint32_t k = gr_key_at(g, w);
+		if (len)
+			visit(len - 1, key);
+		key = k;
+		len++;
+		item = after;
+	}
+	if (len)
+		visit(len - 1, key);
+	return len;
+}
+
+/* every segment's length and edge hashes */
+template <class B>
+__global__ void k_gr_walk_segs(gr_dev<B> g, gr_cut c)
+{
+	const uint32_t nseg = gr_nseg(c), stride = gridDim.x * blockDim.x;
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += stride) {
+		gr_seg &r = c.seg[i];
+		unsigned long long x = 0, s = 0;
+		const uint32_t key = r.key;
+		uint32_t next;
+		const uint32_t len = gr_run(g, c, nseg, r.item, true, r.sink8, &next, [&](uint32_t, uint32_t sk) {
+			const uint64_t m = gr_mix(key, sk);
 			x ^= m;
 			s += m;
-			c++;
+		});
+		r.len = len;
+		r.next = next;
+		r.x = x;
+		r.s = s;
+	}
+}
+
+/* per node: its links in queue order -> count and edge hashes.  start: the
+ * node's place among the sinks (second pass of an export), which also goes
+ * to its segments. */
+template <class B>
+__global__ void k_gr_walk(gr_dev<B> g, uint64_t nodes, gr_cut c, unsigned long long *counts, const uint64_t *start,
+		unsigned long long *sums /* links, xor, sum */)
+{
+	const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	unsigned long long n = 0, x = 0, s = 0;
+	if (i < nodes) {
+		const gr_node *nd = g.reg[i];
+		const uint32_t key = nd->tree.key, nseg = gr_nseg(c);
+		uint32_t next;
+		n = gr_run(g, c, nseg, (unsigned long long)kma_clqueue_first(&nd->links), false, 0, &next,
+			   [&](uint32_t, uint32_t sk) {
+				   const uint64_t m = gr_mix(key, sk);
+				   x ^= m;
+				   s += m;
+			   });
+		/* a segment of another source's edges is a link on the wrong queue:
+		 * it is not counted, nor is anything behind it */
+		for (uint32_t hops = 0; next != GR_NO_SEG && hops <= nseg && c.seg[next].key == key; hops++) {
+			gr_seg &r = c.seg[next];
+			if (start)
+				r.pos = start[i] + n;
+			n += r.len;
+			x ^= r.x;
+			s += r.s;
+			next = r.next;
 		}
 		if (counts)
-			counts[i] = c;
+			counts[i] = n;
 	}
-	if (c)
-		atomicAdd(&sums[0], c);
+	if (start)
+		return;
+	if (n)
+		atomicAdd(&sums[0], n);
 	if (x)
 		atomicXor(&sums[1], x);
 	if (s)
 		atomicAdd(&sums[2], s);
+}
+
+/* every node's sinks, in queue order: from its head to its first segment,
+ * and every segment at its place */
+template <class B>
+__global__ void k_gr_sinks(gr_dev<B> g, uint64_t nodes, gr_cut c, const uint64_t *start, uint32_t *sinks)
+{
+	const uint32_t nseg = gr_nseg(c);
+	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nodes + nseg; i += stride) {
+		const bool seg = i >= nodes;
+		const gr_seg *r = &c.seg[seg ? i - nodes : 0];
+		const unsigned long long pos = seg ? r->pos : start[i];
+		if (pos == ~0ull)
+			continue;
+		uint32_t next;
+		gr_run(g, c, nseg, seg ? r->item : (unsigned long long)kma_clqueue_first(&g.reg[i]->links), seg,
+		       seg ? r->sink8 : 0u, &next, [&](uint32_t k, uint32_t sk) { sinks[pos + k] = sk; });
+	}
 }
 
 /* offset of the block that holds node nd (PMA: of the node itself, its
@@ -193,21 +362,17 @@ __global__ void k_gr_export(gr_dev<B> g, uint64_t nodes, uint32_t *keys, long lo
 	offs[i] = gr_block_off(g.h, nd);
 }
 
-/* teardown: every node frees its links, then itself */
+/* teardown: every link and every node is freed, from the registries: the
+ * hottest queue emptied by its node's thread, one dequeue after the other,
+ * took 480 ms of a 2^20-edge Zipf(1.1) graph.  Neighbouring edges' links come
+ * from the same superblocks, so the warp form frees a warp's with a few
+ * atomics: 0.05 ms. */
 template <class B>
-__global__ void k_gr_free(gr_dev<B> g, uint64_t nodes)
+__global__ void k_gr_free(gr_dev<B> g, uint64_t nodes, uint64_t n)
 {
-	uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= nodes)
-		return;
-	gr_node *nd = g.reg[i];
-	for (;;) {
-		kma_clqueue_item *it = kma_clqueue_dequeue(&nd->links, g.qerr);
-		if (!it)
-			break;
-		B::release(g.h, it);
-	}
-	B::release(g.h, nd);
+	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n + nodes; i += stride)
+		B::release_warp(g.h, i < n ? reinterpret_cast<void *>(g.link[i]) : g.reg[i - n]);
 }
 
 } /* namespace */
@@ -232,10 +397,17 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	memset(st, 0, sizeof(*st));
 	uint64_t cap = 2 * n;
 	void *mem = NULL;
+	/* segments of the walk: a power of two near sqrt(n) / 8 apart, the records
+	 * for twice as many as the hash should give */
+	uint32_t spacing = 1;
+	while ((uint64_t)spacing * spacing * 128 < n)
+		spacing *= 2;
+	const uint32_t segs = (uint32_t)(2 * n / spacing) + 1024;
 	size_t o_tree = 0, o_reg = 256, o_nreg = o_reg + cap * 8, o_acc = o_nreg + 8, o_err = o_acc + 16,
-	       o_sums = (o_err + 8 + 255) & ~(size_t)255, o_tc = o_sums + 64, o_cnt = o_tc + 128, o_start = o_cnt + cap * 8,
+	       o_sums = (o_err + 8 + 255) & ~(size_t)255, o_nseg = o_sums + 24, o_tc = o_sums + 64, o_cnt = o_tc + 128, o_start = o_cnt + cap * 8,
 	       o_sinks = o_start + (cap + 1) * 8, o_keys = o_sinks + n * 4, o_offs = (o_keys + cap * 4 + 7) & ~(size_t)7,
-	       o_edges = o_offs + cap * 8, total = o_edges + n * 8;
+	       o_edges = o_offs + cap * 8, o_link = o_edges + n * 8, o_seg = o_link + n * 8,
+	       total = o_seg + (size_t)segs * sizeof(gr_seg);
 	/* the tree check's work list (16 bytes a node, at most cap nodes) lies over
 	 * the export arrays, which are written after it (44 n + 8 bytes, of which
 	 * it needs 16 cap = 32 n behind a 16-byte boundary) */
@@ -250,10 +422,12 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	g.h = dh;
 	g.tree = (kma_cltree *)(m + o_tree);
 	g.reg = (gr_node **)(m + o_reg);
+	g.link = (unsigned long long *)(m + o_link);
 	g.nreg = (unsigned long long *)(m + o_nreg);
 	g.acc = (unsigned long long *)(m + o_acc);
 	g.qerr = (uint32_t *)(m + o_err);
 	unsigned long long *sums = (unsigned long long *)(m + o_sums);
+	const gr_cut cut = {(gr_seg *)(m + o_seg), (unsigned int *)(m + o_nseg), segs, spacing - 1, (uint32_t)n};
 	if (cudaMemset(m, 0, o_reg) != cudaSuccess || cudaMemset(m + o_nreg, 0, o_cnt - o_nreg) != cudaSuccess ||
 	    cudaMemcpy(m + o_edges, edges, n * 8, cudaMemcpyHostToDevice) != cudaSuccess)
 		rc = KMA_ECUDA;
@@ -276,9 +450,15 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 			     cudaMemcpy(acc, g.acc, 16, cudaMemcpyDeviceToHost) != cudaSuccess))
 		rc = KMA_ECUDA;
 	uint32_t gb = (uint32_t)((nodes + 255) / 256);
+	/* grids of the kernels that stride over the edges, or over the segments */
+	const uint64_t most = 148 * 8;
+	const uint32_t eb = (uint32_t)std::min<uint64_t>((n + nodes + 255) / 256, most);
+	const uint32_t sb = (uint32_t)std::min<uint64_t>((segs + 255) / 256, most);
 	if (rc == KMA_OK && nodes) {
 		unsigned long long *cnt = (unsigned long long *)(m + o_cnt);
-		k_gr_walk<B><<<gb, 256>>>(g, nodes, keys_out ? cnt : NULL, NULL, NULL, sums);
+		k_gr_cut<B><<<eb, 256>>>(g, (const uint32_t *)(m + o_edges), n, cut);
+		k_gr_walk_segs<B><<<sb, 256>>>(g, cut);
+		k_gr_walk<B><<<gb, 256>>>(g, nodes, cut, keys_out ? cnt : NULL, NULL, sums);
 		if (cudaGetLastError() != cudaSuccess)
 			rc = KMA_ECUDA;
 		unsigned long long *tc = (unsigned long long *)(m + o_tc);
@@ -313,9 +493,9 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 			if (rc == KMA_OK && start[nodes] <= n) {
 				if (cudaMemcpy(m + o_start, start.data(), (nodes + 1) * 8, cudaMemcpyHostToDevice) != cudaSuccess)
 					rc = KMA_ECUDA;
-				cudaMemset(sums, 0, 24);
-				k_gr_walk<B><<<gb, 256>>>(g, nodes, NULL, (const uint64_t *)(m + o_start),
-							 (uint32_t *)(m + o_sinks), sums);
+				const uint64_t *dstart = (const uint64_t *)(m + o_start);
+				k_gr_walk<B><<<gb, 256>>>(g, nodes, cut, NULL, dstart, sums);
+				k_gr_sinks<B><<<eb, 256>>>(g, nodes, cut, dstart, (uint32_t *)(m + o_sinks));
 				std::vector<uint32_t> sk(start[nodes] ? start[nodes] : 1);
 				if (rc == KMA_OK && (cudaDeviceSynchronize() != cudaSuccess ||
 						     cudaMemcpy(sk.data(), m + o_sinks, start[nodes] * 4,
@@ -341,8 +521,14 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 			}
 		}
 	}
+	if (rc == KMA_OK && !free_after && nodes) {
+		/* the graph stays in the heap as it was built */
+		k_gr_uncut<<<sb, 256>>>(cut);
+		if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+			rc = KMA_ECUDA;
+	}
 	if (rc == KMA_OK && free_after && nodes) {
-		k_gr_free<B><<<gb, 256>>>(g, nodes);
+		k_gr_free<B><<<eb, 256>>>(g, nodes, n);
 		if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
 			rc = KMA_ECUDA;
 	}

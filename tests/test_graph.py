@@ -78,3 +78,31 @@ def test_gpu_graph_concurrent_conserves_edges(threads):
         assert st["lost_adds"] > 0  # threads raced to add the same key and the losers freed their node
         assert ins.check_canonical_empty(h.snapshot(), h.bitmaps()) == []
         assert h.error_flags() == 0
+
+
+def _star(n):
+    """n edges, most of them from one vertex: its queue is cut into many segments."""
+    rng = np.random.default_rng(n)
+    src = np.where(rng.random(n) < 0.8, 7, rng.integers(100, 140, n))
+    return np.stack([src, rng.integers(1000, 1100, n)], 1).astype(np.uint32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,threads", [(1, 1), (128, 1), (129, 1), (3000, 1), (2, 2048), (3000, 2048), (40000, 2048)])
+def test_gpu_graph_long_queue(n, threads):
+    """A hot vertex's queue comes out whole and in order: one thread appends
+    in edge order; many threads keep every source's sinks as a multiset."""
+    from kma_b200 import Heap, graph
+    from kma_b200 import inspect as ins
+    e = _star(n)
+    with Heap(2048, 14) as h:
+        st, (keys, _, sinks, start) = graph.build(h, e, threads=threads, export=True)
+        m = edge_mix(e[:, 0], e[:, 1])
+        assert (st["links"], st["err"], st["nulls"], st["sorted"]) == (n, 0, 0, 1)
+        assert st["edge_xor"] == int(np.bitwise_xor.reduce(m)) and st["edge_sum"] == int(m.sum(dtype=np.uint64))
+        np.testing.assert_array_equal(keys, np.unique(e))
+        for i, k in enumerate(keys):
+            got, want = sinks[start[i]:start[i + 1]], e[e[:, 0] == k, 1].astype(np.int64)
+            np.testing.assert_array_equal(*((got, want) if threads == 1 else (np.sort(got), np.sort(want))))
+        assert ins.check_canonical_empty(h.snapshot(), h.bitmaps()) == []
+        assert h.error_flags() == 0
