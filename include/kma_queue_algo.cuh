@@ -356,6 +356,237 @@ KQ_FN uint32_t clq_dequeue_n(u64 *headw, u64 *tailw, u64 *out, uint32_t k, uint3
 }
 
 /* ------------------------------------------------------------------ */
+/* dequeue by a whole warp                                             */
+/* ------------------------------------------------------------------ */
+/*
+ * clq_dequeue_v takes what clq_dequeue_n takes, in the same order and under
+ * the same hold, with the 32 lanes of a warp instead of one thread.  What
+ * bounds a hot queue is the hold, a chain of dependent round trips, so the
+ * point is to have fewer of them:
+ *   - a record's entries are one load per lane, and so are the links that
+ *     prove them, so a chain costs two round trips (its record; its links,
+ *     the last of which says where the next chain's record is) however long
+ *     it is.  A chain's length stands in its record (bits 48.. of entry 0), its
+ *     number's low 14 bits in the link into it; the bits above are those of
+ *     the chain before, or one more or less: chains are appended about in
+ *     the order of their numbers, and a wrong guess fails the check;
+ *   - the hold before leaves a note in the log (`resume`): the record in
+ *     which the new head is.  It is read with the head's link, and the
+ *     record with the recheck of the head, so that neither costs a round
+ *     trip.  The note also finds the place in the middle of a chain, where a
+ *     batch that is no multiple of the chains leaves the head for good: no
+ *     link there is marked, and a walk is one round trip per item;
+ *   - taken items get their POISON after the head is released: nobody else
+ *     writes or reads the link of an item behind a held head that has a
+ *     successor, and the caller has the items only when this returns.
+ * A walk goes on only to the next marked link.  As everywhere, records and
+ * notes are hints, believed only where the queue's links say the same.
+ *
+ * Vector policy `V` (32 lanes; on the host, arrays of 32):
+ *   reg<T>        one T per lane; x[j] is lane j's (on the GPU: the caller's)
+ *   each(f)       f(j) on every lane       one(f)   f() on one lane, its result on all
+ *   ballot(x)     bit j: x[j]              get(x, j)  lane j's x, on all lanes
+ *   above(x)      lane j gets lane j+1's x
+ *   fence()       acquire: what the loads before have seen published is visible
+ * Log policy, besides the above:
+ *   raw(p)        relaxed load of an entry of clq_record with its length bits
+ *   taken_chains(n)        n chains were taken from records (a count)
+ *   resume(item, &recno)   whether there is a note for item
+ *   note(item, recno)      leave one
+ * Output `OUT`: run(at, items, first, n) puts items[first .. first+n) at
+ * at.., one(at, item) puts one; each_taken(r, f) calls f(item) for those at
+ * 1 .. r-1.
+ */
+const uint32_t LOG_LOW_BITS = 14;
+const uint32_t LOG_LOW_MASK = (1u << LOG_LOW_BITS) - 1u;
+const int LOG_LEN_SHIFT = PTR_BITS;
+
+/* the number with the low bits `low` that is nearest to ref (mod 2^24) */
+KQ_FN uint32_t log_near(uint32_t ref, uint32_t low)
+{
+	const uint32_t half = 1u << (LOG_LOW_BITS - 1);
+	const uint32_t up = (low - ref) & LOG_LOW_MASK; /* steps up from ref */
+	return (up < half ? ref + up : ref + up - (LOG_LOW_MASK + 1u)) & LOG_RECNO_MASK;
+}
+
+template <class O, class L, class V, class OUT, class LG>
+KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint32_t limit, bool *timed_out,
+		const LG *log)
+{
+	typedef typename V::template reg<u64> vec;
+	*timed_out = false;
+	uint32_t it = 0, idle = 0;
+	u64 last = ~0ull;
+	for (;;) {
+		const u64 h = V::one([&] { return O::ld_rlx(headw); });
+		if (h != last) {
+			last = h;
+			idle = 0;
+		} else if (++idle >= limit) {
+			break;
+		}
+		const u64 hp = qp_ptr(h);
+		if (hp == 0)
+			return 0;
+		u64 *hl = L::at(hp);
+		uint32_t recno = 0;
+		bool noted = false;
+		const u64 seen = V::one([&] {
+			const u64 l = O::ld_rlx(hl);
+			noted = log && log->resume(hp, &recno);
+			return l;
+		});
+		if (seen == POISON) {
+			O::pause(it++);
+			continue;
+		}
+		const u64 nx = V::one([&] { return O::xchg(hl, POISON); });
+		if (nx == POISON) {
+			O::pause(it++);
+			continue;
+		}
+		noted = V::one([&] { return noted; });
+		recno = V::one([&] { return recno; });
+		/* the record of the note, if there is one, beside the recheck */
+		vec raw;
+		if (noted) {
+			const u64 *rec = log->clq_record(recno);
+			V::each([&](uint32_t j) { raw[j] = LG::raw(rec + j); });
+		}
+		if (V::one([&] { return O::ld(headw); }) != h) {
+			V::one([&] {
+				O::st(hl, nx);
+				return 0u;
+			});
+			O::pause(it++);
+			continue;
+		}
+		/* held: cur is the next item to take, curl its link where known */
+		uint32_t r = 0, chains = 0;
+		u64 cur = hp, curl = nx, untried = ~0ull;
+		bool have = noted, end = nx == 0;
+		while (r < k && !end) {
+			if (have) {
+				const uint32_t len = (uint32_t)(V::get(raw, 0) >> LOG_LEN_SHIFT);
+				vec item, link;
+				typename V::template reg<bool> hit, bad;
+				V::each([&](uint32_t j) {
+					item[j] = qp_ptr(raw[j]);
+					hit[j] = j < len && item[j] == cur;
+				});
+				const uint32_t at = V::ballot(hit);
+				uint32_t p = 0;
+				while (at && !((at >> p) & 1u))
+					p++;
+				const uint32_t n = at ? (len < LOG_CHAIN_MAX ? len : LOG_CHAIN_MAX) - p : 0u;
+				uint32_t m = n < k - r ? n : k - r;
+				/* the links of the items to take; an entry that is no item
+				 * pointer is not followed */
+				V::each([&](uint32_t j) {
+					const bool mine = j >= p && j < p + m;
+					bad[j] = mine && item[j] <= POISON;
+					link[j] = 0;
+					if (mine && !bad[j])
+						link[j] = curl && j == p ? curl : O::ld_rlx(L::at(item[j]));
+				});
+				const vec next = V::above(item);
+				V::each([&](uint32_t j) {
+					if (j >= p && j < p + m)
+						bad[j] = bad[j] || link[j] == POISON ||
+							 (j + 1 < p + n && qp_ptr(link[j]) != next[j]);
+				});
+				if (m && !V::ballot(bad)) {
+					const u64 ll = V::get(link, (p + m - 1u) & 31u);
+					const bool whole = m == n;
+					u64 nh = qp_ptr(ll);
+					if (nh == 0) {
+						/* its last item has no successor yet: it stays, as the head */
+						m--;
+						nh = V::get(item, (p + m) & 31u);
+						end = true;
+					}
+					if (nh != 0 && !(end && !whole)) {
+						out.run(r, item, p, m);
+						r += m;
+						chains += m != 0;
+						cur = nh;
+						curl = 0;
+						if (whole && !end) {
+							have = (ll & CLQ_INTO) && !(ll & CLQ_LOG);
+							recno = log_near(recno, (uint32_t)(ll >> PTR_BITS) & LOG_LOW_MASK);
+							if (have && r < k) {
+								const u64 *rec = log->clq_record(recno);
+								V::each([&](uint32_t j) { raw[j] = LG::raw(rec + j); });
+							}
+						}
+						continue;
+					}
+					end = false;
+				}
+				have = false;
+			}
+			/* no record that fits: one link */
+			if (!curl)
+				curl = V::one([&] { return O::ld(L::at(cur)); });
+			if (curl == 0 || curl == POISON)
+				break; /* cur is the last linked item: it stays, as the head */
+			if ((curl & CLQ_LOG) && log && cur != untried) {
+				untried = cur;
+				const u64 second = qp_ptr(curl);
+				const uint32_t lo = V::one([&] {
+					return (uint32_t)(O::ld_rlx(L::at(second)) >> PTR_BITS) & LOG_LOW_MASK;
+				});
+				recno = (((uint32_t)(curl >> PTR_BITS) & 0x3FFu) << LOG_LOW_BITS) | lo;
+				const u64 *rec = log->clq_record(recno);
+				V::each([&](uint32_t j) { raw[j] = LG::raw(rec + j); });
+				have = true;
+				continue;
+			}
+			out.one(r++, cur);
+			cur = qp_ptr(curl);
+			curl = 0;
+		}
+		if (r) {
+			V::one([&] {
+				if (have)
+					log->note(cur, recno);
+				O::st(headw, qp_next(h, cur));
+				return 0u;
+			});
+			if (chains && log)
+				V::one([&] {
+					log->taken_chains(chains);
+					return 0u;
+				});
+			out.each_taken(r, [&](u64 item) { O::st_rlx(L::at(item), POISON); });
+			V::fence();
+			return r;
+		}
+		/* hp is the last linked item: see clq_dequeue_n */
+		if (V::one([&] { return O::cas(tailw, hp, 0ull); }) == hp) {
+			V::one([&] {
+				O::st(headw, qp_next(h, 0ull));
+				return 0u;
+			});
+			out.one(0, hp);
+			V::fence();
+			return 1;
+		}
+		V::one([&] {
+			O::st(hl, 0ull);
+			return 0u;
+		});
+		while (idle < limit && V::one([&] { return O::ld(hl); }) == 0ull &&
+		       V::one([&] { return O::ld(headw); }) == h) {
+			O::pause(it++);
+			idle++;
+		}
+	}
+	*timed_out = true;
+	return 0;
+}
+
+/* ------------------------------------------------------------------ */
 /* indexed queue (clIndexedQueue)                                      */
 /* ------------------------------------------------------------------ */
 /* Words {tag:32 | index:32}, index 0 = none.  The Michael-Scott queue

@@ -113,6 +113,98 @@ struct gpu_ops_t {
 		__nanosleep(t < CAP ? t : CAP);
 	}
 };
+/* The vector policy of the queue algorithms: 32 lanes of a warp, all of
+ * which call. */
+struct gpu_lanes {
+	template <class T>
+	struct reg {
+		T v;
+		__device__ __forceinline__ T &operator[](uint32_t) { return v; }
+		__device__ __forceinline__ const T &operator[](uint32_t) const { return v; }
+	};
+	template <class F>
+	static __device__ __forceinline__ void each(F f)
+	{
+		f(lane_id());
+	}
+	template <class F>
+	static __device__ __forceinline__ auto one(F f) -> decltype(f())
+	{
+		decltype(f()) r = 0;
+		if (lane_id() == 0)
+			r = f();
+		__syncwarp();
+		return shfl(r, 0);
+	}
+	static __device__ __forceinline__ uint32_t ballot(const reg<bool> &x) { return __ballot_sync(0xffffffffu, x.v); }
+	template <class T>
+	static __device__ __forceinline__ T get(const reg<T> &x, uint32_t j)
+	{
+		return shfl(x.v, j);
+	}
+	template <class T>
+	static __device__ __forceinline__ reg<T> above(const reg<T> &x)
+	{
+		return reg<T>{__shfl_down_sync(0xffffffffu, x.v, 1)};
+	}
+	static __device__ __forceinline__ void fence() { fence_acqrel(); }
+	template <class T>
+	static __device__ __forceinline__ T shfl(T v, uint32_t j)
+	{
+		return __shfl_sync(0xffffffffu, v, j);
+	}
+	static __device__ __forceinline__ bool shfl(bool v, uint32_t j) { return __shfl_sync(0xffffffffu, (int)v, j) != 0; }
+};
+/* Where gpu_lanes' dequeues put what they take: an array all lanes can
+ * read (shared memory), */
+struct lanes_out_array {
+	unsigned long long *a;
+	__device__ __forceinline__ void run(uint32_t at, const gpu_lanes::reg<unsigned long long> &item, uint32_t first,
+			uint32_t n)
+	{
+		const uint32_t j = lane_id() - first;
+		if (j < n)
+			a[at + j] = item.v;
+	}
+	__device__ __forceinline__ void one(uint32_t at, unsigned long long item)
+	{
+		if (lane_id() == 0)
+			a[at] = item;
+	}
+	template <class F>
+	__device__ __forceinline__ void each_taken(uint32_t r, F f)
+	{
+		__syncwarp();
+		for (uint32_t i = 1 + lane_id(); i < r; i += 32)
+			f(a[i]);
+	}
+};
+/* or the lanes' own registers (lane base + i gets the i-th). */
+struct lanes_out_regs {
+	unsigned long long mine;
+	uint32_t base;
+	__device__ __forceinline__ void run(uint32_t at, const gpu_lanes::reg<unsigned long long> &item, uint32_t first,
+			uint32_t n)
+	{
+		const uint32_t i = lane_id() - base - at;
+		const unsigned long long x = __shfl_sync(0xffffffffu, item.v, (i + first) & 31u);
+		if (i < n)
+			mine = x;
+	}
+	__device__ __forceinline__ void one(uint32_t at, unsigned long long item)
+	{
+		if (lane_id() == base + at)
+			mine = item;
+	}
+	template <class F>
+	__device__ __forceinline__ void each_taken(uint32_t r, F f)
+	{
+		const uint32_t i = lane_id() - base;
+		if (i >= 1 && i < r)
+			f(mine);
+	}
+};
+
 /* per-thread calls */
 typedef gpu_ops_t<KMA_QUEUE_PAUSE_MAX_NS> gpu_ops;
 /* the warp and block forms */
@@ -136,12 +228,15 @@ typedef gpu_ops_t<KMA_QUEUE_GROUP_PAUSE_MAX_NS> gpu_ops_group;
  * log may serve any number of queues of one kind.  No counterpart in the
  * reference.
  */
+#define KMA_LOG_NOTES_LOG2 10
+#define KMA_LOG_NOTES (1u << KMA_LOG_NOTES_LOG2)
 struct kma_chain_log {
 	static constexpr bool enabled = true;
 	unsigned long long *rec; /* [mask + 1][32] pointers, or [mask + 1][64] u32 indices (first 32 used) */
 	unsigned int *next;      /* record counter, a line of its own */
 	uint32_t mask;
 	uint32_t pad;
+	ulonglong2 *notes;       /* [KMA_LOG_NOTES] {item, record number}: see kma_q::clq_dequeue_v */
 
 	/* a record's slot; its entries are read with ld (relaxed) */
 	__device__ __forceinline__ const unsigned long long *clq_record(uint32_t recno) const
@@ -152,14 +247,38 @@ struct kma_chain_log {
 	{
 		return reinterpret_cast<const uint32_t *>(&rec[(size_t)(recno & mask) * 32]);
 	}
-	static __device__ __forceinline__ unsigned long long ld(const unsigned long long *p)
+	/* (entry 0 of a pointer record has the chain's length above the pointer) */
+	static __device__ __forceinline__ unsigned long long raw(const unsigned long long *p)
 	{
 		return kma_detail::ld_relaxed64(p);
+	}
+	static __device__ __forceinline__ unsigned long long ld(const unsigned long long *p)
+	{
+		return raw(p) & kma_q::PTR_MASK;
+	}
+	/* one of the notes per item (by hash), overwritten freely: a queue needs
+	 * one at a time, its head's */
+	__device__ __forceinline__ ulonglong2 *note_of(unsigned long long item) const
+	{
+		return &notes[((item >> 3) * 0x9E3779B97F4A7C15ull) >> (64 - KMA_LOG_NOTES_LOG2)];
+	}
+	__device__ __forceinline__ bool resume(unsigned long long item, uint32_t *recno) const
+	{
+		unsigned long long i, r;
+		asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(i), "=l"(r) : "l"(note_of(item)) : "memory");
+		*recno = (uint32_t)r;
+		return i == item;
+	}
+	__device__ __forceinline__ void note(unsigned long long item, uint32_t recno) const
+	{
+		asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};"
+			     ::"l"(note_of(item)), "l"(item), "l"((unsigned long long)recno) : "memory");
 	}
 	static __device__ __forceinline__ uint32_t ld(const uint32_t *p) { return kma_detail::ld_relaxed(p); }
 	__device__ __forceinline__ uint32_t take() { return atomicAdd(next, 1u) & kma_q::LOG_RECNO_MASK; }
 	/* chains taken from their records (next[1], a count for reports) */
 	__device__ __forceinline__ void taken(uint32_t) const { atomicAdd(next + 1, 1u); }
+	__device__ __forceinline__ void taken_chains(uint32_t n) const { atomicAdd(next + 1, n); }
 	__device__ __forceinline__ unsigned long long *clq_slot(uint32_t recno) { return &rec[(size_t)(recno & mask) * 32]; }
 	__device__ __forceinline__ uint32_t *iq_slot(uint32_t recno)
 	{
@@ -348,7 +467,8 @@ __device__ inline int kma_clqueue_enqueue_warp(kma_clqueue *q, kma_clqueue_item 
 	if (ok) {
 		unsigned long long link = gp.next != lane ? nip : 0ull;
 		if (logged) {
-			log->clq_slot(recno)[gp.rank] = ip;
+			log->clq_slot(recno)[gp.rank] =
+				gp.rank == 0 ? ip | (unsigned long long)gp.size << kma_q::LOG_LEN_SHIFT : ip;
 			link |= gp.rank == 0 ? kma_q::clq_mark_first(recno, gp.size)
 					     : (gp.rank == 1 ? kma_q::clq_mark_second(recno) : 0ull);
 		}
@@ -381,6 +501,21 @@ __device__ inline kma_clqueue_item *kma_clqueue_dequeue_warp(kma_clqueue *q, uin
 	const uint32_t active = __activemask();
 	const uint32_t lane = lane_id();
 	const lane_group gp = group_by(active, lane, q ? (unsigned long long)q : ~0ull);
+	if (log && q && gp.peers == 0xffffffffu) {
+		/* a full warp on one queue: all its lanes take part in the hold */
+		lanes_out_regs o = {0ull, 0u};
+		for (uint32_t turn = 0; o.base < 32 && turn < 32; turn++) {
+			bool timed_out = false;
+			const uint32_t r = kma_q::clq_dequeue_v<gpu_ops_group, clq_link_head, gpu_lanes>(
+				&q->head, &q->tail, o, 32u - o.base, spin_limit, &timed_out, log);
+			if (timed_out && lane == 0)
+				flag_err(err, KMA_ERR_TIMEOUT);
+			if (r == 0)
+				break;
+			o.base += r;
+		}
+		return reinterpret_cast<kma_clqueue_item *>(o.mine);
+	}
 	unsigned long long got = 0;
 	uint32_t served = 0;
 	bool more = q != nullptr;
@@ -441,11 +576,15 @@ __device__ inline uint32_t block_rank(bool want, unsigned int *cnt, uint32_t *to
 } /* namespace kma_detail */
 
 /* Block form of dequeue: every thread of the block calls it, all with the
- * same q; a thread with `want` false takes nothing (NULL).  One thread
- * serves the block's requests, in turns of one hold of the head each, and
- * a hold takes several logged chains in a row, so a block takes its items
- * in a few more round trips than a warp takes its own instead of one hold
- * per warp.  smem: blockDim + 1 words of shared memory the call may use.
+ * same q; a thread with `want` false takes nothing (NULL).  With a chain
+ * log the first warp serves the block's requests (kma_q::clq_dequeue_v),
+ * without one (a walk, one item at a time) or in a block of less than a
+ * warp its first thread, in turns of one hold of the head each.  A hold
+ * takes several logged chains in a row, and is a chain of round trips
+ * whatever the load: 4 to take the head, 2 a chain, 10.4 us for 256 items
+ * (24 M items/s; 12.2 with one thread and 3 a chain).  Where the chains do
+ * not fill the batches (2^18 + 77 threads) 22.5 M items/s; with one thread,
+ * which walks from a head in the middle of a chain, 4.  smem: blockDim + 1 words of shared memory the call may use.
  * Items go to the wanting threads in the order block_rank numbers them;
  * threads left over when the queue runs empty get NULL.  No counterpart in
  * the reference. */
@@ -457,7 +596,26 @@ __device__ inline kma_clqueue_item *kma_clqueue_dequeue_block(kma_clqueue *q, bo
 	uint32_t k = 0;
 	const uint32_t rank = block_rank(want && q, &w[0], &k);
 	unsigned long long *out = smem + 1;
-	if (block_tid() == 0) {
+	const uint32_t tid = block_tid();
+	if (log && q && blockDim.x * blockDim.y * blockDim.z >= 32) {
+		/* all lanes of the first warp take part in the hold */
+		if (tid < 32) {
+			uint32_t served = 0;
+			for (uint32_t turn = 0; served < k && turn < k; turn++) {
+				bool timed_out = false;
+				lanes_out_array o = {out + served};
+				const uint32_t r = kma_q::clq_dequeue_v<gpu_ops_group, clq_link_head, gpu_lanes>(
+					&q->head, &q->tail, o, k - served, spin_limit, &timed_out, log);
+				if (timed_out && tid == 0)
+					flag_err(err, KMA_ERR_TIMEOUT);
+				if (r == 0)
+					break;
+				served += r;
+			}
+			if (tid == 0)
+				w[1] = served;
+		}
+	} else if (tid == 0) {
 		uint32_t served = 0;
 		for (uint32_t turn = 0; q && served < k && turn < k; turn++) {
 			bool timed_out = false;

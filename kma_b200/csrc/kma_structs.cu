@@ -654,8 +654,8 @@ extern "C" int kma_chain_log_create(uint32_t records, int device, void *stream, 
 		return KMA_ENOMEM;
 	l->device = current_device();
 	/* header line, counter line, then the records (zeroed: an entry is 0
-	 * until a chain fills it) */
-	const size_t hdr = 256, bytes = hdr + (size_t)records * 256;
+	 * until a chain fills it) and the notes */
+	const size_t hdr = 256, rec = (size_t)records * 256, bytes = hdr + rec + KMA_LOG_NOTES * sizeof(ulonglong2);
 	if (cudaMalloc(&l->mem, bytes) != cudaSuccess) {
 		cudaGetLastError();
 		free(l);
@@ -667,6 +667,7 @@ extern "C" int kma_chain_log_create(uint32_t records, int device, void *stream, 
 	hl.rec = (unsigned long long *)((unsigned char *)l->mem + hdr);
 	hl.next = (unsigned int *)((unsigned char *)l->mem + 128);
 	hl.mask = records - 1;
+	hl.notes = (ulonglong2 *)((unsigned char *)l->mem + hdr + rec);
 	cudaStream_t st = kma_stream(stream);
 	int rc = KMA_OK;
 	if (cudaMemsetAsync(l->mem, 0, bytes, st) != cudaSuccess)

@@ -31,7 +31,7 @@
  *     and report it.
  *
  *   queue_harness clq|iq THREADS CHAINS MAX_CHAIN DEQ_BATCH DELAY_PROB SEED
- *                 [PRODUCERS [RECYCLE [LOG_RECORDS [PHASED]]]]
+ *                 [PRODUCERS [RECYCLE [LOG_RECORDS [PHASED [LANES]]]]]
  *   queue_harness stuck
  *
  * PRODUCERS of the threads (default half) append CHAINS fresh chains of
@@ -41,7 +41,9 @@
  * With few producers the queue is mostly empty, so the empty <-> one-item
  * transitions and the append window are met all the time; PHASED 1 holds
  * the consumers back until the producers are done (config 3's order), so
- * batches meet whole logged chains and take several per hold.  Prints one
+ * batches meet whole logged chains and take several per hold; LANES 1
+ * dequeues with the warp's text (clq_dequeue_v), its 32 lanes as arrays:
+ * LANES 2 every other batch, so that both texts meet on one queue.  Prints one
  * JSON line (with the chains taken from records and the dequeue calls
  * that took items); exits 0 when every check passed.  The reference's own
  * queues are the parity oracle (serial replays against tests/golden);
@@ -127,14 +129,92 @@ struct HostLog {
 	std::vector<uint32_t> iq;
 	uint32_t mask = 0;
 	std::atomic<uint32_t> next{0};
+	/* notes of clq_dequeue_v: {item, record number} by the item's hash */
+	static const uint32_t NOTES = 64;
+	mutable std::atomic<u64> note_item[NOTES] = {}, note_rec[NOTES] = {};
+	static uint32_t note_of(u64 item) { return (uint32_t)(((item >> 3) * 0x9E3779B97F4A7C15ull) >> 58); }
+	bool resume(u64 item, uint32_t *recno) const
+	{
+		const uint32_t i = note_of(item);
+		*recno = (uint32_t)note_rec[i].load(std::memory_order_relaxed);
+		return note_item[i].load(std::memory_order_relaxed) == item;
+	}
+	void note(u64 item, uint32_t recno) const
+	{
+		const uint32_t i = note_of(item);
+		note_item[i].store(item, std::memory_order_relaxed);
+		note_rec[i].store(recno, std::memory_order_relaxed);
+	}
 	const u64 *clq_record(uint32_t recno) const { return &clq[(size_t)(recno & mask) * 32]; }
 	const uint32_t *iq_record(uint32_t recno) const { return &iq[(size_t)(recno & mask) * 32]; }
-	static u64 ld(const u64 *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
+	static u64 raw(const u64 *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
+	static u64 ld(const u64 *p) { return raw(p) & kma_q::PTR_MASK; }
 	static uint32_t ld(const uint32_t *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
 	uint32_t take() { return next.fetch_add(1) & kma_q::LOG_RECNO_MASK; }
 	mutable std::atomic<uint64_t> chains{0};
 	void taken(uint32_t) const { chains++; }
+	void taken_chains(uint32_t n) const { chains += n; }
 };
+
+/* The vector policy on the host: 32 lanes as arrays, and a batch's output. */
+struct HostLanes {
+	template <class T>
+	struct reg {
+		T v[32];
+		T &operator[](uint32_t j) { return v[j]; }
+		const T &operator[](uint32_t j) const { return v[j]; }
+	};
+	template <class F>
+	static void each(F f)
+	{
+		for (uint32_t j = 0; j < 32; j++)
+			f(j);
+	}
+	template <class F>
+	static auto one(F f) -> decltype(f())
+	{
+		return f();
+	}
+	static uint32_t ballot(const reg<bool> &x)
+	{
+		uint32_t b = 0;
+		for (uint32_t j = 0; j < 32; j++)
+			b |= (uint32_t)x[j] << j;
+		return b;
+	}
+	template <class T>
+	static T get(const reg<T> &x, uint32_t j)
+	{
+		return x[j];
+	}
+	template <class T>
+	static reg<T> above(const reg<T> &x)
+	{
+		reg<T> y;
+		for (uint32_t j = 0; j < 32; j++)
+			y[j] = x[j < 31 ? j + 1 : j];
+		return y;
+	}
+	static void fence() { std::atomic_thread_fence(std::memory_order_acquire); }
+};
+struct HostOut {
+	u64 *a;
+	void run(uint32_t at, const HostLanes::reg<u64> &item, uint32_t first, uint32_t n)
+	{
+		for (uint32_t i = 0; i < n; i++)
+			a[at + i] = item[first + i];
+	}
+	void one(uint32_t at, u64 item) { a[at] = item; }
+	template <class F>
+	void each_taken(uint32_t r, F f)
+	{
+		for (uint32_t i = 1; i < r; i++)
+			f(a[i]);
+	}
+};
+/* dequeue with the warp's text: 0 never, 1 always, 2 every other batch */
+int g_lanes = 0;
+
 HostLog g_log;
 const HostLog *log_ptr() { return g_log.mask || !g_log.clq.empty() || !g_log.iq.empty() ? &g_log : nullptr; }
 
@@ -203,7 +283,8 @@ void run_clq(int threads, int chains, int maxc, int batch, double recycle, uint6
 			__atomic_fetch_add(&bk.appends[(size_t)(v[j] - items.data())], 1, __ATOMIC_RELAXED);
 			u64 link = j + 1 < len ? (u64)v[j + 1] : 0ull;
 			if (logged) {
-				__atomic_store_n(&g_log.clq[(size_t)(recno & g_log.mask) * 32 + j], (u64)v[j], __ATOMIC_RELAXED);
+				__atomic_store_n(&g_log.clq[(size_t)(recno & g_log.mask) * 32 + j],
+						 (u64)v[j] | (j == 0 ? (u64)len << kma_q::LOG_LEN_SHIFT : 0ull), __ATOMIC_RELAXED);
 				link |= j == 0 ? kma_q::clq_mark_first(recno, (uint32_t)len)
 					       : (j == 1 ? kma_q::clq_mark_second(recno) : 0ull);
 			}
@@ -240,8 +321,10 @@ void run_clq(int threads, int chains, int maxc, int batch, double recycle, uint6
 			bool done = producing.load() == 0;
 			bool to = false;
 			uint32_t k = g_fixed_batch ? (uint32_t)batch : 1 + (uint32_t)(rnd() % batch);
-			uint32_t r = kma_q::clq_dequeue_n<HostOps, LinkAtItem>(&q[0], &q[1], out.data(), k, LIMIT, &to,
-									       log_ptr());
+			HostOut ho = {out.data()};
+			uint32_t r = g_lanes == 1 || (g_lanes == 2 && (rnd() & 1))
+				? kma_q::clq_dequeue_v<HostOps, LinkAtItem, HostLanes>(&q[0], &q[1], ho, k, LIMIT, &to, log_ptr())
+				: kma_q::clq_dequeue_n<HostOps, LinkAtItem>(&q[0], &q[1], out.data(), k, LIMIT, &to, log_ptr());
 			if (to)
 				bk.tmo++;
 			back.clear();
@@ -459,6 +542,17 @@ int run_stuck()
 		printf("{\"case\": \"iq_head_held\", \"taken\": %u, \"timed_out\": %s}\n", r, to ? "true" : "false");
 		ok &= r == 0 && to && ends[0] == kma_q::tw_make(1, 1);
 	}
+	for (int state = 0; state < 2; state++) { /* the same two with the warp's text */
+		Item a{}, b{};
+		u64 q[2] = {(u64)&a, (u64)&b};
+		a.next = state == 0 ? kma_q::POISON : 0ull;
+		u64 buf[4];
+		HostOut out = {buf};
+		bool to = false;
+		uint32_t r = kma_q::clq_dequeue_v<HostOps, LinkAtItem, HostLanes>(&q[0], &q[1], out, 4, limit, &to,
+										 (const HostLog *)nullptr);
+		ok &= r == 0 && to && a.next == (state == 0 ? kma_q::POISON : 0ull) && q[0] == (u64)&a;
+	}
 	printf("{\"stuck_ok\": %s}\n", ok ? "true" : "false");
 	return ok ? 0 : 1;
 }
@@ -467,9 +561,9 @@ int main(int argc, char **argv)
 {
 	if (argc == 2 && strcmp(argv[1], "stuck") == 0)
 		return run_stuck();
-	if (argc < 8 || argc > 12) {
+	if (argc < 8 || argc > 13) {
 		fprintf(stderr, "usage: %s clq|iq THREADS CHAINS MAX_CHAIN DEQ_BATCH DELAY_PROB SEED "
-			"[PRODUCERS [RECYCLE [LOG_RECORDS [PHASED]]]]\n       %s stuck\n", argv[0], argv[0]);
+			"[PRODUCERS [RECYCLE [LOG_RECORDS [PHASED [LANES]]]]]\n       %s stuck\n", argv[0], argv[0]);
 		return 2;
 	}
 	const bool clq = strcmp(argv[1], "clq") == 0;
@@ -490,6 +584,7 @@ int main(int argc, char **argv)
 	const double recycle = argc >= 10 ? atof(argv[9]) : 0.5;
 	const uint32_t log_records = argc >= 11 ? (uint32_t)strtoul(argv[10], NULL, 0) : 0u;
 	g_phased = argc >= 12 && atoi(argv[11]) != 0;
+	g_lanes = argc >= 13 ? atoi(argv[12]) : 0;
 	if (log_records) {
 		if (log_records & (log_records - 1))
 			return 2; /* a power of two */

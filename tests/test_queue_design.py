@@ -184,3 +184,35 @@ def test_harness_detects_planted_mistakes(harness, tmp_path, name):
         if rc != 0:
             return
     raise AssertionError(f"mutant {name} passed unnoticed: {st}")
+
+
+# the warp's text of the dequeue (clq_dequeue_v), always (1) or mixed with
+# the one-thread text on one queue (2)
+LANES_CONFIGS = [
+    "8 20000 1 1 0.01 1 1 0.5 64 0",           # single items, the queue mostly empty
+    "8 5000 32 32 0.02 7 4 0.5 65536 0",
+    "8 5000 32 32 0.02 8 4 0.5 8 0",           # stale records and notes
+    "8 20000 8 64 0.01 13 2 0.5 2 0",
+    "8 5000 32 256 0.02 12 4 0.5 1024 0",
+    "8 5000 -32 -256 0.02 15 4 0.5 65536 1",
+    "8 5000 32 -256 0.02 19 4 0.5 65536 1",    # heads in the middle of chains
+    "3 20000 8 8 0.01 6 1 0.5 0 0",            # no log
+]
+
+
+@pytest.mark.parametrize("lanes", [1, 2])
+@pytest.mark.parametrize("cfg", LANES_CONFIGS)
+def test_warp_text_conserves_and_keeps_order(harness, cfg, lanes):
+    rc, st = run(harness, "clq", f"{cfg} {lanes}")
+    assert rc == 0 and st.get("ok"), st
+    assert st["taken"] + st["left"] >= st["appended"] > 0
+    assert st["conservation_faults"] == 0 and st["order_faults"] == 0 and st["timeouts"] == 0
+
+
+@pytest.mark.parametrize("batch", [256, 250])
+def test_warp_text_takes_chains_from_the_log(harness, batch):
+    """Whole chains of a hold come from their records, also where the
+    batches end in the middle of chains (250) and each hold starts there."""
+    rc, st = run(harness, "clq", f"8 5000 -32 -{batch} 0 15 4 0 65536 1 1")
+    assert rc == 0 and st.get("ok"), st
+    assert st["log_chains"] / st["dequeue_calls"] > 6

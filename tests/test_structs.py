@@ -373,3 +373,18 @@ def test_gpu_tree_check_over_shapes(shape):
     assert (st["sorted"], st["err"], st["live_keys"]) == (1, 0, len(want))
     assert st["keys_sum"] == int(want.sum())
     assert st["keys_xor"] == int(np.bitwise_xor.reduce(want)) if len(want) else st["keys_xor"] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["warp", "block"])
+@pytest.mark.parametrize("threads,per", [(1, 3), (31, 5), (33, 5), (257, 9), (4096 + 37, 16), (65536 + 33, 3)])
+def test_gpu_clqueue_ragged_chains_conserve(form, threads, per):
+    """Thread counts that leave short chains, so that holds end, and later
+    ones begin, in the middle of chains."""
+    from kma_b200 import structs
+    flag = {"warp": structs.C3_WARP, "block": structs.C3_BLOCK}[form]
+    st = structs.c3_queue(structs.C3_CLQUEUE | flag, threads, per, 1, seed=threads)
+    n = threads * per
+    assert st["err"] == 0 and st["walk_ok"] == 1 and st["empty"] == 0
+    assert st["enqueued"] == st["out_count"] == n
+    assert st["out_xor"] == st["in_xor"] and st["out_sum"] == st["in_sum"] == n * (n - 1) // 2
