@@ -11,9 +11,10 @@
 
 namespace kma_wl {
 
+const uint64_t SPLITMIX_STEP = 0x9E3779B97F4A7C15ull;
 __device__ __forceinline__ uint64_t splitmix(uint64_t &s)
 {
-	uint64_t z = (s += 0x9E3779B97F4A7C15ull);
+	uint64_t z = (s += SPLITMIX_STEP);
 	z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
 	z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
 	return z ^ (z >> 31);

@@ -131,3 +131,23 @@ def test_gpu_serve_plain_calls_equal_warp_calls():
             assert a["status"] == b["status"] == "ok"
             assert (a["checksum"], a["edges"], a["mallocs"]) == (b["checksum"], b["edges"], b["mallocs"])
         _empty(h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("block_dim", [32, 256, 1024])
+@pytest.mark.parametrize("deg_max,gamma", [(1, 2.1), (127, 1.05), (128, 1.05), (129, 1.05), (4096, 1.2)])
+def test_gpu_serve_degrees_and_blocks(deg_max, gamma, block_dim):
+    """Partial warps and blocks, and degrees on both sides of where a page or
+    a vertex is a whole warp's work (a small gamma makes many of them)."""
+    from kma_b200 import Heap
+    from kma_b200.serve import Server
+    nv = [1, 31, 33, 1000, 2049]
+    seeds = [deg_max * 10 + i for i in range(len(nv))]
+    with Heap(32768, 14) as h, Server(h, slots=2, max_vertices=2049, deg_max=deg_max, gamma=gamma,
+                                      block_dim=block_dim) as s:
+        for _ in range(2):  # a slot's counters start at zero again
+            res, _ = s.run(nv, seeds)
+            for r, n, sd in zip(res, nv, seeds):
+                assert r["status"] == "ok" and r["nulls"] == 0 and r["mallocs"] == r["frees"] >= n
+                assert (r["checksum"], r["edges"]) == expected_result(sd, n, deg_max, gamma)
+        _empty(h)
