@@ -160,9 +160,9 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
 	asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
 	return v;
 }
-__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v)
+__device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v)
 {
-	asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+	asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ void st_release64(unsigned long long *p, unsigned long long v)
 {
@@ -363,8 +363,11 @@ __device__ __forceinline__ unsigned long long global_warp()
 }
 __device__ __forceinline__ uint32_t my_shard(const kma_heap *h, uint32_t c)
 {
-	uint32_t n = h->cls_nsh[c];
-	return n > 1 ? (uint32_t)(global_warp() % n) : 0u;
+	const uint32_t n = __ldg(&h->cls_nsh[c]);
+	const unsigned long long w = global_warp();
+	/* a 64-bit remainder is some hundred instructions: only for grids of
+	 * 2^32 warps and more */
+	return (w >> 32) ? (uint32_t)(w % n) : (uint32_t)w % n;
 }
 __device__ __forceinline__ uint32_t *cls_word(kma_heap *h, uint32_t c, uint32_t shard)
 {
@@ -461,10 +464,15 @@ __device__ __forceinline__ int64_t msq_dequeue(kma_heap *h)
  * through the number it read, so tickets, counts and the slot read are
  * relaxed; a count seen before its slot store only makes a dequeuer wait
  * on the slot's sequence number. */
+/* ticket -> slot: as the 64-bit remainder, which only tickets past 2^32 take */
+__device__ __forceinline__ uint32_t ring_slot(unsigned long long pos, uint32_t cap)
+{
+	return (pos >> 32) ? (uint32_t)(pos % cap) : (uint32_t)pos % cap;
+}
 __device__ __forceinline__ int ring_enqueue(kma_heap *h, uint32_t s)
 {
 	unsigned long long pos = add64_relaxed(&h->free_tail.v, 1ull);
-	unsigned long long *slot = &h->ring[pos % h->ring_cap];
+	unsigned long long *slot = &h->ring[ring_slot(pos, __ldg(&h->ring_cap))];
 	uint32_t lim = h->spin_limit;
 	for (uint32_t it = 0; it < lim; it++) {
 		unsigned long long w = ld_relaxed64(slot);
@@ -477,6 +485,24 @@ __device__ __forceinline__ int ring_enqueue(kma_heap *h, uint32_t s)
 	}
 	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RING_ENQ);
 	return 0;
+}
+
+/* the superblock of head ticket `pos` (claimed against ring_avail) */
+__device__ __forceinline__ int64_t ring_take(kma_heap *h, unsigned long long pos)
+{
+	const uint32_t cap = __ldg(&h->ring_cap);
+	unsigned long long *slot = &h->ring[ring_slot(pos, cap)];
+	uint32_t lim = h->spin_limit;
+	for (uint32_t it = 0; it < lim; it++) {
+		unsigned long long w = ld_relaxed64(slot);
+		if ((uint32_t)(w >> 32) == (uint32_t)(pos + 1)) {
+			st_relaxed64(slot, (unsigned long long)(uint32_t)(pos + cap) << 32);
+			return (int64_t)(uint32_t)w;
+		}
+		backoff(it);
+	}
+	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RING_DEQ);
+	return -2;
 }
 
 __device__ __forceinline__ int64_t ring_dequeue(kma_heap *h)
@@ -501,19 +527,39 @@ __device__ __forceinline__ int64_t ring_dequeue(kma_heap *h)
 			}
 		}
 	}
-	unsigned long long pos = add64_relaxed(&h->free_head.v, 1ull);
-	unsigned long long *slot = &h->ring[pos % h->ring_cap];
-	uint32_t lim = h->spin_limit;
-	for (uint32_t it = 0; it < lim; it++) {
-		unsigned long long w = ld_relaxed64(slot);
-		if ((uint32_t)(w >> 32) == (uint32_t)(pos + 1)) {
-			st_relaxed64(slot, (unsigned long long)(uint32_t)(pos + h->ring_cap) << 32);
-			return (int64_t)(uint32_t)w;
-		}
-		backoff(it);
+	return ring_take(h, add64_relaxed(&h->free_head.v, 1ull));
+}
+
+/* The calling lanes (`active`) that `want` one each take superblocks
+ * together: one claim of the availability count and one ticket add for all
+ * of them.  Each gets what a ring_dequeue in lane order would: lanes beyond
+ * the count go through ring_dequeue's own near-empty path. */
+__device__ __forceinline__ int64_t ring_dequeue_lanes(kma_heap *h, uint32_t active, bool want)
+{
+	const uint32_t m = __ballot_sync(active, want);
+	if (!m)
+		return -1;
+	const uint32_t first = __ffs(m) - 1, rank = __popc(m & lanemask_lt());
+	int32_t granted = 0;
+	unsigned long long pos = 0;
+	if (lane_id() == first) {
+		int32_t *avail = reinterpret_cast<int32_t *>(&h->ring_avail.v);
+		const int32_t n = __popc(m);
+		const int32_t old = atomicSub(avail, n);
+		/* of n single claims the ones that find at least two succeed */
+		granted = old - 1 < 0 ? 0 : old - 1 < n ? old - 1 : n;
+		if (granted < n)
+			atomicAdd(avail, n - granted);
+		if (granted)
+			pos = add64_relaxed(&h->free_head.v, (unsigned long long)granted);
 	}
-	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RING_DEQ);
-	return -2;
+	granted = __shfl_sync(active, granted, first);
+	pos = __shfl_sync(active, pos, first);
+	if (!want)
+		return -1;
+	if ((int32_t)rank >= granted)
+		return ring_dequeue(h);
+	return ring_take(h, pos + rank);
 }
 
 __device__ __forceinline__ int sb_enqueue(kma_heap *h, uint32_t s)
@@ -524,11 +570,19 @@ __device__ __forceinline__ int64_t sb_dequeue(kma_heap *h)
 {
 	return (h->flags & KMA_HEAP_RING) ? ring_dequeue(h) : msq_dequeue(h);
 }
+/* for the calling lanes that want one; every lane of `active` calls */
+__device__ __forceinline__ int64_t sb_dequeue_lanes(kma_heap *h, uint32_t active, bool want)
+{
+	if (h->flags & KMA_HEAP_RING)
+		return ring_dequeue_lanes(h, active, want);
+	return want ? msq_dequeue(h) : -1;
+}
 
 /* Prepare superblock s for class c: zero its bitmap except the bits in
  * [pre_lo, slots), which are pre-set (claimed by the refiller), record its
- * home shard, then publish state = (c, slots, free).  kma.cl:177-189, with
- * the bitmap written before the state becomes visible. */
+ * home shard and the state (c, slots, free).  kma.cl:177-189.  Nobody else
+ * can reach s yet: the caller's release of the class slot that names it (or
+ * of the pointers it hands out) publishes all three. */
 __device__ __forceinline__ void sb_format(kma_heap *h, uint32_t s, uint32_t c, uint32_t pre_lo,
 		uint32_t fr, uint32_t shard)
 {
@@ -549,7 +603,7 @@ __device__ __forceinline__ void sb_format(kma_heap *h, uint32_t s, uint32_t c, u
 		*bitmap_word(h, sb, k) = v;
 	}
 	h->sb_home[s] = (uint16_t)shard;
-	st_release(&h->sb_state[s], st_make(c, slots, fr));
+	st_relaxed(&h->sb_state[s], st_make(c, slots, fr));
 }
 
 } /* namespace kma_detail */
@@ -814,201 +868,47 @@ __device__ __forceinline__ void tally(kma_tally *t, int k)
 		t->n[k]++;
 }
 
-/* Leader-side state of one group's reservation.  kword/known: the last
- * bitmap word this reservation touched and its value as the atomicOr
- * returned it (claims go blind on a word first: setting a bit that is
- * already set changes nothing, and the returned word says what is free). */
+/* Leader-side state of one group's reservation.  kword/known: a bitmap word
+ * and its value as this reservation last saw it (claims go blind on a word
+ * it has not seen: setting a bit that is already set changes nothing, and
+ * the returned word says what is free). */
 struct warp_resv {
-	uint32_t sb, cls, left, cursor, pre_hi, hint, kword, known;
+	uint32_t sb, left, cursor, pre_hi, hint, kword, known;
 	bool pre;
 };
 
-/* Reserve up to `want` slots of class c.  On success fills r (sb, left =
- * number reserved, cursor = first slot to scan from, hint) and returns 1;
- * returns 0 when the heap is exhausted or a spin expired. */
-__device__ __forceinline__ int warp_reserve(kma_heap *h, uint32_t c, uint32_t want, warp_resv &r,
-		kma_tally *tl, uint32_t *hint)
+/* A superblock that is no class slot's current one is reserved from, when a
+ * hint names it, if it serves the whole request and its free bits are quick
+ * to find: in at most two bitmap words, or a quarter of its slots. */
+__device__ __forceinline__ bool hint_serves(const kma_heap *h, uint32_t c, uint32_t slots, uint32_t want, uint32_t st)
 {
-	uint32_t slots = h->cls_slots[c];
-	uint32_t shard = my_shard(h, c);
-	if (want >= slots && slots > 1) {
-		/* the group fills a whole superblock: take a fresh one privately
-		 * (it would be detached at once anyway) */
-		tally(tl, KMA_T_REFILL);
-		int64_t s = sb_dequeue(h);
-		if (s < 0)
-			return 0;
-		sb_format(h, (uint32_t)s, c, 0, 0, shard);
-		r.sb = (uint32_t)s;
-		r.cls = c;
-		r.left = slots;
-		r.cursor = 0;
-		r.pre_hi = slots;
-		r.hint = slots - 1;
-		r.pre = true;
-		r.kword = 0xffffffffu;
-		return 1;
-	}
-	uint32_t *clsw = cls_word(h, c, shard);
-	uint32_t lim = h->spin_limit;
-	/* the superblock this warp last reserved from in class c: its state is
-	 * loaded together with the class word, and used when the class word
-	 * still names it (saving the dependent load) */
-	uint32_t guess = hint ? hint[c] : 0u;
-	for (uint32_t it = 0; it < lim; it++) {
-		tally(tl, KMA_T_TRY);
-		uint32_t cur = ld_relaxed(clsw);
-		uint32_t st_guess = guess ? ld_relaxed(&h->sb_state[guess - KMA_CLS_BASE]) : 0u;
-		const bool poisoned = cur == KMA_POISON;
-		if (cur == 0 || (poisoned && slots <= KMA_PRIVATE_REFILL_SLOTS)) {
-			/* cur == 0: the reference's refill under POISON (kma.cl:166-195).
-			 * POISON on a class with few slots per superblock: the refill in
-			 * flight yields about one group's worth, so rather than queue
-			 * behind it take a fresh superblock without holding the class
-			 * slot, and publish the leftover slots only if the slot is empty
-			 * by then.  Serial execution never observes POISON. */
-			bool locked = false;
-			if (!poisoned) {
-				if (cas_relaxed(clsw, 0, KMA_POISON) != 0)
-					continue;
-				locked = true;
-			}
-			tally(tl, KMA_T_REFILL);
-			int64_t s = sb_dequeue(h);
-			if (s < 0) {
-				if (locked)
-					atomicExch(clsw, 0);
-				return 0;
-			}
-			uint32_t t = want < slots ? want : slots;
-			sb_format(h, (uint32_t)s, c, slots - t, slots - t, shard);
-			/* the refiller takes the top t slots, which are exactly the
-			 * hints slots-1 .. slots-t of t serial reservations */
-			uint32_t pub = t == slots ? 0u : (uint32_t)s + KMA_CLS_BASE;
-			/* release: a thread that finds s in the slot must find
-			 * its formatted state (a stale one would read as full and
-			 * get s detached with free slots nobody can reach) */
-			if (locked)
-				cas_release(clsw, KMA_POISON, pub);
-			else if (pub)
-				cas_release(clsw, 0, pub);
-			if (hint && pub)
-				hint[c] = pub;
-			r.sb = (uint32_t)s;
-			r.cls = c;
-			r.left = t;
-			r.cursor = slots - t;
-			r.pre_hi = slots;
-			r.hint = slots - 1;
-			r.pre = true;
-			r.kword = 0xffffffffu;
-			return 1;
-		}
-		if (poisoned) {
-			tally(tl, KMA_T_POISON);
-			backoff(it);
-			continue;
-		}
-		uint32_t s = cur - KMA_CLS_BASE;
-		uint32_t *stp = &h->sb_state[s];
-		const bool speculated = cur == guess;
-		uint32_t st = speculated ? st_guess : ld_relaxed(stp);
-		guess = cur;
-		if (st_class(st) != c || st_free(st) == 0) {
-			tally(tl, KMA_T_STALE);
-			/* the speculative state load may be older than cur */
-			if (speculated)
-				st = ld_relaxed(stp);
-			if (st_class(st) != c || st_free(st) == 0)
-				clear_stale(clsw, cur);
-			continue;
-		}
-		uint32_t fr = st_free(st);
-		uint32_t t = want < fr ? want : fr;
-		/* the first bitmap word the claim will visit is known already:
-		 * load it alongside the CAS instead of after it */
-		uint32_t k0 = (fr - t) >> 5;
-		uint32_t spec = ld_relaxed(bitmap_word(h, sb_addr(h, s), k0));
-		if (cas_relaxed(stp, st, st - t) != st) {
-			tally(tl, KMA_T_CASFAIL);
-			continue;
-		}
-		if (fr == t)
-			cas_relaxed(clsw, cur, 0);
-		if (hint)
-			hint[c] = cur;
-		r.sb = s;
-		r.cls = c;
-		r.left = t;
-		r.cursor = fr - t; /* lowest of the t serial hints fr-1 .. fr-t */
-		r.pre = false;
-		r.kword = k0;
-		r.known = spec;
-		r.hint = fr - 1;
-		return 1;
-	}
-	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RESERVE);
-	return 0;
+	const uint32_t fr = st_free(st);
+	return st_class(st) == c && fr >= want && (__ldg(&h->cls_words[c]) <= 2 || fr * 4 >= slots);
 }
 
-/* One claim step on the reservation: claims bits in one bitmap word.
- * Returns the claimed mask (possibly 0 when another thread won the bits
- * and the word must be re-read), and the word index in `word`. */
-__device__ __forceinline__ uint32_t warp_claim_step(kma_heap *h, warp_resv &r, uint32_t &word)
+/* The bits of bitmap word `word` that reservation r takes next, given what
+ * is known of it: the lowest `left` candidates at or above the cursor. */
+__device__ __forceinline__ uint32_t claim_pick(const kma_heap *h, const warp_resv &r, uint32_t c, uint32_t slots,
+		uint32_t &cand)
 {
-	uint32_t slots = h->cls_slots[r.cls];
-	uint32_t k = r.cursor >> 5;
-	word = k;
-	uint32_t lo = r.cursor & 31;
-	if (r.pre) {
-		/* bits [cursor, pre_hi) were set by sb_format */
-		uint32_t hi = r.pre_hi < (k + 1) * 32 ? r.pre_hi - k * 32 : 32;
-		uint32_t n = hi - lo;
-		uint32_t got = (n == 32 ? 0xffffffffu : ((1u << n) - 1u)) << lo;
-		r.cursor = k * 32 + hi;
-		r.left -= n;
-		return got;
-	}
-	unsigned char *sb = sb_addr(h, r.sb);
-	uint32_t *wp = bitmap_word(h, sb, k);
-	uint32_t words = h->cls_words[r.cls];
-	uint32_t valid = (k == words - 1 && (slots & 31)) ? ((1u << (slots & 31)) - 1u) : 0xffffffffu;
+	const uint32_t k = r.cursor >> 5, lo = r.cursor & 31;
+	const uint32_t valid = ((k + 1) * 32 > slots) ? ((1u << (slots & 31)) - 1u) : 0xffffffffu;
 	/* first visit of a word: assume its bits are clear; the atomicOr's
 	 * result then says which ones really were */
-	uint32_t v = r.kword == k ? r.known : 0u;
-	uint32_t cand = ~v & valid & (0xffffffffu << lo);
-	uint32_t pick = 0;
-	/* take the lowest `left` candidate bits */
-	if (__popc(cand) <= (int)r.left) {
-		pick = cand;
-	} else {
-		uint32_t top = nth_set_bit(cand, r.left - 1);
-		pick = cand & (top == 31 ? 0xffffffffu : ((2u << top) - 1u));
-	}
-	uint32_t got = 0;
-	if (pick) {
-		uint32_t old = bm_or(wp, pick);
-		got = pick & ~old;
-		r.kword = k;
-		r.known = old | pick;
-	}
-	r.left -= __popc(got);
-	if (got == pick) {
-		/* every candidate we wanted is ours: move on if more are needed */
-		if (r.left && __popc(cand) <= __popc(pick)) {
-			r.cursor = (k + 1) * 32;
-			if (r.cursor >= slots)
-				r.cursor = 0;
-			/* what is known of this word may predate the reservation
-			 * (the speculative load): the next visit, possibly of this
-			 * same word after a wrap, claims afresh.  An atomicOr's
-			 * result always shows at least `left` clear bits, which
-			 * is what guarantees progress. */
-			r.kword = 0xffffffffu;
-		}
-	}
-	return got;
+	const uint32_t v = r.kword == k ? r.known : 0u;
+	cand = ~v & valid & (0xffffffffu << lo);
+	if (__popc(cand) <= (int)r.left)
+		return cand;
+	const uint32_t top = nth_set_bit(cand, r.left - 1);
+	return cand & (top == 31 ? 0xffffffffu : ((2u << top) - 1u));
 }
+
+/* One lane's part in a step of kma_malloc_warp: */
+#define KMA_R_NONE 0u   /* nothing to reserve, or nothing got */
+#define KMA_R_TAKE 1u   /* reserve from superblock s */
+#define KMA_R_LOCK 2u   /* refill an empty class slot (POISON) */
+#define KMA_R_OWN 3u    /* take a superblock without the class slot */
+#define KMA_R_WAIT 4u   /* another refill is in progress */
 
 } /* namespace kma_detail */
 
@@ -1023,79 +923,237 @@ __device__ inline void *kma_malloc_warp(kma_heap *h, size_t size, kma_tally *tl 
 	using namespace kma_detail;
 	const uint32_t active = __activemask();
 	const uint32_t lane = lane_id();
-	int c = kma_class_of(h, size);
-	uint32_t peers = __match_any_sync(active, c);
-	uint32_t leader = __ffs(peers) - 1;
-	uint32_t rank = __popc(peers & lanemask_lt());
-	uint32_t gsize = __popc(peers);
-	bool need = c >= 0;
+	const int cls = kma_class_of(h, size);
+	const uint32_t peers = __match_any_sync(active, cls);
+	const uint32_t leader = __ffs(peers) - 1;
+	const uint32_t rank = __popc(peers & lanemask_lt());
+	const uint32_t gsize = __popc(peers);
+	bool need = cls >= 0;
 	void *res = NULL;
 
 	/* leader-only state: the leader serves its whole group, not only itself */
+	const bool leads = lane == leader && need;
+	const uint32_t c = need ? (uint32_t)cls : 0u;
+	const uint32_t slots = __ldg(&h->cls_slots[c]);
+	const uint32_t shard = my_shard(h, c);
+	uint32_t *const clsw = cls_word(h, c, shard);
+	const uint32_t lim = h->spin_limit;
 	warp_resv r;
 	r.left = 0;
-	uint32_t served = 0;
+	uint32_t served = 0, tries = 0, empty = 0, rounds = 0;
 	bool failed = false;
-	const uint32_t lim = h->spin_limit;
-	uint32_t rounds = 0;
 
-	while (__any_sync(active, need)) {
-		/* every lane runs every iteration, so this bound ends the loop for
-		 * all of them together */
-		if (++rounds > lim) {
-			if (need) {
-				need = false;
-				set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_WARP);
-			}
-			continue;
-		}
-		uint32_t bsb = 0, bword = 0, bgot = 0, bbase = 0, bhint = 0, bfail = 0;
-		if (lane == leader && c >= 0 && served < gsize && !failed) {
+	/* Every lane runs every iteration, and each group's leader takes one step
+	 * of its own reservation in it.  The steps of different leaders are the
+	 * same instructions, or are issued before any of their results is used,
+	 * so that an iteration costs the round trips of its longest step (a
+	 * refill), not the sum over the groups.  A leader gives up, for its whole
+	 * group, after `lim` attempts at one reservation or `lim` claims that got
+	 * nothing, which ends the loop. */
+	for (; __any_sync(active, need); rounds++) {
+		const bool open = leads && served < gsize && !failed;
+		const uint32_t want = gsize - served;
+		uint32_t kind = KMA_R_NONE, cur = 0, s = 0, st = 0;
+		bool known = false;
+		/* 1. the class slot, and beside it the state of the superblock this
+		 * warp last reserved from in the class */
+		if (open && r.left == 0) {
 			tally(tl, KMA_T_ITER);
-			if (r.left == 0) {
-				if (!warp_reserve(h, (uint32_t)c, gsize - served, r, tl, hint))
-					failed = true;
+			tally(tl, KMA_T_TRY);
+			if (++tries > lim) {
+				failed = true;
+				set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RESERVE);
+			} else if (want >= slots && slots > 1) {
+				/* the group fills a whole superblock: take a fresh one
+				 * privately (it would be detached at once anyway) */
+				kind = KMA_R_OWN;
+			} else {
+				const uint32_t guess = hint ? hint[c] : 0u;
+				cur = ld_relaxed(clsw);
+				if (guess)
+					st = ld_relaxed(&h->sb_state[guess - KMA_CLS_BASE]);
+				if (guess && hint_serves(h, c, slots, want, st)) {
+					kind = KMA_R_TAKE;
+					known = true;
+					cur = guess;
+				} else if (cur == 0) {
+					/* the reference's refill under POISON (kma.cl:166-195) */
+					kind = KMA_R_LOCK;
+				} else if (cur != KMA_POISON) {
+					kind = KMA_R_TAKE;
+					known = cur == guess && st_class(st) == c && st_free(st) != 0;
+				} else if (slots <= KMA_PRIVATE_REFILL_SLOTS) {
+					/* a class with few slots per superblock: the refill in
+					 * flight yields about one group's worth, so rather than
+					 * queue behind it take a fresh superblock without the
+					 * class slot, and publish the leftover slots only if the
+					 * slot is empty by then.  Serial execution never
+					 * observes POISON. */
+					kind = KMA_R_OWN;
+				} else {
+					tally(tl, KMA_T_POISON);
+					kind = KMA_R_WAIT;
+				}
+				s = cur - KMA_CLS_BASE;
 			}
-			if (!failed) {
-				uint32_t w;
-				uint32_t hint0 = r.hint;
-				uint32_t got = warp_claim_step(h, r, w);
-				tally(tl, KMA_T_CLAIM);
-				if (!got)
-					tally(tl, KMA_T_EMPTY);
-				bsb = r.sb;
-				bword = w;
-				bgot = got;
-				bbase = served;
-				bhint = hint0;
-				served += __popc(got);
-				r.hint -= __popc(got);
-			}
-			bfail = failed;
 		}
-		bsb = __shfl_sync(active, bsb, leader);
-		bword = __shfl_sync(active, bword, leader);
-		bgot = __shfl_sync(active, bgot, leader);
-		bbase = __shfl_sync(active, bbase, leader);
-		bhint = __shfl_sync(active, bhint, leader);
-		bfail = __shfl_sync(active, bfail, leader);
+		/* 2. its state, where step 1 did not have it */
+		if (kind == KMA_R_TAKE && !known) {
+			st = ld_relaxed(&h->sb_state[s]);
+			if (st_class(st) != c || st_free(st) == 0) {
+				tally(tl, KMA_T_STALE);
+				clear_stale(clsw, cur);
+				kind = KMA_R_NONE;
+			}
+		}
+		/* 3. the reservation, with the first bitmap word the claim will visit
+		 * loaded beside it; and the locks of empty class slots */
+		uint32_t got = 0, spec = 0, t = 0;
+		if (kind == KMA_R_TAKE) {
+			t = want < st_free(st) ? want : st_free(st);
+			spec = ld_relaxed(bitmap_word(h, sb_addr(h, s), (st_free(st) - t) >> 5));
+			got = cas_relaxed(&h->sb_state[s], st, st - t);
+		}
+		if (kind == KMA_R_LOCK)
+			got = cas_relaxed(clsw, 0, KMA_POISON);
+		if (kind == KMA_R_TAKE) {
+			if (got == st) {
+				const uint32_t fr = st_free(st);
+				if (fr == t)
+					cas_relaxed(clsw, cur, 0);
+				if (hint)
+					hint[c] = cur;
+				tries = 0;
+				r.sb = s;
+				r.left = t;
+				r.cursor = fr - t; /* lowest of the t serial hints fr-1 .. fr-t */
+				r.pre = false;
+				r.kword = r.cursor >> 5;
+				r.known = spec;
+				r.hint = fr - 1;
+			} else {
+				tally(tl, KMA_T_CASFAIL);
+			}
+		}
+		if (kind == KMA_R_LOCK && got != 0)
+			kind = KMA_R_NONE;
+		/* 4. claim bits of the word at the cursor; the result is used after
+		 * the refills */
+		uint32_t pick = 0, cand = 0, old = 0, word = 0;
+		const bool claims = open && r.left && !r.pre;
+		if (claims) {
+			word = r.cursor >> 5;
+			pick = claim_pick(h, r, c, slots, cand);
+			if (pick)
+				old = bm_or(bitmap_word(h, sb_addr(h, r.sb), word), pick);
+		}
+		/* 5. refills: superblocks for all leaders that need one */
+		const bool refill = kind == KMA_R_LOCK || kind == KMA_R_OWN;
+		if (__any_sync(active, refill)) {
+			const int64_t f = sb_dequeue_lanes(h, active, refill);
+			if (refill) {
+				tally(tl, KMA_T_REFILL);
+				if (f < 0) {
+					if (kind == KMA_R_LOCK)
+						atomicExch(clsw, 0);
+					failed = true;
+				} else {
+					/* the refiller takes the top t slots, which are exactly
+					 * the hints slots-1 .. slots-t of t serial reservations */
+					t = want < slots ? want : slots;
+					sb_format(h, (uint32_t)f, c, slots - t, slots - t, shard);
+					const uint32_t pub = t == slots ? 0u : (uint32_t)f + KMA_CLS_BASE;
+					/* release: a thread that finds f in the slot must find
+					 * its bitmap and its state (a stale one would read as
+					 * full and get f detached with free slots nobody can
+					 * reach) */
+					if (kind == KMA_R_LOCK)
+						cas_release(clsw, KMA_POISON, pub);
+					else if (pub)
+						cas_release(clsw, 0, pub);
+					if (hint && pub)
+						hint[c] = pub;
+					tries = 0;
+					r.sb = (uint32_t)f;
+					r.left = t;
+					r.cursor = slots - t;
+					r.pre_hi = slots;
+					r.hint = slots - 1;
+					r.pre = true;
+					r.kword = 0xffffffffu;
+				}
+			}
+		}
+		/* 6. what was claimed: from the atomicOr of step 4, or the bits that
+		 * a refill has set already */
+		uint32_t bgot = 0;
+		const uint32_t bbase = served, bhint = r.hint;
+		if (claims) {
+			tally(tl, KMA_T_CLAIM);
+			bgot = pick & ~old;
+			if (!bgot) {
+				tally(tl, KMA_T_EMPTY);
+				if (++empty > lim) {
+					failed = true;
+					set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_WARP);
+				}
+			}
+			r.left -= __popc(bgot);
+			if (pick) {
+				r.kword = word;
+				r.known = old | pick;
+			}
+			if (bgot == pick && r.left && pick == cand) {
+				/* every candidate is ours and more are needed: move on.  What
+				 * is known of this word may predate the reservation (the
+				 * load beside it): the next visit, possibly of this same
+				 * word after a wrap, claims afresh.  An atomicOr's result
+				 * always shows at least `left` clear bits, which is what
+				 * guarantees progress. */
+				r.cursor = (word + 1) * 32;
+				if (r.cursor >= slots)
+					r.cursor = 0;
+				r.kword = 0xffffffffu;
+			}
+		} else if (leads && r.left && r.pre) {
+			/* bits [cursor, pre_hi) were set by sb_format */
+			word = r.cursor >> 5;
+			const uint32_t hi = r.pre_hi < (word + 1) * 32 ? r.pre_hi - word * 32 : 32u, lo = r.cursor & 31;
+			const uint32_t n = hi - lo;
+			bgot = (n == 32 ? 0xffffffffu : ((1u << n) - 1u)) << lo;
+			r.cursor = word * 32 + hi;
+			r.left -= n;
+			tally(tl, KMA_T_CLAIM);
+		}
+		served += __popc(bgot);
+		r.hint -= __popc(bgot);
+		/* 7. hand them out: rank j of the claim takes the j-th highest bit,
+		 * matching the serial hint order fr-1, fr-2, ... */
+		const uint32_t gsb = __shfl_sync(active, r.sb, leader);
+		const uint32_t gword = __shfl_sync(active, word, leader);
+		const uint32_t ggot = __shfl_sync(active, bgot, leader);
+		const uint32_t gbase = __shfl_sync(active, bbase, leader);
+		const uint32_t ghint = __shfl_sync(active, bhint, leader);
+		const bool gfail = __shfl_sync(active, (int)failed, leader);
 		if (need) {
-			uint32_t n = __popc(bgot);
-			if (rank >= bbase && rank < bbase + n) {
-				/* rank j of this claim takes the j-th highest claimed bit,
-				 * matching the serial hint order fr-1, fr-2, ... */
-				uint32_t j = rank - bbase;
-				uint32_t b = nth_set_bit(bgot, n - 1 - j);
-				uint32_t slot = bword * 32 + b;
-				unsigned char *p = sb_addr(h, bsb) + KMA_SB_HDR + (size_t)slot * h->cls_size[c];
-				*reinterpret_cast<uint32_t *>(p) = bhint - j;
+			const uint32_t n = __popc(ggot), j = rank - gbase;
+			if (j < n) {
+				const uint32_t slot = gword * 32 + nth_set_bit(ggot, n - 1 - j);
+				unsigned char *p = sb_addr(h, gsb) + KMA_SB_HDR + (size_t)slot * __ldg(&h->cls_size[c]);
+				*reinterpret_cast<uint32_t *>(p) = ghint - j;
 				res = p;
 				need = false;
-			} else if (bfail) {
+			} else if (gfail) {
 				need = false;
 			}
 		}
+		/* nobody got anything and somebody waits */
+		if (__any_sync(active, kind == KMA_R_WAIT) && !__any_sync(active, ggot != 0))
+			backoff(rounds);
 	}
+	/* a leader's plain stores (a refill's bitmap and state) before its peers'
+	 * use of the blocks */
+	__syncwarp(active);
 	return res;
 }
 
