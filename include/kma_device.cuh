@@ -26,8 +26,9 @@
  * Class table (kma.h:84): each class c has cls_nsh[c] words ("shards"),
  * each 0 (empty), 1 (POISON, refill in progress) or s+2 (superblock s is
  * that shard's current superblock for class c), every one on its own
- * 128-byte line.  A warp uses shard (global warp id) % cls_nsh[c], so one
- * thread of warp 0 -- a serial replay -- always uses shard 0; a heap with
+ * 128-byte line.  A warp uses shard (global warp id) % cls_nsh[c] (its
+ * per-thread calls: thread_shard), so one thread of warp 0, lane 0 -- a
+ * serial replay -- always uses shard 0; a heap with
  * one shard per class is the reference's single table.  Only a shard's
  * current superblock is contended, so kma_create gives every class
  * pages/32 shards (at most 2048): enough to spread a full GPU's warps,
@@ -86,7 +87,6 @@
 #define KMA_ERR_AT_RING_DEQ (1u << 11)  /* ring: slot not yet filled */
 #define KMA_ERR_AT_CLAIM (1u << 12)     /* plain malloc: bitmap claim */
 #define KMA_ERR_AT_MALLOC (1u << 13)    /* plain malloc: reservation */
-#define KMA_ERR_AT_FREE (1u << 14)      /* plain free: count update */
 #define KMA_ERR_AT_RESERVE (1u << 15)   /* warp malloc: reservation (POISON / stale waits) */
 #define KMA_ERR_AT_WARP (1u << 16)      /* warp malloc: leader turns */
 
@@ -344,6 +344,9 @@ __device__ __forceinline__ unsigned long long tw_make(uint32_t tag, uint32_t idx
 	return ((unsigned long long)tag << 32) | idx;
 }
 
+/* (Plain loads of the geometry: through the read-only path the compiler
+ * keeps more of it in registers across a call, and the batched form measured
+ * 39.1 ms instead of 37.7 for 64 jobs, spills and all.) */
 __device__ __forceinline__ unsigned char *sb_addr(const kma_heap *h, uint32_t s)
 {
 	return h->sb_base + ((size_t)s << h->sb_log2);
@@ -363,11 +366,22 @@ __device__ __forceinline__ unsigned long long global_warp()
 }
 __device__ __forceinline__ uint32_t my_shard(const kma_heap *h, uint32_t c)
 {
-	const uint32_t n = __ldg(&h->cls_nsh[c]);
+	const uint32_t n = h->cls_nsh[c];
 	const unsigned long long w = global_warp();
 	/* a 64-bit remainder is some hundred instructions: only for grids of
 	 * 2^32 warps and more */
 	return (w >> 32) ? (uint32_t)(w % n) : (uint32_t)w % n;
+}
+/* The shard of a per-thread call.  Lanes that reserve each for itself collide
+ * on one superblock's count, so a warp spreads over eight shards, lane % 8:
+ * config 2's program per thread (24 rounds, 300 / 50021 / 250000 items) took
+ * 0.80 / 1.13 / 3.06 ms, with one shard a warp 1.24 / 1.23 / 3.12, with one a
+ * lane 0.67 / 1.10 / 3.67 (a full GPU's lanes then touch as many lines). */
+__device__ __forceinline__ uint32_t thread_shard(const kma_heap *h, uint32_t c)
+{
+	const uint32_t n = h->cls_nsh[c];
+	const unsigned long long t = global_warp() * 8 + lane_id() % 8;
+	return (t >> 32) ? (uint32_t)(t % n) : (uint32_t)t % n;
 }
 __device__ __forceinline__ uint32_t *cls_word(kma_heap *h, uint32_t c, uint32_t shard)
 {
@@ -387,11 +401,11 @@ __device__ __forceinline__ uint32_t *cls_word(kma_heap *h, uint32_t c, uint32_t 
  * class 0, which is what a zero-initialised reference build returns. */
 __device__ __forceinline__ int kma_class_of(const kma_heap *h, size_t size)
 {
-	if (size > __ldg(&h->max_request))
+	if (size > h->max_request)
 		return -1;
 	uint32_t s = (uint32_t)size;
 	int c = s < 4 ? 0 : (int)(29 - __clz(s)); /* floor(log2 s) - 2 */
-	while (__ldg(&h->cls_size[c]) < s)
+	while (h->cls_size[c] < s)
 		c++;
 	return c;
 }
@@ -459,26 +473,29 @@ __device__ __forceinline__ int64_t msq_dequeue(kma_heap *h)
  * enqueue with ticket p".  ring_avail counts completed enqueues not yet
  * claimed by a dequeue; a dequeue needs two (one stays behind, as the
  * reference's dummy does).  The ring carries only superblock numbers: the
- * enqueuer publishes with a release store (ordering its detach of the
- * superblock first), and everything a dequeuer then writes is addressed
- * through the number it read, so tickets, counts and the slot read are
- * relaxed; a count seen before its slot store only makes a dequeuer wait
+ * enqueuer stores one after its detach of the superblock has returned
+ * (ring_put), and everything a dequeuer then writes is addressed
+ * through the number it read, so tickets, counts and slots are relaxed; a
+ * count seen before its slot store only makes a dequeuer wait
  * on the slot's sequence number. */
 /* ticket -> slot: as the 64-bit remainder, which only tickets past 2^32 take */
 __device__ __forceinline__ uint32_t ring_slot(unsigned long long pos, uint32_t cap)
 {
 	return (pos >> 32) ? (uint32_t)(pos % cap) : (uint32_t)pos % cap;
 }
-__device__ __forceinline__ int ring_enqueue(kma_heap *h, uint32_t s)
+/* Put superblock s into the slot of tail ticket `pos`.  detached: the value
+ * an atomic that detached s returned.  It must have returned before s can be
+ * handed out again (a late clearing of s's old class slot would hit its next
+ * incarnation); the store waits for it by using it -- no class slot holds
+ * 0xffffffff -- where a release store would wait out a fence. */
+__device__ __forceinline__ int ring_put(kma_heap *h, unsigned long long pos, uint32_t s, uint32_t detached)
 {
-	unsigned long long pos = add64_relaxed(&h->free_tail.v, 1ull);
-	unsigned long long *slot = &h->ring[ring_slot(pos, __ldg(&h->ring_cap))];
+	unsigned long long *slot = h->ring + ring_slot(pos, h->ring_cap);
 	uint32_t lim = h->spin_limit;
 	for (uint32_t it = 0; it < lim; it++) {
 		unsigned long long w = ld_relaxed64(slot);
-		if ((uint32_t)(w >> 32) == (uint32_t)pos) {
-			st_release64(slot, ((unsigned long long)(uint32_t)(pos + 1) << 32) | s);
-			atomicAdd(&h->ring_avail.v, 1u);
+		if ((uint32_t)(w >> 32) == (uint32_t)pos && detached != 0xffffffffu) {
+			st_relaxed64(slot, ((unsigned long long)(uint32_t)(pos + 1) << 32) | s);
 			return 1;
 		}
 		backoff(it);
@@ -486,12 +503,31 @@ __device__ __forceinline__ int ring_enqueue(kma_heap *h, uint32_t s)
 	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RING_ENQ);
 	return 0;
 }
+__device__ __forceinline__ void ring_enqueue(kma_heap *h, uint32_t s, uint32_t detached)
+{
+	if (ring_put(h, add64_relaxed(&h->free_tail.v, 1ull), s, detached))
+		atomicAdd(&h->ring_avail.v, 1u);
+}
+/* The calling lanes (`active`) that `want` to put theirs take tickets
+ * together.  Every lane of `active` calls. */
+__device__ __forceinline__ void ring_enqueue_lanes(kma_heap *h, uint32_t active, bool want, uint32_t s,
+		uint32_t detached)
+{
+	const uint32_t m = __ballot_sync(active, want);
+	const uint32_t first = __ffs(m) - 1;
+	unsigned long long pos = 0;
+	if (lane_id() == first)
+		pos = add64_relaxed(&h->free_tail.v, (unsigned long long)__popc(m));
+	pos = __shfl_sync(active, pos, first) + __popc(m & lanemask_lt());
+	if (want && ring_put(h, pos, s, detached))
+		atomicAdd(&h->ring_avail.v, 1u);
+}
 
 /* the superblock of head ticket `pos` (claimed against ring_avail) */
 __device__ __forceinline__ int64_t ring_take(kma_heap *h, unsigned long long pos)
 {
-	const uint32_t cap = __ldg(&h->ring_cap);
-	unsigned long long *slot = &h->ring[ring_slot(pos, cap)];
+	const uint32_t cap = h->ring_cap;
+	unsigned long long *slot = h->ring + ring_slot(pos, cap);
 	uint32_t lim = h->spin_limit;
 	for (uint32_t it = 0; it < lim; it++) {
 		unsigned long long w = ld_relaxed64(slot);
@@ -562,10 +598,6 @@ __device__ __forceinline__ int64_t ring_dequeue_lanes(kma_heap *h, uint32_t acti
 	return ring_take(h, pos + rank);
 }
 
-__device__ __forceinline__ int sb_enqueue(kma_heap *h, uint32_t s)
-{
-	return (h->flags & KMA_HEAP_RING) ? ring_enqueue(h, s) : msq_enqueue(h, s);
-}
 __device__ __forceinline__ int64_t sb_dequeue(kma_heap *h)
 {
 	return (h->flags & KMA_HEAP_RING) ? ring_dequeue(h) : msq_dequeue(h);
@@ -639,8 +671,10 @@ __device__ __forceinline__ void clear_stale(uint32_t *clsw, uint32_t cur)
 }
 
 /* kma.cl:232-273: claim a bitmap bit at or above `hint` (wrapping),
- * write the hint into word 0 of the block. */
-__device__ __forceinline__ void *sb_get_block(kma_heap *h, uint32_t s, uint32_t c, uint32_t hint)
+ * write the hint into word 0 of the block.  v: the hint's bitmap word as the
+ * caller has seen it, perhaps before its reservation: bits that look free
+ * are tried first, and the atomicOr decides. */
+__device__ __forceinline__ void *sb_get_block(kma_heap *h, uint32_t s, uint32_t c, uint32_t hint, uint32_t v)
 {
 	unsigned char *sb = sb_addr(h, s);
 	uint32_t slots = h->cls_slots[c];
@@ -651,7 +685,8 @@ __device__ __forceinline__ void *sb_get_block(kma_heap *h, uint32_t s, uint32_t 
 	for (uint32_t it = 0; it < lim; it++) {
 		uint32_t k = slot >> 5;
 		uint32_t *wp = bitmap_word(h, sb, k);
-		uint32_t v = ld_relaxed(wp);
+		if (it)
+			v = ld_relaxed(wp);
 		uint32_t valid = (k == words - 1 && (slots & 31)) ? ((1u << (slots & 31)) - 1u) : 0xffffffffu;
 		uint32_t cand = ~v & valid & (0xffffffffu << (slot & 31));
 		while (cand) {
@@ -674,6 +709,38 @@ __device__ __forceinline__ void *sb_get_block(kma_heap *h, uint32_t s, uint32_t 
 	return NULL;
 }
 
+/* The free list is empty: one slot of class c from the current superblock of
+ * one of the next shards, or NULL.  A warp's per-thread calls spread over
+ * eight shards, so the slots that are left are spread too: without a look at
+ * the neighbours a heap of 224 MiB that just held 60 k items' blocks refused
+ * 100 of 600 k requests.  A thread alone fills no other shard than its own,
+ * so serial replay is unchanged. */
+#define KMA_STEAL_SHARDS 64u
+static __device__ __noinline__ void *steal_block(kma_heap *h, uint32_t c, uint32_t shard)
+{
+	const uint32_t n = h->cls_nsh[c];
+	for (uint32_t i = 1; i < n && i <= KMA_STEAL_SHARDS; i++) {
+		uint32_t *clsw = cls_word(h, c, (shard + i) % n);
+		const uint32_t cur = ld_relaxed(clsw);
+		if (cur < KMA_CLS_BASE)
+			continue;
+		const uint32_t s = cur - KMA_CLS_BASE;
+		for (uint32_t tries = 0; tries < 4; tries++) {
+			const uint32_t st = ld_relaxed(&h->sb_state[s]);
+			if (st_class(st) != c || st_free(st) == 0)
+				break;
+			const uint32_t fr = st_free(st) - 1;
+			const uint32_t v = ld_relaxed(bitmap_word(h, sb_addr(h, s), fr >> 5));
+			if (cas_relaxed(&h->sb_state[s], st, st - 1) != st)
+				continue;
+			if (fr == 0)
+				cas_relaxed(clsw, cur, 0);
+			return sb_get_block(h, s, c, fr, v);
+		}
+	}
+	return NULL;
+}
+
 } /* namespace kma_detail */
 
 /* kma.cl:279-303 (with _kma_reserve_block, kma.cl:150-225) */
@@ -683,18 +750,21 @@ __device__ inline void *kma_malloc(kma_heap *h, size_t size)
 	int c = kma_class_of(h, size);
 	if (c < 0)
 		return NULL;
-	uint32_t shard = my_shard(h, (uint32_t)c);
+	uint32_t shard = thread_shard(h, (uint32_t)c);
 	uint32_t *clsw = cls_word(h, (uint32_t)c, shard);
 	uint32_t lim = h->spin_limit;
 	for (uint32_t it = 0; it < lim; it++) {
-		/* kma.cl:163: CAS 0 -> POISON doubles as the read of the slot */
-		uint32_t cur = cas_relaxed(clsw, 0, KMA_POISON);
+		/* kma.cl:163 reads the slot with its CAS 0 -> POISON; here only an
+		 * empty one is CASed, so that threads on one slot do not queue */
+		uint32_t cur = ld_relaxed(clsw);
 		if (cur == 0) {
+			if (cas_relaxed(clsw, 0, KMA_POISON) != 0)
+				continue;
 			/* refill, kma.cl:166-195 */
 			int64_t s = sb_dequeue(h);
 			if (s < 0) {
 				atomicExch(clsw, 0);
-				return NULL;
+				return s == -1 ? steal_block(h, (uint32_t)c, shard) : NULL;
 			}
 			uint32_t slots = h->cls_slots[c];
 			sb_format(h, (uint32_t)s, c, slots, slots - 1, shard);
@@ -704,7 +774,7 @@ __device__ inline void *kma_malloc(kma_heap *h, size_t size)
 			 * block is freed (kma.cl:203-204).  Leave the class empty
 			 * instead, which is what taking the last slot does. */
 			cas_release(clsw, KMA_POISON, slots == 1 ? 0u : (uint32_t)s + KMA_CLS_BASE);
-			return sb_get_block(h, (uint32_t)s, c, slots - 1);
+			return sb_get_block(h, (uint32_t)s, c, slots - 1, 0u);
 		}
 		if (cur == KMA_POISON) {
 			backoff(it);
@@ -712,18 +782,19 @@ __device__ inline void *kma_malloc(kma_heap *h, size_t size)
 		}
 		uint32_t s = cur - KMA_CLS_BASE;
 		uint32_t *stp = &h->sb_state[s];
-		/* kma.cl:198 reads the state with atom_add(.., 0) */
-		uint32_t st = atomicAdd(stp, 0u);
+		uint32_t st = ld_relaxed(stp); /* kma.cl:198: atom_add(.., 0) */
 		if (st_class(st) != (uint32_t)c || st_free(st) == 0) {
 			clear_stale(clsw, cur);
 			continue;
 		}
 		uint32_t fr = st_free(st) - 1;
+		/* the hint's bitmap word beside the reservation, not after it */
+		const uint32_t v = ld_relaxed(bitmap_word(h, sb_addr(h, s), fr >> 5));
 		if (cas_relaxed(stp, st, st - 1) != st)
 			continue;
 		if (fr == 0)
 			cas_relaxed(clsw, cur, 0); /* kma.cl:216-218 */
-		return sb_get_block(h, s, c, fr);
+		return sb_get_block(h, s, c, fr, v);
 	}
 	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_MALLOC);
 	return NULL;
@@ -747,22 +818,34 @@ __device__ __forceinline__ bool block_locate(const kma_heap *h, const void *p, u
 	return slot < h->cls_slots[c];
 }
 
-/* Return superblock s (class c) to the free list once all its slots are
- * free: kma.cl:362-367. */
-__device__ __forceinline__ void sb_recycle(kma_heap *h, uint32_t s, uint32_t c)
+/* Return superblock s (class c, state word `full`: every slot free) to the
+ * free list unless a reservation gets in first: kma.cl:350-367.  The lanes
+ * of `active` that have one do it together; every lane of it calls.
+ *
+ * The home shard of this incarnation was stored before its class slot, and
+ * so before any block of it was handed out; a gpu-scope relaxed load issued
+ * after the count that made it full is served at L2, where that store
+ * already was.  A plain load may be served from this SM's L1, where a line
+ * of sb_home read during an earlier incarnation can still sit: the slot of
+ * the old home would be cleared and the current one left naming a superblock
+ * on the free list. */
+__device__ __forceinline__ void sb_recycle(kma_heap *h, uint32_t active, bool all_free, uint32_t s, uint32_t c,
+		uint32_t full)
 {
-	/* The home shard of this incarnation was stored before the release
-	 * that published its state (sb_format).  This load issues only after
-	 * the caller's CAS on that state has returned (it decides whether to
-	 * recycle), and a gpu-scope relaxed load is served at L2, where that
-	 * store already was: it sees the current home.  A plain load may be
-	 * served from this SM's L1, where a line of sb_home read during an
-	 * earlier incarnation can still sit: the slot of the old home would be
-	 * cleared and the current one left naming a superblock on the free
-	 * list. */
-	uint32_t home = ld_relaxed16(&h->sb_home[s]);
-	cas_relaxed(cls_word(h, c, home), s + KMA_CLS_BASE, 0);
-	sb_enqueue(h, s);
+	uint32_t home = 0, seen = 0, old = 0;
+	if (all_free) {
+		home = ld_relaxed16(&h->sb_home[s]);
+		seen = cas_relaxed(&h->sb_state[s], full, st_make(c, st_slots(full), 0));
+	}
+	const bool mine = all_free && seen == full;
+	if (!__any_sync(active, mine))
+		return;
+	if (mine)
+		old = cas_relaxed(cls_word(h, c, home), s + KMA_CLS_BASE, 0);
+	if (h->flags & KMA_HEAP_RING)
+		ring_enqueue_lanes(h, active, mine, s, old);
+	else if (mine)
+		msq_enqueue(h, s);
 }
 } /* namespace kma_detail */
 
@@ -810,21 +893,12 @@ __device__ inline void kma_free(kma_heap *h, void *p)
 		set_err(h, KMA_ERR_BADFREE); /* a concurrent double free */
 		return;
 	}
-	uint32_t *stp = &h->sb_state[s];
-	uint32_t lim = h->spin_limit;
-	for (uint32_t it = 0; it < lim; it++) {
-		uint32_t st = atomicAdd(stp, 0u); /* kma.cl:343 */
-		uint32_t slots = st_slots(st);
-		uint32_t fr = st_free(st) + 1;
-		bool enq = fr == slots;
-		uint32_t nst = st_make(st_class(st), slots, enq ? 0 : fr);
-		if (cas_relaxed(stp, st, nst) == st) {
-			if (enq)
-				sb_recycle(h, s, c);
-			return;
-		}
-	}
-	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_FREE);
+	/* kma.cl:343-367 re-reads and CASes the count until it fits; an add
+	 * cannot miss, and lanes that free into one superblock need not queue */
+	const uint32_t full = atomicAdd(&h->sb_state[s], 1u) + 1u;
+	const bool all_free = st_free(full) == st_slots(full);
+	const uint32_t active = __activemask();
+	sb_recycle(h, active, all_free, s, c, full);
 }
 
 /* ------------------------------------------------------------------ */
@@ -883,7 +957,7 @@ struct warp_resv {
 __device__ __forceinline__ bool hint_serves(const kma_heap *h, uint32_t c, uint32_t slots, uint32_t want, uint32_t st)
 {
 	const uint32_t fr = st_free(st);
-	return st_class(st) == c && fr >= want && (__ldg(&h->cls_words[c]) <= 2 || fr * 4 >= slots);
+	return st_class(st) == c && fr >= want && (h->cls_words[c] <= 2 || fr * 4 >= slots);
 }
 
 /* The bits of bitmap word `word` that reservation r takes next, given what
@@ -914,9 +988,11 @@ __device__ __forceinline__ uint32_t claim_pick(const kma_heap *h, const warp_res
 
 /* hint (optional): this warp's KMA_MAX_CLASSES words, zeroed once, best
  * in shared memory; the warp's leaders remember there, per class, the
- * superblock they last reserved from, and load its state together with
- * the class word on the next call.  Only a speed hint: any content is
- * safe, a stale one costs the dependent load it would have saved. */
+ * superblock they last reserved from.  Its state is loaded together with the
+ * class word on the next call, and if it still serves the request it is
+ * reserved from, current or not (hint_serves): the class slot does not get
+ * back a detached superblock whose blocks are freed one by one.  Any earlier
+ * content is safe, as a reservation's CAS checks class and count. */
 __device__ inline void *kma_malloc_warp(kma_heap *h, size_t size, kma_tally *tl = nullptr,
 		uint32_t *hint = nullptr)
 {
@@ -934,7 +1010,7 @@ __device__ inline void *kma_malloc_warp(kma_heap *h, size_t size, kma_tally *tl 
 	/* leader-only state: the leader serves its whole group, not only itself */
 	const bool leads = lane == leader && need;
 	const uint32_t c = need ? (uint32_t)cls : 0u;
-	const uint32_t slots = __ldg(&h->cls_slots[c]);
+	const uint32_t slots = h->cls_slots[c];
 	const uint32_t shard = my_shard(h, c);
 	uint32_t *const clsw = cls_word(h, c, shard);
 	const uint32_t lim = h->spin_limit;
@@ -1139,7 +1215,7 @@ __device__ inline void *kma_malloc_warp(kma_heap *h, size_t size, kma_tally *tl 
 			const uint32_t n = __popc(ggot), j = rank - gbase;
 			if (j < n) {
 				const uint32_t slot = gword * 32 + nth_set_bit(ggot, n - 1 - j);
-				unsigned char *p = sb_addr(h, gsb) + KMA_SB_HDR + (size_t)slot * __ldg(&h->cls_size[c]);
+				unsigned char *p = sb_addr(h, gsb) + KMA_SB_HDR + (size_t)slot * h->cls_size[c];
 				*reinterpret_cast<uint32_t *>(p) = ghint - j;
 				res = p;
 				need = false;
@@ -1170,8 +1246,10 @@ __device__ inline void kma_free_warp(kma_heap *h, void *p)
 			set_err(h, KMA_ERR_BADFREE);
 	}
 	/* 1) clear bitmap bits: one atomicAnd per (superblock, word) */
-	uint32_t word = valid ? (slot >> 5) : 0xffffffffu;
-	unsigned long long key = ((unsigned long long)s << 32) | word;
+	uint32_t word = slot >> 5;
+	/* (a superblock of SB bytes has at most SB / 128 bitmap words, and a
+	 * heap 2^31 of them: 256 GiB) */
+	const uint32_t key = valid ? (s << (h->sb_log2 - 7)) | word : 0xffffffffu;
 	uint32_t wpeers = __match_any_sync(active, key);
 	uint32_t bit = valid ? (1u << (slot & 31)) : 0u;
 	uint32_t mask = __reduce_or_sync(wpeers, bit);
@@ -1207,18 +1285,15 @@ __device__ inline void kma_free_warp(kma_heap *h, void *p)
 	uint32_t speers = __match_any_sync(active, good ? s : 0xffffffffu);
 	uint32_t k = __popc(speers);
 	uint32_t sleader = __ffs(speers) - 1;
+	uint32_t full = 0;
+	bool all_free = false;
 	if (good && lane == sleader) {
-		uint32_t *stp = &h->sb_state[s];
-		uint32_t prev = atomicAdd(stp, k);
-		uint32_t slots = st_slots(prev);
-		if (st_free(prev) + k == slots) {
-			/* kma.cl:350-367: all free -- free count 0 and recycle, unless
-			 * a reservation got in first */
-			uint32_t full = prev + k;
-			if (cas_relaxed(stp, full, st_make(st_class(prev), slots, 0)) == full)
-				sb_recycle(h, s, c);
-		}
+		full = atomicAdd(&h->sb_state[s], k) + k;
+		all_free = st_free(full) == st_slots(full);
 	}
+	/* 3) kma.cl:350-367: all free -- recycle */
+	if (__any_sync(active, all_free))
+		sb_recycle(h, active, all_free, s, c, full);
 }
 
 #endif /* KMA_DEVICE_CUH */

@@ -127,3 +127,24 @@ def test_gpu_batch_on_pma(mode):
         assert p.head() == st["fill_bytes"]
         with pytest.raises(Exception):
             b.run(block_dim=256, cache_depth=2)  # the warp cache needs KMA size classes
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 1], ids=["plain", "warp"])
+@pytest.mark.parametrize("sb_log2,mib", [(12, 64), (14, 96), (16, 160)])
+def test_gpu_batch_exhausted_heap(sb_log2, mib, mode):
+    """A heap too small for the jobs' live blocks: requests are refused, and
+    the rest -- slots taken from neighbouring shards, superblocks reserved
+    from again after they left their class slot -- stay sound."""
+    from kma_b200 import Heap
+    from kma_b200.batch import Batch
+    seeds = list(range(401, 401 + len(SMALL_THREADS)))
+    with Heap((mib << 20) >> sb_log2, sb_log2) as h, \
+            Batch(h, SMALL_THREADS, seeds, rounds=12, mode=mode) as b:
+        for _ in range(2):
+            b.run(block_dim=256, cache_depth=0)
+            st = b.stats()
+            assert st["nulls"] > st["refused"]
+            assert st["bad_tags"] == 0 and st["mallocs"] == sum(SMALL_THREADS) * 12
+            assert st["frees"] == st["mallocs"] - st["nulls"]
+            _check_empty(h)
