@@ -57,74 +57,76 @@ __device__ __forceinline__ void pl_st(T *p, T v)
 	*p = v;
 #endif
 }
-/* Tag fill of this lane's own block (p may be NULL).  Blocks start 4 bytes
- * past a 16-byte boundary (12 + slot*size), so the head words go one at a
- * time and the rest as 16-byte stores. */
+/* Blocks of at least this many bytes are filled by the whole warp, one row of
+ * consecutive 16-byte stores after the other; below, a lane's own loop is
+ * shorter than the shuffles.  A loop of its own for every block (a warp's
+ * largest decides how long) took 3.16 instead of 2.81 ms for 24 jobs on the
+ * bump heap and 7.77 instead of 7.49 for config 2; from 128 / 256 / 1024 bytes
+ * up config 2 took 7.52 / 7.47 / 7.48 ms, the per-thread program of 50021
+ * items 1.80 / 1.74 / 1.67 (1.70 at 512). */
+#ifndef WL_FILL_BYTES
+#define WL_FILL_BYTES 512u
+#endif
+/* Tag fill of every calling lane's block (p may be NULL). */
 __device__ __forceinline__ void coop_fill(uint32_t mask, uint32_t lane, void *p, uint32_t n, uint32_t tag)
 {
-	(void)mask;
-	(void)lane;
-	if (!p)
-		return;
 	uint32_t *w = (uint32_t *)p;
-	uint32_t nw = n >> 2, i = 0;
-	while (i < nw && ((uintptr_t)(w + i) & 15))
-		pl_st(&w[i++], tag);
-	uint32_t nv = (nw - i) >> 2;
-	uint4 *v = reinterpret_cast<uint4 *>(w + i);
-	const uint4 t4 = make_uint4(tag, tag, tag, tag);
-#pragma unroll 4
-	for (uint32_t k = 0; k < nv; k++)
-		pl_st(&v[k], t4);
-	for (i += nv * 4; i < nw; i++)
-		pl_st(&w[i], tag);
-}
-
-/* Blocks of at least this many bytes are verified by the whole warp
- * (config 2's rounds kernel: 128 and 256 measured alike, 512 2% slower). */
-#ifndef WL_COOP_BYTES
-#define WL_COOP_BYTES 256u
-#endif
-
-/* The share of the r-th of `width` calling lanes in verifying block p (nw
- * words) cooperatively: head words up to the 16-byte boundary, 16-byte
- * vectors r, r+width, ..., and tail words.  Nonzero if its share differs
- * from the tag. */
-__device__ __forceinline__ uint32_t verify_share(uint32_t r, uint32_t width, const uint32_t *p, uint32_t nw,
-		uint32_t tag)
-{
+	const bool big = p && n >= WL_FILL_BYTES;
+	const uint32_t nw = p ? n >> 2 : 0u;
 	uint32_t head = (uint32_t)((16u - ((uintptr_t)p & 15u)) & 15u) >> 2;
 	head = head < nw ? head : nw;
-	uint32_t nv = (nw - head) >> 2;
-	uint32_t tail = nw - head - 4 * nv;
-	const uint4 *v = reinterpret_cast<const uint4 *>(p + head);
-	uint32_t bad = 0;
-#pragma unroll 4
-	for (uint32_t k = r; k < nv; k += width) {
-		uint4 x = pl_ld(&v[k]);
-		bad |= (x.x ^ tag) | (x.y ^ tag) | (x.z ^ tag) | (x.w ^ tag);
+	const uint32_t nv = (nw - head) >> 2, t0 = head + 4 * nv;
+	uint4 *v = reinterpret_cast<uint4 *>(w + head);
+	const uint4 t4 = make_uint4(tag, tag, tag, tag);
+#pragma unroll
+	for (uint32_t i = 0; i < 3; i++) {
+		if (i < head)
+			pl_st(&w[i], tag);
+		if (t0 + i < nw)
+			pl_st(&w[t0 + i], tag);
 	}
-	for (uint32_t i = r; i < head; i += width)
-		bad |= pl_ld(&p[i]) ^ tag;
-	for (uint32_t i = r; i < tail; i += width)
-		bad |= pl_ld(&p[head + 4 * nv + i]) ^ tag;
-	return bad;
+	const uint32_t own = big ? 0u : nv;
+#pragma unroll 4
+	for (uint32_t k = 0; k < own; k++)
+		pl_st(&v[k], t4);
+	const uint32_t width = __popc(mask), rank = __popc(mask & ((1u << lane) - 1u));
+	for (uint32_t mb = __ballot_sync(mask, big); mb; mb &= mb - 1) {
+		const uint32_t j = __ffs(mb) - 1;
+		uint4 *vj = (uint4 *)__shfl_sync(mask, (unsigned long long)v, j) + rank;
+		const uint32_t nj = __shfl_sync(mask, nv, j), t = __shfl_sync(mask, tag, j);
+		const uint4 tj = make_uint4(t, t, t, t);
+#pragma unroll 4
+		for (uint32_t k = rank; k < nj; k += width, vj += width)
+			pl_st(vj, tj);
+	}
 }
 
-/* Vectors each lane has in flight per batch of coop_verify_rows.  With the
- * streaming payload hints, config 2's rounds kernel (64 registers)
- * measured 7.78 / 7.93 / 8.14 / 8.13 ms per launch at 3 / 2 / 1 / 4, and
- * 8.32 ms block by block (0): deeper batches cost more spills than they
- * hide latency. */
+/* Blocks of at least this many bytes are verified by the whole warp (64 jobs:
+ * 35.1 ms at 128, 35.6 at 256, 36.9 at 512; config 2 within 1%). */
+#ifndef WL_COOP_BYTES
+#define WL_COOP_BYTES 128u
+#endif
+
+/* Vectors each lane has in flight per batch of coop_verify: config 2
+ * (64 registers) took 6.58 / 6.53 / 6.83 / 6.96 ms at 2 / 3 / 4 / 5; deeper
+ * batches cost more spills than they hide latency. */
 #ifndef WL_VERIFY_SLOTS
 #define WL_VERIFY_SLOTS 3
+#endif
+/* Vectors of its own small block that a lane has in flight, beside the words
+ * before and after them: 6.86 / 6.53 / 6.74 ms at 2 / 4 / 5. */
+#ifndef WL_SMALL_SLOTS
+#define WL_SMALL_SLOTS 4
 #endif
 
 /* Verify every lane's block (p may be NULL) against its tag; true in the
  * owner lane of a block with a word that differs.  Every lane of `mask`
  * calls it.
  *
- * Small blocks: the owner reads its own, 16-byte loads unrolled by eight.
+ * Small blocks, and the few words of any block before and after its 16-byte
+ * aligned body: the owner reads its own, every load issued before the first
+ * is compared (word by word and vector by vector, a lane with 64 bytes had
+ * * eleven round trips in a row).
  * Blocks of WL_COOP_BYTES or more: their 16-byte aligned bodies are cut
  * into rows of one vector per calling lane, rows of all big blocks laid
  * end to end in lane order; the r-th calling lane reads vector r of each
@@ -134,11 +136,8 @@ __device__ __forceinline__ uint32_t verify_share(uint32_t r, uint32_t width, con
  * blocks costs one memory round trip per batch rather than one per block
  * (a loop over blocks consumes each block's loads before it can issue the
  * next block's).  The row schedule is the same in every lane, so which
- * block a row belongs to, its base and its tag are broadcast by shuffles;
- * the owner of a big block reads its head and tail words (the few before
- * and after the aligned body) along with the small blocks. */
-#if WL_VERIFY_SLOTS > 0
-__device__ __forceinline__ bool coop_verify_rows(uint32_t mask, uint32_t lane, const void *p, uint32_t n,
+ * block a row belongs to, its base and its tag are broadcast by shuffles. */
+__device__ __forceinline__ bool coop_verify(uint32_t mask, uint32_t lane, const void *p, uint32_t n,
 		uint32_t tag)
 {
 	const uint32_t *w = (const uint32_t *)p;
@@ -149,19 +148,33 @@ __device__ __forceinline__ bool coop_verify_rows(uint32_t mask, uint32_t lane, c
 	const uint32_t nv = (nw - head) >> 2;
 	uint32_t bad = 0;
 	if (p) {
-		/* head words, then (small blocks) the body, then tail words */
-		for (uint32_t i = 0; i < head; i++)
-			bad |= pl_ld(&w[i]) ^ tag;
-		if (!big) {
-			const uint4 *v = reinterpret_cast<const uint4 *>(w + head);
-#pragma unroll 8
-			for (uint32_t k = 0; k < nv; k++) {
-				uint4 x = pl_ld(&v[k]);
-				bad |= (x.x ^ tag) | (x.y ^ tag) | (x.z ^ tag) | (x.w ^ tag);
-			}
+		/* head and tail words and (small blocks) the body, four vectors at a
+		 * time: every load is issued before the first is compared */
+		const uint4 *v = reinterpret_cast<const uint4 *>(w + head);
+		const uint32_t t0 = head + 4 * nv, own = big ? 0u : nv;
+		uint32_t e[6];
+		uint4 x[WL_SMALL_SLOTS];
+#pragma unroll
+		for (uint32_t i = 0; i < 3; i++) {
+			e[i] = i < head ? pl_ld(&w[i]) : tag;
+			e[3 + i] = t0 + i < nw ? pl_ld(&w[t0 + i]) : tag;
 		}
-		for (uint32_t i = head + 4 * nv; i < nw; i++)
-			bad |= pl_ld(&w[i]) ^ tag;
+		uint32_t k = 0;
+		do {
+#pragma unroll
+			for (uint32_t i = 0; i < WL_SMALL_SLOTS; i++) {
+				x[i] = make_uint4(tag, tag, tag, tag);
+				if (k + i < own)
+					x[i] = pl_ld(&v[k + i]);
+			}
+#pragma unroll
+			for (uint32_t i = 0; i < WL_SMALL_SLOTS; i++)
+				bad |= (x[i].x ^ tag) | (x[i].y ^ tag) | (x[i].z ^ tag) | (x[i].w ^ tag);
+			k += WL_SMALL_SLOTS;
+		} while (k < own);
+#pragma unroll
+		for (uint32_t i = 0; i < 6; i++)
+			bad |= e[i] ^ tag;
 	}
 	uint32_t mb = __ballot_sync(mask, big);
 	uint32_t badbits = 0;
@@ -206,60 +219,6 @@ __device__ __forceinline__ bool coop_verify_rows(uint32_t mask, uint32_t lane, c
 	}
 	badbits = __reduce_or_sync(mask, badbits);
 	return bad != 0 || ((badbits >> lane) & 1u);
-}
-#endif
-
-/* Verify every lane's block (p may be NULL) against its tag; true in the
- * owner lane of a block with a word that differs.  Small blocks: each lane
- * reads its own with 16-byte loads unrolled by eight.  Blocks of
- * WL_COOP_BYTES or more: the calling lanes read each together, block by
- * block (each block's loads are consumed before the next block's are
- * issued).  coop_verify's fallback when WL_VERIFY_SLOTS is 0; with the
- * streaming payload hints the row batches measured faster in both the
- * config-2 rounds kernel and the batched form (3737 vs 3633 M ops/s). */
-__device__ __forceinline__ bool coop_verify_blockwise(uint32_t mask, uint32_t lane, const void *p, uint32_t n,
-		uint32_t tag)
-{
-	const uint32_t *w = (const uint32_t *)p;
-	const bool big = p && n >= WL_COOP_BYTES;
-	uint32_t bad = 0;
-	if (p && !big) {
-		uint32_t nw = n >> 2, i = 0;
-		while (i < nw && ((uintptr_t)(w + i) & 15))
-			bad |= pl_ld(&w[i++]) ^ tag;
-		uint32_t nv = (nw - i) >> 2;
-		const uint4 *v = reinterpret_cast<const uint4 *>(w + i);
-#pragma unroll 8
-		for (uint32_t k = 0; k < nv; k++) {
-			uint4 x = pl_ld(&v[k]);
-			bad |= (x.x ^ tag) | (x.y ^ tag) | (x.z ^ tag) | (x.w ^ tag);
-		}
-		for (i += nv * 4; i < nw; i++)
-			bad |= pl_ld(&w[i]) ^ tag;
-	}
-	uint32_t mb = __ballot_sync(mask, big);
-	uint32_t badbits = 0;
-	const uint32_t width = __popc(mask), rank = __popc(mask & ((1u << lane) - 1u));
-	while (mb) {
-		uint32_t j = __ffs(mb) - 1;
-		mb &= mb - 1;
-		const uint32_t *pj = (const uint32_t *)__shfl_sync(mask, (unsigned long long)w, j);
-		uint32_t nj = __shfl_sync(mask, n, j) >> 2;
-		uint32_t tj = __shfl_sync(mask, tag, j);
-		if (verify_share(rank, width, pj, nj, tj))
-			badbits |= 1u << j;
-	}
-	badbits = __reduce_or_sync(mask, badbits);
-	return bad != 0 || ((badbits >> lane) & 1u);
-}
-
-__device__ __forceinline__ bool coop_verify(uint32_t mask, uint32_t lane, const void *p, uint32_t n, uint32_t tag)
-{
-#if WL_VERIFY_SLOTS > 0
-	return coop_verify_rows(mask, lane, p, n, tag);
-#else
-	return coop_verify_blockwise(mask, lane, p, n, tag);
-#endif
 }
 
 /* Position of the (k+1)-th set bit of m; requires k < popc(m). */

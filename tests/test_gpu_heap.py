@@ -223,3 +223,30 @@ def test_bounded_wait_times_out_without_fault():
             # and the flags name the wait: the per-thread reservation, or
             # the warp path's reservation (KMA_ERR_AT_MALLOC / _AT_RESERVE)
             assert flags & ((1 << 13) if mode == MODE_PLAIN else (1 << 15))
+
+
+@pytest.mark.parametrize("mode", MODES, ids=MODE_IDS)
+def test_verify_sees_every_damaged_word(mode):
+    """One word of a live block changed behind the program's back (through a
+    saved and loaded image) is one bad tag when the block is freed, wherever
+    in the block it is and whatever the block's size; others are none."""
+    with Heap(2048, 14) as h, Workload(h, WL_C2, 1000) as wl:
+        wl.begin(0xBAD)
+        wl.rounds(7, mode)
+        assert wl.stats()["bad_tags"] == 0
+        nlive, off, size = wl.live()
+        live = np.argwhere(np.arange(off.shape[0])[:, None] < nlive[None, :])
+        rng = np.random.default_rng(7)
+        img = h.image_save()
+        region = img[len(img) - h.region_bytes:].view(np.uint32)
+        hit = rng.permutation(len(live))[: len(live) // 2]
+        for n, (k, g) in enumerate(live[hit]):
+            words = int(size[k, g]) // 4
+            # the first and last words, those beside them, and any
+            at = [0, words - 1, 1, words - 2, min(3, words - 1), max(0, words - 4), int(rng.integers(words))][n % 7]
+            region[int(off[k, g]) // 4 + at] ^= np.uint32(1 << int(rng.integers(32)))
+        assert set(size[tuple(live[hit].T)]) == {8 << i for i in range(9)}
+        h.image_load(img)
+        wl.drain(mode)
+        assert wl.stats()["bad_tags"] == len(hit)
+        assert h.error_flags() == 0
