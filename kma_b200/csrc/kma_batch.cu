@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "kma_internal.h"
+#include "kma_scratch.h"
 #include "kma_batch.h"
 #include "kma_structs.h"
 #include "kma_backend.cuh"
@@ -495,7 +496,7 @@ int batch_create(kma_heap_s *h, kma_pma_s *pma, const kma_batch_job *jobs, uint3
 	size_t o_meta = o_off + (size_t)BT_CAP * items * 4;
 	size_t o_stats = (o_meta + (size_t)BT_CAP * items * 4 + 255) & ~(size_t)255;
 	size_t total = o_stats + 16 * 8;
-	if (cudaMalloc(&b->scratch, total) != cudaSuccess) {
+	if (kma_device_malloc(&b->scratch, total) != cudaSuccess) {
 		cudaGetLastError();
 		free(b);
 		return KMA_ENOMEM;

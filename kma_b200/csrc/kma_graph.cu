@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "kma_internal.h"
+#include "kma_scratch.h"
 #include "kma_graph.h"
 #include "kma_structs.h"
 #include "kma_structs.cuh"
@@ -396,7 +397,6 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	kma_device_guard gd(device);
 	memset(st, 0, sizeof(*st));
 	uint64_t cap = 2 * n;
-	void *mem = NULL;
 	/* segments of the walk: a power of two near sqrt(n) / 8 apart, the records
 	 * for twice as many as the hash should give */
 	uint32_t spacing = 1;
@@ -412,11 +412,10 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	 * the export arrays, which are written after it (44 n + 8 bytes, of which
 	 * it needs 16 cap = 32 n behind a 16-byte boundary) */
 	const size_t o_list = (o_start + 15) & ~(size_t)15;
-	if (cudaMalloc(&mem, total) != cudaSuccess) {
-		cudaGetLastError();
+	kma_dev_bufs bufs;
+	unsigned char *m = bufs.alloc<unsigned char>(total);
+	if (!m)
 		return KMA_ENOMEM;
-	}
-	unsigned char *m = (unsigned char *)mem;
 	int rc = KMA_OK;
 	gr_dev<B> g;
 	g.h = dh;
@@ -540,7 +539,6 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	st->err = qerr;
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
-	cudaFree(mem);
 	return rc;
 }
 } /* namespace */

@@ -12,6 +12,7 @@
 #include <stdlib.h>
 #include <vector>
 #include "kma_internal.h"
+#include "kma_scratch.h"
 #include "kma_backend.cuh"
 
 /* ------------------------------------------------------------------ */
@@ -247,7 +248,7 @@ extern "C" int kma_create_ex(const kma_config *cfg, void *stream, kma_heap_t *ou
 	size_t fl_bytes = kma_align_up((compat ? nsb : k->hh.ring_cap) * 8, 4096);
 	size_t region = (size_t)nsb << cfg->sb_size_log2;
 	size_t total = hdr + st_bytes + home_bytes + fl_bytes + region;
-	if (cudaMalloc(&k->dev_mem, total) != cudaSuccess) {
+	if (kma_device_malloc(&k->dev_mem, total) != cudaSuccess) {
 		cudaGetLastError();
 		free(k);
 		return KMA_ENOMEM;
@@ -311,6 +312,7 @@ extern "C" int kma_destroy(kma_heap_t h)
 		return KMA_EINVAL;
 	kma_device_guard g(h->device);
 	cudaError_t e = cudaFree(h->dev_mem);
+	kma_scratch_trim();
 	free(h);
 	return e == cudaSuccess ? KMA_OK : KMA_ECUDA;
 }
@@ -484,22 +486,14 @@ extern "C" int kma_replay_host(kma_heap_t h, const int64_t *ops, int64_t n, int6
 	if (n == 0)
 		return KMA_OK;
 	kma_device_guard g(h->device);
-	int64_t *dops = NULL, *dout = NULL;
-	int rc = KMA_OK;
-	if (cudaMalloc(&dops, (size_t)n * 16) != cudaSuccess || cudaMalloc(&dout, (size_t)n * 8) != cudaSuccess) {
-		cudaGetLastError();
-		rc = KMA_ENOMEM;
-	}
-	if (rc == KMA_OK && cudaMemcpy(dops, ops, (size_t)n * 16, cudaMemcpyHostToDevice) != cudaSuccess)
-		rc = KMA_ECUDA;
-	if (rc == KMA_OK)
-		rc = kma_replay(h, dops, n, dout, mode, NULL);
+	kma_dev_bufs b;
+	int64_t *dops = b.alloc<int64_t>((size_t)n * 16), *dout = b.alloc<int64_t>((size_t)n * 8);
+	if (!dops || !dout)
+		return KMA_ENOMEM;
+	KMA_CUDA(cudaMemcpy(dops, ops, (size_t)n * 16, cudaMemcpyHostToDevice));
+	int rc = kma_replay(h, dops, n, dout, mode, NULL);
 	if (rc == KMA_OK && cudaMemcpy(out, dout, (size_t)n * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
 		rc = KMA_ECUDA;
-	if (dops)
-		cudaFree(dops);
-	if (dout)
-		cudaFree(dout);
 	return rc;
 }
 

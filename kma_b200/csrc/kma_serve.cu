@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "kma_internal.h"
+#include "kma_scratch.h"
 #include "kma_serve.h"
 #include "kma_structs.cuh"
 #include "kma_wl_common.cuh"
@@ -420,8 +421,8 @@ extern "C" int kma_serve_create(kma_heap_t h, const kma_serve_cfg *cfg, kma_serv
 	}
 	s->bytes_per_vertex = bpv;
 	int rc = KMA_OK;
-	if (cudaMalloc(&s->deg_cdf, cfg->deg_max * 4) != cudaSuccess ||
-	    cudaMalloc(&s->chunks, s->nchunks * 4) != cudaSuccess ||
+	if (kma_device_malloc((void **)&s->deg_cdf, cfg->deg_max * 4) != cudaSuccess ||
+	    kma_device_malloc((void **)&s->chunks, s->nchunks * 4) != cudaSuccess ||
 	    cudaMallocHost(&s->host_all, (size_t)cfg->slots * SV_WORDS * 8) != cudaSuccess)
 		rc = KMA_ENOMEM;
 	if (rc == KMA_OK && (cudaMemcpy(s->deg_cdf, cdf.data(), cfg->deg_max * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -434,8 +435,8 @@ extern "C" int kma_serve_create(kma_heap_t h, const kma_serve_cfg *cfg, kma_serv
 		if (cudaStreamCreateWithFlags(&sl.st, cudaStreamNonBlocking) != cudaSuccess ||
 		    cudaEventCreateWithFlags(&sl.end, cudaEventDefault) != cudaSuccess)
 			rc = KMA_ECUDA;
-		else if (cudaMalloc(&sl.lists, (size_t)cfg->max_vertices * sizeof(kma_clarraylist)) != cudaSuccess ||
-			 cudaMalloc(&sl.acc, SV_WORDS * 8) != cudaSuccess)
+		else if (kma_device_malloc((void **)&sl.lists, (size_t)cfg->max_vertices * sizeof(kma_clarraylist)) != cudaSuccess ||
+			 kma_device_malloc((void **)&sl.acc, SV_WORDS * 8) != cudaSuccess)
 			rc = KMA_ENOMEM;
 		else if (cudaMemset(sl.acc, 0, SV_WORDS * 8) != cudaSuccess)
 			rc = KMA_ECUDA;

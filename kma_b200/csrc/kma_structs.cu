@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "kma_internal.h"
+#include "kma_scratch.h"
 #include "kma_structs.h"
 #include "kma_structs.cuh"
 #include "kma_backend.cuh"
@@ -50,24 +51,16 @@ int put_sync(void *dst, const void *src, size_t n, cudaStream_t st)
 	return KMA_OK;
 }
 
-/* Temporary device buffers of a host call, freed on every return path. */
-struct dev_bufs {
-	std::vector<void *> v;
-	~dev_bufs()
+typedef kma_dev_bufs dev_bufs;
+
+/* Offsets of the parts of one buffer. */
+struct carve {
+	size_t at = 0;
+	size_t operator()(size_t bytes)
 	{
-		for (void *p : v)
-			cudaFree(p);
-	}
-	template <typename T>
-	T *alloc(size_t bytes)
-	{
-		void *p = NULL;
-		if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess) {
-			cudaGetLastError();
-			return NULL;
-		}
-		v.push_back(p);
-		return (T *)p;
+		const size_t o = at;
+		at = (at + bytes + 255) & ~(size_t)255;
+		return o;
 	}
 };
 
@@ -101,7 +94,7 @@ extern "C" int kma_pma_create(uint64_t bytes, int device, void *stream, kma_pma_
 	size_t hdr = (sizeof(kma_pma) + 255) & ~(size_t)255;
 	/* data + the reference's 24-byte limit slack, rounded to 16 */
 	size_t total = hdr + ((bytes + KMA_PMA_REF_HEADER + 15) & ~15ull);
-	if (cudaMalloc(&p->mem, total) != cudaSuccess) {
+	if (kma_device_malloc(&p->mem, total) != cudaSuccess) {
 		cudaGetLastError();
 		free(p);
 		return KMA_ENOMEM;
@@ -129,6 +122,7 @@ extern "C" int kma_pma_destroy(kma_pma_t p)
 		return KMA_EINVAL;
 	kma_device_guard g(p->device);
 	cudaError_t e = cudaFree(p->mem);
+	kma_scratch_trim();
 	free(p);
 	return e == cudaSuccess ? KMA_OK : KMA_ECUDA;
 }
@@ -209,7 +203,7 @@ extern "C" int kma_clqueue_create(int device, void *stream, kma_clqueue_t *out)
 		return KMA_ENOMEM;
 	q->device = current_device();
 	/* a line of its own: head and tail are the contended words */
-	if (cudaMalloc(&q->dq, 128) != cudaSuccess) {
+	if (kma_device_malloc((void **)&q->dq, 128) != cudaSuccess) {
 		cudaGetLastError();
 		free(q);
 		return KMA_ENOMEM;
@@ -317,6 +311,39 @@ __global__ void k_iq_init(kma_iqueue *q, uint32_t first_idx)
 	q->ends[2 * s].v = kma_detail::tw_make(0, d);
 	q->ends[2 * s + 1].v = kma_detail::tw_make(0, d);
 }
+
+/* An indexed queue in device memory `mem` (iqueue_bytes): header, ends,
+ * internal dummies. */
+size_t iqueue_bytes(uint32_t shards)
+{
+	carve c;
+	c(sizeof(kma_iqueue));
+	c((size_t)shards * 2 * sizeof(kma_line64));
+	c((size_t)shards * 8);
+	return c.at;
+}
+int iqueue_setup(void *mem, void *base, uint32_t stride_l2, uint32_t capacity, uint32_t first_idx, uint32_t shards,
+		kma_chain_log *log, cudaStream_t st)
+{
+	carve c;
+	unsigned char *m = (unsigned char *)mem;
+	kma_iqueue hq;
+	memset(&hq, 0, sizeof(hq));
+	c(sizeof(kma_iqueue));
+	hq.base = (unsigned char *)base;
+	hq.ends = (kma_line64 *)(m + c((size_t)shards * 2 * sizeof(kma_line64)));
+	hq.dummies = (unsigned long long *)(m + c((size_t)shards * 8));
+	hq.stride_l2 = stride_l2;
+	hq.capacity = capacity;
+	hq.nshards = shards;
+	hq.spin_limit = KMA_STRUCT_SPIN;
+	hq.log = log;
+	KMA_CUDA(cudaMemsetAsync(mem, 0, c.at, st));
+	KMA_CUDA(cudaMemcpyAsync(mem, &hq, sizeof(hq), cudaMemcpyHostToDevice, st));
+	k_iq_init<<<(shards + 255) / 256, 256, 0, st>>>((kma_iqueue *)mem, first_idx);
+	KMA_CUDA(cudaGetLastError());
+	return KMA_OK;
+}
 } /* namespace */
 
 extern "C" int kma_iqueue_create(void *base, uint32_t stride_l2, uint32_t capacity, void *first,
@@ -339,34 +366,16 @@ extern "C" int kma_iqueue_create(void *base, uint32_t stride_l2, uint32_t capaci
 	if (!q)
 		return KMA_ENOMEM;
 	q->device = current_device();
-	size_t hdr = (sizeof(kma_iqueue) + 127) & ~(size_t)127;
-	size_t ends = (size_t)shards * 2 * sizeof(kma_line64);
-	size_t dum = (((size_t)shards * 8) + 127) & ~(size_t)127;
-	if (cudaMalloc(&q->mem, hdr + ends + dum) != cudaSuccess) {
+	if (kma_device_malloc(&q->mem, iqueue_bytes(shards)) != cudaSuccess) {
 		cudaGetLastError();
 		free(q);
 		return KMA_ENOMEM;
 	}
 	q->dq = (kma_iqueue *)q->mem;
-	kma_iqueue hq;
-	memset(&hq, 0, sizeof(hq));
-	hq.base = (unsigned char *)base;
-	hq.ends = (kma_line64 *)((unsigned char *)q->mem + hdr);
-	hq.dummies = (unsigned long long *)((unsigned char *)q->mem + hdr + ends);
-	hq.stride_l2 = stride_l2;
-	hq.capacity = capacity;
-	hq.nshards = shards;
-	hq.spin_limit = KMA_STRUCT_SPIN;
 	cudaStream_t st = kma_stream(stream);
-	int rc = KMA_OK;
-	if (cudaMemsetAsync(q->mem, 0, hdr + ends + dum, st) != cudaSuccess ||
-	    cudaMemcpyAsync(q->dq, &hq, sizeof(hq), cudaMemcpyHostToDevice, st) != cudaSuccess)
+	int rc = iqueue_setup(q->mem, base, stride_l2, capacity, (uint32_t)(off >> stride_l2) + 1, shards, NULL, st);
+	if (rc == KMA_OK && cudaStreamSynchronize(st) != cudaSuccess)
 		rc = KMA_ECUDA;
-	if (rc == KMA_OK) {
-		k_iq_init<<<(shards + 255) / 256, 256, 0, st>>>(q->dq, (uint32_t)(off >> stride_l2) + 1);
-		if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
-			rc = KMA_ECUDA;
-	}
 	if (rc != KMA_OK) {
 		cudaFree(q->mem);
 		free(q);
@@ -639,6 +648,28 @@ extern "C" int kma_iqueue_replay_host(uint32_t n_items, uint32_t stride_l2, cons
 /* chain log                                                           */
 /* ------------------------------------------------------------------ */
 
+namespace {
+/* A chain log in device memory `mem`: header line, counter line, the records
+ * and the notes, all zero (an entry is 0 until a chain fills it). */
+size_t chain_log_bytes(uint32_t records)
+{
+	return 256 + (size_t)records * 256 + KMA_LOG_NOTES * sizeof(ulonglong2);
+}
+int chain_log_setup(void *mem, uint32_t records, cudaStream_t st)
+{
+	unsigned char *m = (unsigned char *)mem;
+	kma_chain_log hl;
+	memset(&hl, 0, sizeof(hl));
+	hl.rec = (unsigned long long *)(m + 256);
+	hl.next = (unsigned int *)(m + 128);
+	hl.mask = records - 1;
+	hl.notes = (ulonglong2 *)(m + 256 + (size_t)records * 256);
+	KMA_CUDA(cudaMemsetAsync(mem, 0, chain_log_bytes(records), st));
+	KMA_CUDA(cudaMemcpyAsync(mem, &hl, sizeof(hl), cudaMemcpyHostToDevice, st));
+	return KMA_OK;
+}
+} /* namespace */
+
 extern "C" int kma_chain_log_create(uint32_t records, int device, void *stream, kma_chain_log_t *out)
 {
 	if (!out)
@@ -653,27 +684,16 @@ extern "C" int kma_chain_log_create(uint32_t records, int device, void *stream, 
 	if (!l)
 		return KMA_ENOMEM;
 	l->device = current_device();
-	/* header line, counter line, then the records (zeroed: an entry is 0
-	 * until a chain fills it) and the notes */
-	const size_t hdr = 256, rec = (size_t)records * 256, bytes = hdr + rec + KMA_LOG_NOTES * sizeof(ulonglong2);
-	if (cudaMalloc(&l->mem, bytes) != cudaSuccess) {
+	if (kma_device_malloc(&l->mem, chain_log_bytes(records)) != cudaSuccess) {
 		cudaGetLastError();
 		free(l);
 		return KMA_ENOMEM;
 	}
 	l->dl = (kma_chain_log *)l->mem;
-	kma_chain_log hl;
-	memset(&hl, 0, sizeof(hl));
-	hl.rec = (unsigned long long *)((unsigned char *)l->mem + hdr);
-	hl.next = (unsigned int *)((unsigned char *)l->mem + 128);
-	hl.mask = records - 1;
-	hl.notes = (ulonglong2 *)((unsigned char *)l->mem + hdr + rec);
 	cudaStream_t st = kma_stream(stream);
-	int rc = KMA_OK;
-	if (cudaMemsetAsync(l->mem, 0, bytes, st) != cudaSuccess)
+	int rc = chain_log_setup(l->mem, records, st);
+	if (rc == KMA_OK && cudaStreamSynchronize(st) != cudaSuccess)
 		rc = KMA_ECUDA;
-	if (rc == KMA_OK)
-		rc = put_sync(l->dl, &hl, sizeof(hl), st);
 	if (rc != KMA_OK) {
 		cudaFree(l->mem);
 		free(l);
@@ -720,7 +740,7 @@ extern "C" int kma_cltree_create(int device, void *stream, kma_cltree_t *out)
 	if (!t)
 		return KMA_ENOMEM;
 	t->device = current_device();
-	if (cudaMalloc(&t->dt, 128) != cudaSuccess) {
+	if (kma_device_malloc((void **)&t->dt, 128) != cudaSuccess) {
 		cudaGetLastError();
 		free(t);
 		return KMA_ENOMEM;
@@ -867,7 +887,7 @@ extern "C" int kma_clarraylist_create(uint32_t obj_size, kma_heap_t kma, kma_pma
 	if (!l)
 		return KMA_ENOMEM;
 	l->device = current_device();
-	if (cudaMalloc(&l->dl, 128) != cudaSuccess) {
+	if (kma_device_malloc((void **)&l->dl, 128) != cudaSuccess) {
 		cudaGetLastError();
 		free(l);
 		return KMA_ENOMEM;
@@ -1298,87 +1318,78 @@ extern "C" int kma_c3_queue_run(int kind, uint32_t threads, uint32_t per_thread,
 	if (!g.ok)
 		return KMA_ENODEV;
 	memset(st, 0, sizeof(*st));
+	/* warp forms: a chain log of one record per 16 payloads (every chain
+	 * of this run keeps its record: chains hold up to 32 payloads) */
+	uint32_t rec = 0;
+	if (warp)
+		for (rec = 1; rec < n / 16 && rec < (1u << 24);)
+			rec <<= 1;
+	const bool clq = kind == KMA_C3_CLQUEUE;
+	const size_t items_bytes = (size_t)(n + 1) * QITEM, q_bytes = clq ? (size_t)shards * 128 : iqueue_bytes(shards);
+	carve at;
+	const size_t o_acc = at(16 * 8), o_err = at(4), o_q = at(q_bytes), o_items = at(items_bytes),
+		     o_log = at(warp ? chain_log_bytes(rec) : 0);
 	dev_bufs b;
-	unsigned long long *acc = b.alloc<unsigned long long>(16 * 8);
-	uint32_t *err = b.alloc<uint32_t>(4);
-	unsigned char *items = b.alloc<unsigned char>((size_t)(n + 1) * QITEM);
-	if (!acc || !err || !items)
+	unsigned char *mem = b.alloc<unsigned char>(at.at);
+	if (!mem)
 		return KMA_ENOMEM;
-	KMA_CUDA(cudaMemset(acc, 0, 16 * 8));
-	KMA_CUDA(cudaMemset(err, 0, 4));
-	KMA_CUDA(cudaMemset(items, 0, (size_t)(n + 1) * QITEM));
+	unsigned long long *acc = (unsigned long long *)(mem + o_acc);
+	uint32_t *err = (uint32_t *)(mem + o_err);
+	unsigned char *items = mem + o_items, *qs = mem + o_q;
+	kma_iqueue *iq = (kma_iqueue *)qs;
+	kma_chain_log *dl = warp ? (kma_chain_log *)(mem + o_log) : NULL;
+	int rc = KMA_OK;
+	if (cudaMemsetAsync(mem, 0, o_q, NULL) != cudaSuccess || cudaMemsetAsync(items, 0, items_bytes, NULL) != cudaSuccess)
+		rc = KMA_ECUDA;
+	if (rc == KMA_OK && warp)
+		rc = chain_log_setup(dl, rec, NULL);
+	if (rc == KMA_OK && clq && cudaMemsetAsync(qs, 0, q_bytes, NULL) != cudaSuccess)
+		rc = KMA_ECUDA;
+	if (rc == KMA_OK && !clq)
+		rc = iqueue_setup(iq, items, 4, n + 1, 1, shards, dl, NULL);
+	if (rc != KMA_OK)
+		return rc;
 	cudaEvent_t e0, e1, e2;
 	cudaEventCreate(&e0);
 	cudaEventCreate(&e1);
 	cudaEventCreate(&e2);
-	uint32_t blocks = (threads + 255) / 256;
-	int rc = KMA_OK;
-	kma_iqueue_t iq = NULL;
-	/* warp forms: a chain log of one record per 16 payloads (every chain
-	 * of this run keeps its record: chains hold up to 32 payloads) */
-	kma_chain_log_t log = NULL;
-	if (warp) {
-		uint32_t rec = 1;
-		while (rec < n / 16 && rec < (1u << 24))
-			rec <<= 1;
-		rc = kma_chain_log_create(rec, -1, NULL, &log);
-	}
-	if (rc != KMA_OK) {
-		/* no log: nothing ran */
-	} else if (kind == KMA_C3_CLQUEUE) {
-		unsigned char *qs = b.alloc<unsigned char>((size_t)shards * 128);
-		if (!qs)
-			rc = KMA_ENOMEM;
-		if (rc == KMA_OK) {
-			cudaMemset(qs, 0, (size_t)shards * 128);
-			cudaEventRecord(e0);
-			kma_chain_log *dl = kma_chain_log_device_ptr(log);
-			if (warp)
-				k_c3_clq_enq<true><<<blocks, 256>>>(qs, shards, items, per_thread, n, seed, acc, err, dl);
-			else
-				k_c3_clq_enq<false><<<blocks, 256>>>(qs, shards, items, per_thread, n, seed, acc, err, dl);
-			cudaEventRecord(e1);
-			if (block)
-				k_c3_clq_deq_block<<<blocks, 256>>>((kma_clqueue *)qs, per_thread, threads, acc, err, dl);
-			else if (warp)
-				k_c3_clq_deq<true><<<blocks, 256>>>(qs, shards, per_thread, threads, acc, err, dl);
-			else
-				k_c3_clq_deq<false><<<blocks, 256>>>(qs, shards, per_thread, threads, acc, err, dl);
-			cudaEventRecord(e2);
-			k_c3_clq_walk<<<(shards + 127) / 128, 128>>>(qs, shards, n, acc);
-		}
-	} else {
-		rc = kma_iqueue_create(items, 4, n + 1, items, shards, -1, NULL, &iq);
-		if (rc == KMA_OK && log)
-			rc = kma_iqueue_set_chain_log(iq, log, NULL);
-		if (rc == KMA_OK) {
-			cudaEventRecord(e0);
-			if (warp)
-				k_c3_iq_enq<true><<<blocks, 256>>>(iq->dq, per_thread, n, seed, acc);
-			else
-				k_c3_iq_enq<false><<<blocks, 256>>>(iq->dq, per_thread, n, seed, acc);
-			cudaEventRecord(e1);
-			if (block)
-				k_c3_iq_deq_block<<<blocks, 256>>>(iq->dq, per_thread, threads, acc);
-			else if (warp)
-				k_c3_iq_deq<true><<<blocks, 256>>>(iq->dq, per_thread, threads, acc);
-			else
-				k_c3_iq_deq<false><<<blocks, 256>>>(iq->dq, per_thread, threads, acc);
-			cudaEventRecord(e2);
-			k_c3_iq_walk<<<(shards + 127) / 128, 128>>>(iq->dq, n, acc);
-		}
-	}
+	const uint32_t blocks = (threads + 255) / 256;
+	cudaEventRecord(e0);
+	if (clq && warp)
+		k_c3_clq_enq<true><<<blocks, 256>>>(qs, shards, items, per_thread, n, seed, acc, err, dl);
+	else if (clq)
+		k_c3_clq_enq<false><<<blocks, 256>>>(qs, shards, items, per_thread, n, seed, acc, err, dl);
+	else if (warp)
+		k_c3_iq_enq<true><<<blocks, 256>>>(iq, per_thread, n, seed, acc);
+	else
+		k_c3_iq_enq<false><<<blocks, 256>>>(iq, per_thread, n, seed, acc);
+	cudaEventRecord(e1);
+	if (clq && block)
+		k_c3_clq_deq_block<<<blocks, 256>>>((kma_clqueue *)qs, per_thread, threads, acc, err, dl);
+	else if (clq && warp)
+		k_c3_clq_deq<true><<<blocks, 256>>>(qs, shards, per_thread, threads, acc, err, dl);
+	else if (clq)
+		k_c3_clq_deq<false><<<blocks, 256>>>(qs, shards, per_thread, threads, acc, err, dl);
+	else if (block)
+		k_c3_iq_deq_block<<<blocks, 256>>>(iq, per_thread, threads, acc);
+	else if (warp)
+		k_c3_iq_deq<true><<<blocks, 256>>>(iq, per_thread, threads, acc);
+	else
+		k_c3_iq_deq<false><<<blocks, 256>>>(iq, per_thread, threads, acc);
+	cudaEventRecord(e2);
+	if (clq)
+		k_c3_clq_walk<<<(shards + 127) / 128, 128>>>(qs, shards, n, acc);
+	else
+		k_c3_iq_walk<<<(shards + 127) / 128, 128>>>(iq, n, acc);
 	if (rc == KMA_OK && (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess))
 		rc = KMA_ECUDA;
 	unsigned long long h[16];
 	if (rc == KMA_OK && cudaMemcpy(h, acc, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess)
 		rc = KMA_ECUDA;
 	uint32_t e = 0;
+	if (rc == KMA_OK && cudaMemcpy(&e, clq ? err : &iq->err, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+		rc = KMA_ECUDA;
 	if (rc == KMA_OK) {
-		if (kind == KMA_C3_CLQUEUE)
-			cudaMemcpy(&e, err, 4, cudaMemcpyDeviceToHost);
-		else
-			kma_iqueue_error_flags(iq, NULL, &e, 0);
 		st->enqueued = h[0];
 		st->in_xor = h[1];
 		st->in_sum = h[2];
@@ -1392,18 +1403,10 @@ extern "C" int kma_c3_queue_run(int kind, uint32_t threads, uint32_t per_thread,
 		st->err = e;
 		cudaEventElapsedTime(&st->enqueue_ms, e0, e1);
 		cudaEventElapsedTime(&st->dequeue_ms, e1, e2);
-		if (log) {
-			kma_chain_log hl;
-			unsigned int cnt[2] = {0, 0};
-			if (cudaMemcpy(&hl, log->dl, sizeof(hl), cudaMemcpyDeviceToHost) == cudaSuccess &&
-			    cudaMemcpy(cnt, hl.next, sizeof(cnt), cudaMemcpyDeviceToHost) == cudaSuccess)
-				st->log_chains = cnt[1];
-		}
+		unsigned int cnt[2] = {0, 0};
+		if (warp && cudaMemcpy(cnt, mem + o_log + 128, sizeof(cnt), cudaMemcpyDeviceToHost) == cudaSuccess)
+			st->log_chains = cnt[1];
 	}
-	if (iq)
-		kma_iqueue_destroy(iq);
-	if (log)
-		kma_chain_log_destroy(log);
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
 	cudaEventDestroy(e2);
@@ -1458,23 +1461,24 @@ extern "C" int kma_c3_tree_run(const uint8_t *kinds, const uint32_t *keys, uint6
 		for (uint64_t j = 0; j < n_ops; j++)
 			order[pos[keys[j] % threads]++] = (uint32_t)j;
 	}
-	kma_cltree_t t;
-	int rc = kma_cltree_create(-1, NULL, &t);
-	if (rc != KMA_OK)
-		return rc;
+	int rc = KMA_OK;
 	{
+		carve at;
+		const size_t o_tree = at(128), o_pool = at(n_ops * sizeof(kma_cltree_node)), o_kinds = at(n_ops),
+			     o_keys = at(n_ops * 4), o_ord = at(n_ops * 4), o_offs = at(((size_t)threads + 1) * 8),
+			     o_res = at(n_ops), o_list = at(n_ops * sizeof(ulonglong2)), o_sum = at(KMA_TC_WORDS * 8);
 		dev_bufs b;
-		kma_cltree_node *pool = b.alloc<kma_cltree_node>(n_ops * sizeof(kma_cltree_node));
-		uint8_t *dk = b.alloc<uint8_t>(n_ops);
-		uint32_t *dkeys = b.alloc<uint32_t>(n_ops * 4);
-		uint32_t *dord = b.alloc<uint32_t>(n_ops * 4);
-		uint64_t *doffs = b.alloc<uint64_t>(((size_t)threads + 1) * 8);
-		int8_t *dres = b.alloc<int8_t>(n_ops);
-		ulonglong2 *list = b.alloc<ulonglong2>(n_ops * sizeof(ulonglong2));
-		unsigned long long *summ = b.alloc<unsigned long long>(KMA_TC_WORDS * 8);
-		if (!pool || !dk || !dkeys || !dord || !doffs || !dres || !list || !summ)
-			rc = KMA_ENOMEM;
-		if (rc == KMA_OK &&
+		unsigned char *m = b.alloc<unsigned char>(at.at);
+		if (!m)
+			return KMA_ENOMEM;
+		kma_cltree *dt = (kma_cltree *)(m + o_tree);
+		kma_cltree_node *pool = (kma_cltree_node *)(m + o_pool);
+		uint8_t *dk = m + o_kinds;
+		uint32_t *dkeys = (uint32_t *)(m + o_keys), *dord = (uint32_t *)(m + o_ord);
+		uint64_t *doffs = (uint64_t *)(m + o_offs);
+		int8_t *dres = (int8_t *)(m + o_res);
+		unsigned long long *summ = (unsigned long long *)(m + o_sum);
+		if (cudaMemset(dt, 0, 128) != cudaSuccess ||
 		    (cudaMemcpy(dk, kinds, n_ops, cudaMemcpyHostToDevice) != cudaSuccess ||
 		     cudaMemcpy(dkeys, keys, n_ops * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
 		     cudaMemcpy(dord, order.data(), n_ops * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -1485,12 +1489,12 @@ extern "C" int kma_c3_tree_run(const uint8_t *kinds, const uint32_t *keys, uint6
 			cudaEventCreate(&e0);
 			cudaEventCreate(&e1);
 			cudaEventRecord(e0);
-			k_c3_tree<<<(threads + 255) / 256, 256>>>(t->dt, pool, dk, dkeys, dord, doffs, threads, dres);
+			k_c3_tree<<<(threads + 255) / 256, 256>>>(dt, pool, dk, dkeys, dord, doffs, threads, dres);
 			cudaEventRecord(e1);
 			if (cudaGetLastError() != cudaSuccess)
 				rc = KMA_ECUDA;
 			if (rc == KMA_OK)
-				rc = tree_check(t->dt, list, n_ops, summ, t->device, NULL);
+				rc = tree_check(dt, m + o_list, n_ops, summ, current_device(), NULL);
 			if (rc == KMA_OK && cudaDeviceSynchronize() != cudaSuccess)
 				rc = KMA_ECUDA;
 			cudaEventElapsedTime(&st->ms, e0, e1);
@@ -1509,6 +1513,5 @@ extern "C" int kma_c3_tree_run(const uint8_t *kinds, const uint32_t *keys, uint6
 			st->err = s[KMA_TC_OVERFLOW] ? 1u : 0u;
 		}
 	}
-	kma_cltree_destroy(t);
 	return rc;
 }

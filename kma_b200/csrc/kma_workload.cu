@@ -24,6 +24,7 @@
 #include <stdlib.h>
 #include <mutex>
 #include "kma_internal.h"
+#include "kma_scratch.h"
 #include "kma_wl_common.cuh"
 
 #define WL_CAP 32
@@ -512,7 +513,7 @@ extern "C" int kma_wl_create(kma_heap_t h, int program, uint64_t items, kma_wl_t
 	size_t off_stats = (off_lsize + 4 * n * WL_CAP + 255) & ~(size_t)255;
 	size_t off_seeds = off_stats + 8 * WL_STATS_WORDS;
 	size_t total = off_seeds + 8 * n;
-	if (cudaMalloc(&w->scratch, total) != cudaSuccess) {
+	if (kma_device_malloc(&w->scratch, total) != cudaSuccess) {
 		cudaGetLastError();
 		free(w);
 		return KMA_ENOMEM;
