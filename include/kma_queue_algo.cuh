@@ -788,6 +788,52 @@ KQ_FN uint32_t iq_dequeue_n(const Q &q, u64 *headw, uint32_t *out, uint32_t k, u
 	return 0;
 }
 
+/* Dequeue one old dummy into *out: what iq_dequeue_n does with k = 1, without
+ * the hold.  A hold is five dependent round trips during which nobody else can
+ * take (read the head and its link, take the hold, the link again, give the
+ * new head back); one item needs only a CAS of the head to the successor that
+ * was read, two round trips, and the losers of a race have lost theirs.  The
+ * successor cannot be out of date when the CAS succeeds: the head's tag counts
+ * every change, so the dummy was the head throughout, and a head's link is
+ * written once.  Both loads are acquires: with them a dummy's link, reset
+ * before it was appended, is read as reset or as its successor, never as what
+ * it was in an earlier turn of the item.  A head held by iq_dequeue_n (odd
+ * tag) is waited for as there. */
+template <class O, class Q>
+KQ_FN uint32_t iq_dequeue_1(const Q &q, u64 *headw, uint32_t *out, uint32_t limit, bool *timed_out)
+{
+	*timed_out = false;
+	uint32_t idle = 0;
+	u64 last = ~0ull;
+	for (uint32_t it = 0;; it++) {
+		const u64 hd = O::ld(headw);
+		if (hd != last) {
+			last = hd;
+			idle = 0;
+		} else if (++idle >= limit) {
+			break;
+		}
+		if (iq_head_held(hd)) {
+			O::pause(it);
+			continue;
+		}
+		const uint32_t cur = tw_idx(hd), next = tw_idx(O::ld(q.link(cur)));
+		if (next == 0) {
+			/* only the dummy: empty, if the head is still this one */
+			if (O::ld_rlx(headw) == hd)
+				return 0;
+			continue;
+		}
+		if (O::cas(headw, hd, tw_make(tw_tag(hd) + 2u, next)) == hd) {
+			*out = cur;
+			return 1;
+		}
+		O::pause(it);
+	}
+	*timed_out = true;
+	return 0;
+}
+
 } /* namespace kma_q */
 
 #endif /* KMA_QUEUE_ALGO_CUH */

@@ -43,7 +43,8 @@
  * the consumers back until the producers are done (config 3's order), so
  * batches meet whole logged chains and take several per hold; LANES 1
  * dequeues with the warp's text (clq_dequeue_v), its 32 lanes as arrays:
- * LANES 2 every other batch, so that both texts meet on one queue.  Prints one
+ * LANES 2 every other batch, so that both texts meet on one queue.  (Indexed
+ * queue: LANES takes one item at a time, with iq_dequeue_1.)  Prints one
  * JSON line (with the chains taken from records and the dequeue calls
  * that took items); exits 0 when every check passed.  The reference's own
  * queues are the parity oracle (serial replays against tests/golden);
@@ -445,7 +446,9 @@ void run_iq(int threads, int chains, int maxc, int batch, double recycle, uint64
 			bool done = producing.load() == 0;
 			bool to = false;
 			uint32_t k = g_fixed_batch ? (uint32_t)batch : 1 + (uint32_t)(rnd() % batch);
-			uint32_t r = kma_q::iq_dequeue_n<HostOps>(q, &ends[0], out.data(), k, LIMIT, &to, log_ptr());
+			uint32_t r = g_lanes == 1 || (g_lanes == 2 && (rnd() & 1))
+				? kma_q::iq_dequeue_1<HostOps>(q, &ends[0], out.data(), LIMIT, &to)
+				: kma_q::iq_dequeue_n<HostOps>(q, &ends[0], out.data(), k, LIMIT, &to, log_ptr());
 			if (to)
 				bk.tmo++;
 			back.clear();
@@ -552,6 +555,15 @@ int run_stuck()
 		uint32_t r = kma_q::clq_dequeue_v<HostOps, LinkAtItem, HostLanes>(&q[0], &q[1], out, 4, limit, &to,
 										 (const HostLog *)nullptr);
 		ok &= r == 0 && to && a.next == (state == 0 ? kma_q::POISON : 0ull) && q[0] == (u64)&a;
+	}
+	{
+		std::vector<u64> links(4, 0);
+		IdxQ iq{&links};
+		links[1] = kma_q::tw_make(0, 2);
+		u64 ends[2] = {kma_q::tw_make(1, 1), kma_q::tw_make(0, 2)};
+		uint32_t out[1];
+		bool to = false;
+		ok &= kma_q::iq_dequeue_1<HostOps>(iq, &ends[0], out, limit, &to) == 0 && to && ends[0] == kma_q::tw_make(1, 1);
 	}
 	printf("{\"stuck_ok\": %s}\n", ok ? "true" : "false");
 	return ok ? 0 : 1;

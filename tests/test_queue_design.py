@@ -201,9 +201,10 @@ LANES_CONFIGS = [
 
 
 @pytest.mark.parametrize("lanes", [1, 2])
+@pytest.mark.parametrize("kind", ["clq", "iq"])  # iq: iq_dequeue_1, one item at a time
 @pytest.mark.parametrize("cfg", LANES_CONFIGS)
-def test_warp_text_conserves_and_keeps_order(harness, cfg, lanes):
-    rc, st = run(harness, "clq", f"{cfg} {lanes}")
+def test_warp_text_conserves_and_keeps_order(harness, cfg, kind, lanes):
+    rc, st = run(harness, kind, f"{cfg} {lanes}")
     assert rc == 0 and st.get("ok"), st
     assert st["taken"] + st["left"] >= st["appended"] > 0
     assert st["conservation_faults"] == 0 and st["order_faults"] == 0 and st["timeouts"] == 0
