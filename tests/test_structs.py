@@ -388,3 +388,24 @@ def test_gpu_clqueue_ragged_chains_conserve(form, threads, per):
     assert st["err"] == 0 and st["walk_ok"] == 1 and st["empty"] == 0
     assert st["enqueued"] == st["out_count"] == n
     assert st["out_xor"] == st["in_xor"] and st["out_sum"] == st["in_sum"] == n * (n - 1) // 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,threads,repeat", [
+    (1, 1, 1), (64, 1, 1), (65, 1, 1),       # one owner: the longest slice the device sorts, and one more
+    (3000, 1023, 1), (3000, 1024, 1), (3000, 1025, 1),  # the counts fill a tile, and run over it
+    (5000, 5000, 64), (5000, 5000, 65), (100, 70000, 1)])
+def test_gpu_c3_tree_groups_by_owner(n, threads, repeat):
+    """Every owner's operations run in their order, grouped on the device or
+    (longer slices) on the host: one key is used `repeat` times."""
+    from kma_b200 import structs
+    rng = np.random.default_rng(n + threads + repeat)
+    kinds = rng.choice(3, size=n, p=(0.5, 0.2, 0.3)).astype(np.uint8)
+    keys = rng.integers(0, max(2, n // 2), size=n).astype(np.uint32) * 7 + 1
+    if repeat > 1:
+        keys = np.arange(n, dtype=np.uint32) + 10
+        keys[rng.permutation(n)[:repeat]] = 3
+    res, st = structs.c3_tree(kinds, keys, threads=threads)
+    mout, mkeys = tree_model(np.stack([kinds, keys], 1))
+    np.testing.assert_array_equal(res.astype(np.int64), np.where(kinds == 1, (mout >= 0).astype(np.int64), mout))
+    assert (st["err"], st["sorted"], st["live_keys"], st["keys_sum"]) == (0, 1, len(mkeys), int(mkeys.sum()))
