@@ -84,10 +84,28 @@ __device__ __forceinline__ uint32_t geom_quarter(uint64_t x)
 	return t ? (uint32_t)(__ffsll((long long)t) - 1) / 2 + 1 : 32u;
 }
 
+/* A warp's counters (kma_batch_stats order) in shared memory: a lane's own
+ * would be twelve of its 64 registers. */
+enum { BT_MALLOCS, BT_FREES, BT_NULLS, BT_BAD, BT_FILL, BT_VERIFY, BT_HITS, BT_PUTS, BT_RETIRED, BT_REFUSED, BT_WORDS };
 struct bt_counters {
-	uint32_t mallocs, frees, nulls, bad, hits, puts, retired, refused;
-	unsigned long long fill, verify;
+	unsigned long long *n;
 };
+/* add x (the same in every lane) */
+__device__ __forceinline__ void bt_count(const bt_counters &ct, uint32_t lane, uint32_t k, uint32_t x)
+{
+	if (lane == 0)
+		ct.n[k] += x;
+}
+/* add the number of lanes with b set; every lane of the warp calls */
+__device__ __forceinline__ void bt_count_if(const bt_counters &ct, uint32_t lane, uint32_t k, bool b)
+{
+	bt_count(ct, lane, k, __popc(__ballot_sync(0xffffffffu, b)));
+}
+/* add every lane's x (of a sum below 2^32) */
+__device__ __forceinline__ void bt_count_sum(const bt_counters &ct, uint32_t lane, uint32_t k, uint32_t x)
+{
+	bt_count(ct, lane, k, __reduce_add_sync(0xffffffffu, x));
+}
 
 /* per-warp shared memory: cnt[BT_NCLS], hint[BT_NCLS], slot[BT_NCLS][depth] */
 struct bt_cache {
@@ -120,7 +138,7 @@ __device__ __forceinline__ uint32_t bt_bytes(uint32_t meta) { return (meta & 0x3
  * for q's class, else to the heap.  Every lane of the warp calls it. */
 template <class B, bool WARP>
 __device__ __forceinline__ void bt_free(typename B::heap *h, const bt_cache &cc, uint32_t lane, void *q, uint32_t n,
-		bt_counters &ct)
+		const bt_counters &ct)
 {
 	bool keep = false;
 	if constexpr (WARP && B::id == KMA_BACKEND_ID_KMA) {
@@ -131,7 +149,6 @@ __device__ __forceinline__ void bt_free(typename B::heap *h, const bt_cache &cc,
 				if (s < (int)cc.depth) {
 					cc.slot[c * cc.depth + s] = bt_off<B>(h, q);
 					keep = true;
-					ct.puts++;
 				}
 			}
 		}
@@ -140,6 +157,7 @@ __device__ __forceinline__ void bt_free(typename B::heap *h, const bt_cache &cc,
 			if (lane < BT_NCLS && cc.cnt[lane] > (int)cc.depth)
 				cc.cnt[lane] = (int)cc.depth;
 			__syncwarp();
+			bt_count_if(ct, lane, BT_PUTS, keep);
 		}
 	}
 	if (WARP)
@@ -152,7 +170,7 @@ __device__ __forceinline__ void bt_free(typename B::heap *h, const bt_cache &cc,
  * a block of n's class, else from the heap.  Every lane calls it. */
 template <class B, bool WARP>
 __device__ __forceinline__ void *bt_malloc(typename B::heap *h, const bt_cache &cc, uint32_t lane, bool want,
-		uint32_t n, bt_counters &ct)
+		uint32_t n, const bt_counters &ct)
 {
 	void *p = NULL;
 	bool need = want;
@@ -165,7 +183,6 @@ __device__ __forceinline__ void *bt_malloc(typename B::heap *h, const bt_cache &
 					if (old > 0) {
 						p = bt_block<B>(h, cc.slot[c * cc.depth + old - 1]);
 						need = false;
-						ct.hits++;
 					}
 				}
 			}
@@ -173,6 +190,7 @@ __device__ __forceinline__ void *bt_malloc(typename B::heap *h, const bt_cache &
 			if (lane < BT_NCLS && cc.cnt[lane] < 0)
 				cc.cnt[lane] = 0;
 			__syncwarp();
+			bt_count_if(ct, lane, BT_HITS, want && !need);
 		}
 		void *q = kma_malloc_warp(h, need ? (size_t)n : B::no_request, nullptr, cc.hint);
 		return need ? q : p;
@@ -187,7 +205,7 @@ __device__ __forceinline__ void *bt_malloc(typename B::heap *h, const bt_cache &
 /* One round of every lane's item (act = the lane has one). */
 template <class B, bool WARP>
 __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, const bt_cache &cc, uint32_t lane,
-		bool act, uint64_t g, uint32_t r, uint64_t &rng, uint32_t &nl, bt_counters &ct)
+		bool act, uint64_t g, uint32_t r, uint64_t &rng, uint32_t &nl, const bt_counters &ct)
 {
 	const uint32_t mask = 0xffffffffu;
 	const uint64_t items = w.items;
@@ -211,13 +229,10 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 			q = bt_block<B>(h, w.off4[e]);
 			qn = bt_bytes(w.meta[e]);
 		}
-		if (coop_verify(mask, lane, q, qn, (uint32_t)o_g))
-			ct.bad++;
+		bt_count_if(ct, lane, BT_BAD, coop_verify(mask, lane, q, qn, (uint32_t)o_g));
 		bt_free<B, WARP>(h, cc, lane, q, qn, ct);
-		if (q) {
-			ct.frees++;
-			ct.verify += qn;
-		}
+		bt_count_if(ct, lane, BT_FREES, mine);
+		bt_count_sum(ct, lane, BT_VERIFY, qn);
 	}
 	/* other lanes read this lane's table above; it is compacted next */
 	__syncwarp(mask);
@@ -245,13 +260,12 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 			q = bt_block<B>(h, w.off4[g]);
 			qn = bt_bytes(w.meta[g]);
 		}
-		if (coop_verify(mask, lane, q, qn, tag))
-			ct.bad++;
+		bt_count_if(ct, lane, BT_BAD, coop_verify(mask, lane, q, qn, tag));
 		bt_free<B, WARP>(h, cc, lane, q, qn, ct);
+		bt_count_if(ct, lane, BT_FREES, full);
+		bt_count_if(ct, lane, BT_RETIRED, full);
+		bt_count_sum(ct, lane, BT_VERIFY, qn);
 		if (full) {
-			ct.frees++;
-			ct.retired++;
-			ct.verify += qn;
 			for (uint32_t i = 1; i < BT_CAP; i++) {
 				w.off4[(uint64_t)(i - 1) * items + g] = w.off4[(uint64_t)i * items + g];
 				w.meta[(uint64_t)(i - 1) * items + g] = w.meta[(uint64_t)i * items + g];
@@ -263,20 +277,18 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 	uint32_t n = zipf_size(w.zipf, splitmix(rng));
 	uint32_t life = geom_quarter(splitmix(rng));
 	void *p = bt_malloc<B, WARP>(h, cc, lane, act, n, ct);
-	if (act) {
-		ct.mallocs++;
-		if (p) {
-			w.off4[(uint64_t)nl * items + g] = bt_off<B>(h, p);
-			w.meta[(uint64_t)nl * items + g] = (n / 8u) | ((r + life) << 16);
-			nl++;
-			ct.fill += n;
-		} else {
-			ct.nulls++;
-			if (n > B::max_request(h))
-				ct.refused++;
-		}
+	if (act && p) {
+		w.off4[(uint64_t)nl * items + g] = bt_off<B>(h, p);
+		w.meta[(uint64_t)nl * items + g] = (n / 8u) | ((r + life) << 16);
+		nl++;
 	}
 	__syncwarp(mask);
+	bt_count_if(ct, lane, BT_MALLOCS, act);
+	bt_count_sum(ct, lane, BT_FILL, act && p ? n : 0u);
+	if (__any_sync(mask, act && !p)) {
+		bt_count_if(ct, lane, BT_NULLS, act && !p);
+		bt_count_if(ct, lane, BT_REFUSED, act && !p && n > B::max_request(h));
+	}
 	coop_fill(mask, lane, act ? p : NULL, n, tag);
 }
 
@@ -297,7 +309,11 @@ __global__ void __launch_bounds__(512, 2) k_bt_rounds(typename B::heap *h, bt_de
 		cc.hint[lane] = 0;
 	}
 	__syncwarp();
-	bt_counters ct = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+	__shared__ unsigned long long s_ct[512 / 32][BT_WORDS];
+	const bt_counters ct = {s_ct[wid]};
+	if (lane < BT_WORDS)
+		ct.n[lane] = 0;
+	__syncwarp();
 	for (uint32_t r = 0; r <= w.rounds; r++) {
 		for (uint64_t base = 0; base < w.items; base += T) {
 			uint64_t g = base + tid;
@@ -325,22 +341,9 @@ __global__ void __launch_bounds__(512, 2) k_bt_rounds(typename B::heap *h, bt_de
 			B::free_block_warp(h, q);
 		}
 	}
-	const uint32_t mask = 0xffffffffu;
-	unsigned long long v[10] = {__reduce_add_sync(mask, ct.mallocs), __reduce_add_sync(mask, ct.frees),
-				    __reduce_add_sync(mask, ct.nulls), __reduce_add_sync(mask, ct.bad), 0, 0,
-				    __reduce_add_sync(mask, ct.hits), __reduce_add_sync(mask, ct.puts),
-				    __reduce_add_sync(mask, ct.retired), __reduce_add_sync(mask, ct.refused)};
-	unsigned long long f = ct.fill, vb = ct.verify;
-	for (int d = 16; d > 0; d >>= 1) {
-		f += __shfl_down_sync(mask, f, d);
-		vb += __shfl_down_sync(mask, vb, d);
-	}
-	v[4] = f;
-	v[5] = vb;
-	if (lane == 0)
-		for (int k = 0; k < 10; k++)
-			if (v[k])
-				atomicAdd(&w.stats[k], v[k]);
+	__syncwarp();
+	if (lane < BT_WORDS && ct.n[lane])
+		atomicAdd(&w.stats[lane], ct.n[lane]);
 }
 
 __global__ void k_bt_begin(bt_dev w)

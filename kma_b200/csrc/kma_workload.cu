@@ -70,7 +70,11 @@ __device__ __forceinline__ uint32_t c2_size(uint64_t d) { return 8u << (uint32_t
 template <int MODE>
 __device__ __forceinline__ void *wl_malloc(kma_heap *h, size_t n, kma_tally *tl, uint32_t *hint)
 {
-	return (MODE & KMA_MODE_WARP) ? kma_malloc_warp(h, n, (MODE & KMA_MODE_PROFILE) ? tl : nullptr, hint)
+	/* without the sweep: the programs draw every class equally often, few of
+	 * them with many slots, and make 1.2 claims to a reservation; the sweep's
+	 * registers cost this kernel more (config 2: 7.29 ms with it, 6.40
+	 * without) */
+	return (MODE & KMA_MODE_WARP) ? kma_malloc_warp_t<false>(h, n, (MODE & KMA_MODE_PROFILE) ? tl : nullptr, hint)
 				      : kma_malloc(h, n);
 }
 template <int MODE>
@@ -82,13 +86,21 @@ __device__ __forceinline__ void wl_free(kma_heap *h, void *p)
 		kma_free(h, p);
 }
 
+/* A thread's counters, in shared memory: they are written a few times a round
+ * and would be six of a thread's 64 registers. */
+enum { CT_MALLOCS, CT_FREES, CT_NULLS, CT_BAD, CT_FILL, CT_VERIFY, CT_WORDS };
+#define WL_BLOCK 256
 struct wl_counters {
-	uint32_t mallocs, frees, nulls, bad, fill, verify;
+	uint32_t *n; /* this thread's words, WL_BLOCK apart */
 	unsigned long long cyc[4];
 	kma_tally tl;
 	uint32_t *hint; /* the warp's kma_malloc_warp hint words (shared memory), or NULL */
 };
 
+__device__ __forceinline__ void count(wl_counters &ct, uint32_t k, uint32_t x)
+{
+	ct.n[k * WL_BLOCK] += x;
+}
 template <int MODE>
 __device__ __forceinline__ void phase(wl_counters &ct, int k, long long &t0)
 {
@@ -115,20 +127,20 @@ __device__ __forceinline__ void c1_round(kma_heap *h, uint32_t mask, uint32_t la
 	void *p = NULL;
 	if (act) {
 		p = wl_malloc<MODE>(h, n, &ct.tl, ct.hint);
-		ct.mallocs++;
+		count(ct, CT_MALLOCS, 1);
 		it.hash = hash_step(it.hash, p ? (int64_t)((unsigned char *)p - h->sb_base) : -1);
 		if (!p)
-			ct.nulls++;
+			count(ct, CT_NULLS, 1);
 	}
 	__syncwarp(mask);
 	coop_fill(mask, lane, p, n, (uint32_t)g);
 	if (coop_verify(mask, lane, p, n, (uint32_t)g))
-		ct.bad++;
+		count(ct, CT_BAD, 1);
 	wl_free<MODE>(h, p);
 	if (p) {
-		ct.frees++;
-		ct.fill += n;
-		ct.verify += n;
+		count(ct, CT_FREES, 1);
+		count(ct, CT_FILL, n);
+		count(ct, CT_VERIFY, n);
 	}
 }
 
@@ -153,13 +165,13 @@ __device__ __forceinline__ void c2_free_packed(kma_heap *h, const wl_dev &w, uin
 			qn = w.live_size[e];
 		}
 		if (coop_verify(full, lane, q, qn, (uint32_t)o_g))
-			ct.bad++;
+			count(ct, CT_BAD, 1);
 		phase<MODE>(ct, 2, t0);
 		wl_free<MODE>(h, q);
 		phase<MODE>(ct, 3, t0);
 		if (q) {
-			ct.frees++;
-			ct.verify += qn;
+			count(ct, CT_FREES, 1);
+			count(ct, CT_VERIFY, qn);
 		}
 	}
 	/* other lanes read this lane's live table above; it is compacted next */
@@ -186,11 +198,11 @@ __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t 
 			qn = w.live_size[g];
 		}
 		if (coop_verify(mask, lane, q, qn, tag))
-			ct.bad++;
+			count(ct, CT_BAD, 1);
 		wl_free<MODE>(h, q);
 		if (full) {
-			ct.frees++;
-			ct.verify += qn;
+			count(ct, CT_FREES, 1);
+			count(ct, CT_VERIFY, qn);
 			for (uint32_t i = 1; i < WL_CAP; i++) {
 				w.live_off[(i - 1) * items + g] = w.live_off[i * items + g];
 				w.live_size[(i - 1) * items + g] = w.live_size[i * items + g];
@@ -201,16 +213,16 @@ __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t 
 	void *p = NULL;
 	if (act) {
 		p = wl_malloc<MODE>(h, n, &ct.tl, ct.hint);
-		ct.mallocs++;
+		count(ct, CT_MALLOCS, 1);
 		int64_t off = p ? (int64_t)((unsigned char *)p - h->sb_base) : -1;
 		it.hash = hash_step(it.hash, off);
 		if (p) {
 			w.live_off[(uint64_t)it.nlive * items + g] = (unsigned long long)off;
 			w.live_size[(uint64_t)it.nlive * items + g] = n;
 			it.nlive++;
-			ct.fill += n;
+			count(ct, CT_FILL, n);
 		} else {
-			ct.nulls++;
+			count(ct, CT_NULLS, 1);
 		}
 	}
 	__syncwarp(mask);
@@ -239,13 +251,13 @@ __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t 
 			qn = w.live_size[(uint64_t)i * items + g];
 		}
 		if (coop_verify(mask, lane, q, qn, tag))
-			ct.bad++;
+			count(ct, CT_BAD, 1);
 		phase<MODE>(ct, 2, t0);
 		wl_free<MODE>(h, q);
 		phase<MODE>(ct, 3, t0);
 		if (q) {
-			ct.frees++;
-			ct.verify += qn;
+			count(ct, CT_FREES, 1);
+			count(ct, CT_VERIFY, qn);
 		}
 	}
 	if (fmask) {
@@ -278,11 +290,11 @@ __device__ __forceinline__ void c2_drain(kma_heap *h, const wl_dev &w, uint32_t 
 			qn = w.live_size[(uint64_t)i * w.items + g];
 		}
 		if (coop_verify(mask, lane, q, qn, (uint32_t)g))
-			ct.bad++;
+			count(ct, CT_BAD, 1);
 		wl_free<MODE>(h, q);
 		if (q) {
-			ct.frees++;
-			ct.verify += qn;
+			count(ct, CT_FREES, 1);
+			count(ct, CT_VERIFY, qn);
 		}
 	}
 	if (act)
@@ -291,12 +303,11 @@ __device__ __forceinline__ void c2_drain(kma_heap *h, const wl_dev &w, uint32_t 
 
 __device__ __forceinline__ void flush_counters(const wl_dev &w, uint32_t mask, uint32_t lane, const wl_counters &ct)
 {
-	uint32_t a = __reduce_add_sync(mask, ct.mallocs);
-	uint32_t b = __reduce_add_sync(mask, ct.frees);
-	uint32_t c = __reduce_add_sync(mask, ct.nulls);
-	uint32_t d = __reduce_add_sync(mask, ct.bad);
-	unsigned long long e = __reduce_add_sync(mask, ct.fill);
-	unsigned long long f = __reduce_add_sync(mask, ct.verify);
+	for (uint32_t k = 0; k < CT_WORDS; k++) {
+		const uint32_t v = __reduce_add_sync(mask, ct.n[k * WL_BLOCK]);
+		if (v && lane == (uint32_t)(__ffs(mask) - 1))
+			atomicAdd(&w.stats[k], (unsigned long long)v);
+	}
 	if (lane == (uint32_t)(__ffs(mask) - 1)) {
 		for (int k = 0; k < 4; k++)
 			if (ct.cyc[k])
@@ -306,14 +317,6 @@ __device__ __forceinline__ void flush_counters(const wl_dev &w, uint32_t mask, u
 		uint32_t v = __reduce_add_sync(mask, ct.tl.n[k]);
 		if (v && lane == (uint32_t)(__ffs(mask) - 1))
 			atomicAdd(&w.stats[16 + k], (unsigned long long)v);
-	}
-	if (lane == (uint32_t)(__ffs(mask) - 1)) {
-		if (a) atomicAdd(&w.stats[0], (unsigned long long)a);
-		if (b) atomicAdd(&w.stats[1], (unsigned long long)b);
-		if (c) atomicAdd(&w.stats[2], (unsigned long long)c);
-		if (d) atomicAdd(&w.stats[3], (unsigned long long)d);
-		if (e) atomicAdd(&w.stats[4], e);
-		if (f) atomicAdd(&w.stats[5], f);
 	}
 }
 
@@ -325,17 +328,20 @@ __device__ __forceinline__ void flush_counters(const wl_dev &w, uint32_t mask, u
  * their rounds and pin their last live blocks while later waves start,
  * which fragments the heap far beyond what concurrent items do.) */
 template <int MODE, bool C2>
-__global__ void __launch_bounds__(256, 4) k_wl_rounds(kma_heap *h, wl_dev w, uint32_t nrounds, int drain)
+__global__ void __launch_bounds__(WL_BLOCK, 4) k_wl_rounds(kma_heap *h, wl_dev w, uint32_t nrounds, int drain)
 {
 	const uint32_t mask = 0xffffffffu;
 	const uint32_t lane = threadIdx.x & 31;
 	const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
 	const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	__shared__ uint32_t s_hint[256 / 32][KMA_MAX_CLASSES];
+	__shared__ uint32_t s_hint[WL_BLOCK / 32][KMA_MAX_CLASSES];
 	if (lane < KMA_MAX_CLASSES)
 		s_hint[threadIdx.x >> 5][lane] = 0;
+	__shared__ uint32_t s_ct[CT_WORDS * WL_BLOCK];
+	for (uint32_t k = 0; k < CT_WORDS; k++)
+		s_ct[k * WL_BLOCK + threadIdx.x] = 0;
 	__syncwarp();
-	wl_counters ct = {0, 0, 0, 0, 0, 0, {0, 0, 0, 0}, {{0, 0, 0, 0, 0, 0, 0, 0}}, s_hint[threadIdx.x >> 5]};
+	wl_counters ct = {s_ct + threadIdx.x, {0, 0, 0, 0}, {{0, 0, 0, 0, 0, 0, 0, 0}}, s_hint[threadIdx.x >> 5]};
 	/* one kernel per program: a kernel carrying both programs' paths
 	 * spilled 148 bytes per thread at the 64-register cap, the config-2
 	 * one alone 48 */
@@ -391,7 +397,10 @@ __global__ void k_wl_serial(kma_heap *h, wl_dev w, uint32_t nrounds, int round_m
 	if (blockIdx.x != 0 || threadIdx.x != 0)
 		return;
 	const uint32_t mask = 1u;
-	wl_counters ct = {0, 0, 0, 0, 0, 0, {0, 0, 0, 0}, {{0, 0, 0, 0, 0, 0, 0, 0}}, nullptr};
+	__shared__ uint32_t s_ct[CT_WORDS * WL_BLOCK];
+	for (uint32_t k = 0; k < CT_WORDS; k++)
+		s_ct[k * WL_BLOCK] = 0;
+	wl_counters ct = {s_ct, {0, 0, 0, 0}, {{0, 0, 0, 0, 0, 0, 0, 0}}, nullptr};
 	if (!round_major) {
 		for (uint64_t g = 0; g < w.items; g++) {
 			wl_item it = {w.rng[g], w.hash[g], w.nlive[g]};
@@ -426,12 +435,8 @@ __global__ void k_wl_serial(kma_heap *h, wl_dev w, uint32_t nrounds, int round_m
 				w.nlive[g] = it.nlive;
 			}
 	}
-	w.stats[0] += ct.mallocs;
-	w.stats[1] += ct.frees;
-	w.stats[2] += ct.nulls;
-	w.stats[3] += ct.bad;
-	w.stats[4] += ct.fill;
-	w.stats[5] += ct.verify;
+	for (uint32_t k = 0; k < CT_WORDS; k++)
+		w.stats[k] += ct.n[k * WL_BLOCK];
 }
 
 __global__ void k_wl_begin(wl_dev w, uint64_t seed, const uint64_t *seeds)
