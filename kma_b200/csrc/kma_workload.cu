@@ -90,6 +90,7 @@ __device__ __forceinline__ void wl_free(kma_heap *h, void *p)
  * and would be six of a thread's 64 registers. */
 enum { CT_MALLOCS, CT_FREES, CT_NULLS, CT_BAD, CT_FILL, CT_VERIFY, CT_WORDS };
 #define WL_BLOCK 256
+#define WL_WIDE_SLOTS 6
 struct wl_counters {
 	uint32_t *n; /* this thread's words, WL_BLOCK apart */
 	unsigned long long cyc[4];
@@ -118,7 +119,7 @@ struct wl_item {
 };
 
 /* C1 round (every lane in `mask` takes part; act = this lane has an item) */
-template <int MODE>
+template <int MODE, int SLOTS>
 __device__ __forceinline__ void c1_round(kma_heap *h, uint32_t mask, uint32_t lane, bool act, uint64_t g,
 		wl_item &it, wl_counters &ct)
 {
@@ -134,7 +135,7 @@ __device__ __forceinline__ void c1_round(kma_heap *h, uint32_t mask, uint32_t la
 	}
 	__syncwarp(mask);
 	coop_fill(mask, lane, p, n, (uint32_t)g);
-	if (coop_verify(mask, lane, p, n, (uint32_t)g))
+	if (coop_verify<SLOTS>(mask, lane, p, n, (uint32_t)g))
 		count(ct, CT_BAD, 1);
 	wl_free<MODE>(h, p);
 	if (p) {
@@ -147,7 +148,7 @@ __device__ __forceinline__ void c1_round(kma_heap *h, uint32_t mask, uint32_t la
 /* The whole warp's frees of one C2 round (bit i of a lane's fmask: entry
  * i of its live table), packed 32 to a pass (warp_pack); each block is
  * verified against its owner's tag and freed by the lane that takes it. */
-template <int MODE>
+template <int MODE, int SLOTS>
 __device__ __forceinline__ void c2_free_packed(kma_heap *h, const wl_dev &w, uint32_t lane, uint64_t g,
 		uint32_t fmask, wl_counters &ct, long long &t0)
 {
@@ -164,7 +165,7 @@ __device__ __forceinline__ void c2_free_packed(kma_heap *h, const wl_dev &w, uin
 			q = h->sb_base + w.live_off[e];
 			qn = w.live_size[e];
 		}
-		if (coop_verify(full, lane, q, qn, (uint32_t)o_g))
+		if (coop_verify<SLOTS>(full, lane, q, qn, (uint32_t)o_g))
 			count(ct, CT_BAD, 1);
 		phase<MODE>(ct, 2, t0);
 		wl_free<MODE>(h, q);
@@ -179,7 +180,7 @@ __device__ __forceinline__ void c2_free_packed(kma_heap *h, const wl_dev &w, uin
 }
 
 /* C2 round */
-template <int MODE>
+template <int MODE, int SLOTS>
 __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t mask, uint32_t lane, bool act,
 		uint64_t g, wl_item &it, wl_counters &ct)
 {
@@ -197,7 +198,7 @@ __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t 
 			q = h->sb_base + w.live_off[g];
 			qn = w.live_size[g];
 		}
-		if (coop_verify(mask, lane, q, qn, tag))
+		if (coop_verify<SLOTS>(mask, lane, q, qn, tag))
 			count(ct, CT_BAD, 1);
 		wl_free<MODE>(h, q);
 		if (full) {
@@ -239,7 +240,7 @@ __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t 
 	uint32_t fmask = nl ? ((uint32_t)bits & (nl >= 32 ? 0xffffffffu : ((1u << nl) - 1u))) : 0u;
 	uint32_t npass = mask == 0xffffffffu ? 0u : __reduce_max_sync(mask, (uint32_t)__popc(fmask));
 	if (mask == 0xffffffffu)
-		c2_free_packed<MODE>(h, w, lane, g, fmask, ct, t0);
+		c2_free_packed<MODE, SLOTS>(h, w, lane, g, fmask, ct, t0);
 	uint32_t rest = fmask;
 	for (uint32_t pass = 0; pass < npass; pass++) {
 		void *q = NULL;
@@ -250,7 +251,7 @@ __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t 
 			q = h->sb_base + w.live_off[(uint64_t)i * items + g];
 			qn = w.live_size[(uint64_t)i * items + g];
 		}
-		if (coop_verify(mask, lane, q, qn, tag))
+		if (coop_verify<SLOTS>(mask, lane, q, qn, tag))
 			count(ct, CT_BAD, 1);
 		phase<MODE>(ct, 2, t0);
 		wl_free<MODE>(h, q);
@@ -276,7 +277,7 @@ __device__ __forceinline__ void c2_round(kma_heap *h, const wl_dev &w, uint32_t 
 	}
 }
 
-template <int MODE>
+template <int MODE, int SLOTS>
 __device__ __forceinline__ void c2_drain(kma_heap *h, const wl_dev &w, uint32_t mask, uint32_t lane, bool act,
 		uint64_t g, wl_item &it, wl_counters &ct)
 {
@@ -289,7 +290,7 @@ __device__ __forceinline__ void c2_drain(kma_heap *h, const wl_dev &w, uint32_t 
 			q = h->sb_base + w.live_off[(uint64_t)i * w.items + g];
 			qn = w.live_size[(uint64_t)i * w.items + g];
 		}
-		if (coop_verify(mask, lane, q, qn, (uint32_t)g))
+		if (coop_verify<SLOTS>(mask, lane, q, qn, (uint32_t)g))
 			count(ct, CT_BAD, 1);
 		wl_free<MODE>(h, q);
 		if (q) {
@@ -327,8 +328,10 @@ __device__ __forceinline__ void flush_counters(const wl_dev &w, uint32_t mask, u
  * (Launching one thread per item instead lets early waves finish all
  * their rounds and pin their last live blocks while later waves start,
  * which fragments the heap far beyond what concurrent items do.) */
-template <int MODE, bool C2>
-__global__ void __launch_bounds__(WL_BLOCK, 4) k_wl_rounds(kma_heap *h, wl_dev w, uint32_t nrounds, int drain)
+/* PER_SM: blocks an SM must hold, 4 (64 registers a thread) or, when half the
+ * GPU's threads hold every item, 2 (wl_per_sm). */
+template <int MODE, bool C2, int PER_SM>
+__global__ void __launch_bounds__(WL_BLOCK, PER_SM) k_wl_rounds(kma_heap *h, wl_dev w, uint32_t nrounds, int drain)
 {
 	const uint32_t mask = 0xffffffffu;
 	const uint32_t lane = threadIdx.x & 31;
@@ -346,6 +349,7 @@ __global__ void __launch_bounds__(WL_BLOCK, 4) k_wl_rounds(kma_heap *h, wl_dev w
 	 * spilled 148 bytes per thread at the 64-register cap, the config-2
 	 * one alone 48 */
 	const bool c2 = C2;
+	constexpr int SLOTS = PER_SM == 2 ? WL_WIDE_SLOTS : WL_VERIFY_SLOTS;
 	{
 		for (uint32_t r = 0; r <= nrounds; r++) {
 			if (r == nrounds && !(drain && c2))
@@ -358,11 +362,11 @@ __global__ void __launch_bounds__(WL_BLOCK, 4) k_wl_rounds(kma_heap *h, wl_dev w
 				it.hash = act ? w.hash[g] : 0;
 				it.nlive = act ? w.nlive[g] : 0;
 				if (r == nrounds)
-					c2_drain<MODE>(h, w, mask, lane, act, g, it, ct);
+					c2_drain<MODE, SLOTS>(h, w, mask, lane, act, g, it, ct);
 				else if (c2)
-					c2_round<MODE>(h, w, mask, lane, act, g, it, ct);
+					c2_round<MODE, SLOTS>(h, w, mask, lane, act, g, it, ct);
 				else
-					c1_round<MODE>(h, mask, lane, act, g, it, ct);
+					c1_round<MODE, SLOTS>(h, mask, lane, act, g, it, ct);
 				if (act) {
 					w.rng[g] = it.rng;
 					w.hash[g] = it.hash;
@@ -374,26 +378,46 @@ __global__ void __launch_bounds__(WL_BLOCK, 4) k_wl_rounds(kma_heap *h, wl_dev w
 	flush_counters(w, mask, lane, ct);
 }
 
-/* The rounds kernel of a call style for a program (config 2, or config 1). */
+typedef void (*wl_rounds_fn)(kma_heap *, wl_dev, uint32_t, int);
+
 template <int MODE>
-const void *wl_rounds_fn(bool c2)
-{
-	return c2 ? (const void *)k_wl_rounds<MODE, true> : (const void *)k_wl_rounds<MODE, false>;
-}
-template <int MODE>
-void wl_rounds_launch(bool c2, uint32_t nb, uint32_t bd, cudaStream_t st, kma_heap *h, const wl_dev &d,
-		      uint32_t nrounds, int drain)
+wl_rounds_fn wl_rounds_of(bool c2, bool wide)
 {
 	if (c2)
-		k_wl_rounds<MODE, true><<<nb, bd, 0, st>>>(h, d, nrounds, drain);
-	else
-		k_wl_rounds<MODE, false><<<nb, bd, 0, st>>>(h, d, nrounds, drain);
+		return wide ? k_wl_rounds<MODE, true, 2> : k_wl_rounds<MODE, true, 4>;
+	return wide ? k_wl_rounds<MODE, false, 2> : k_wl_rounds<MODE, false, 4>;
+}
+
+/* Launch the rounds kernel of a call style and a program (config 2, or config
+ * 1) as a persistent grid: no more blocks than stay resident on all SMs.
+ *
+ * When there are no more items than 2 blocks an SM hold, the instantiation
+ * with 128 registers a thread runs them: nothing spills, and six vectors are
+ * in flight in the verify instead of three (50021 items, per thread / warp
+ * calls: 1.10 and 0.87 ms a launch instead of 1.17 and 0.90).  With more, the missing warps cost more (config 2
+ * with 24 warps an SM: +9%). */
+int wl_rounds_launch(const wl_dev &d, kma_heap *h, int device, uint32_t nrounds, int mode, uint32_t bd, int drain,
+		cudaStream_t st)
+{
+	int per_sm = 0, sms = 0;
+	KMA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+	const bool c2 = d.program == KMA_WL_C2, wide = d.items <= (uint64_t)sms * 2 * WL_BLOCK;
+	const wl_rounds_fn fns[4] = {wl_rounds_of<0>(c2, wide), wl_rounds_of<1>(c2, wide), wl_rounds_of<2>(c2, wide),
+				     wl_rounds_of<3>(c2, wide)};
+	KMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fns[mode], (int)bd, 0));
+	const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)(sms > 0 ? sms : 1);
+	uint64_t nb = (d.items + bd - 1) / bd;
+	nb = nb < 1 ? 1 : nb > resident ? resident : nb;
+	fns[mode]<<<(uint32_t)nb, bd, 0, st>>>(h, d, nrounds, drain);
+	KMA_CUDA(cudaGetLastError());
+	return KMA_OK;
 }
 
 /* One thread runs every item (round_major: round by round). */
 template <int MODE>
 __global__ void k_wl_serial(kma_heap *h, wl_dev w, uint32_t nrounds, int round_major)
 {
+	constexpr int SLOTS = WL_VERIFY_SLOTS;
 	if (blockIdx.x != 0 || threadIdx.x != 0)
 		return;
 	const uint32_t mask = 1u;
@@ -406,12 +430,12 @@ __global__ void k_wl_serial(kma_heap *h, wl_dev w, uint32_t nrounds, int round_m
 			wl_item it = {w.rng[g], w.hash[g], w.nlive[g]};
 			for (uint32_t r = 0; r < nrounds; r++) {
 				if (w.program == KMA_WL_C1)
-					c1_round<MODE>(h, mask, 0, true, g, it, ct);
+					c1_round<MODE, SLOTS>(h, mask, 0, true, g, it, ct);
 				else
-					c2_round<MODE>(h, w, mask, 0, true, g, it, ct);
+					c2_round<MODE, SLOTS>(h, w, mask, 0, true, g, it, ct);
 			}
 			if (w.program == KMA_WL_C2)
-				c2_drain<MODE>(h, w, mask, 0, true, g, it, ct);
+				c2_drain<MODE, SLOTS>(h, w, mask, 0, true, g, it, ct);
 			w.rng[g] = it.rng;
 			w.hash[g] = it.hash;
 			w.nlive[g] = it.nlive;
@@ -421,9 +445,9 @@ __global__ void k_wl_serial(kma_heap *h, wl_dev w, uint32_t nrounds, int round_m
 			for (uint64_t g = 0; g < w.items; g++) {
 				wl_item it = {w.rng[g], w.hash[g], w.nlive[g]};
 				if (w.program == KMA_WL_C1)
-					c1_round<MODE>(h, mask, 0, true, g, it, ct);
+					c1_round<MODE, SLOTS>(h, mask, 0, true, g, it, ct);
 				else
-					c2_round<MODE>(h, w, mask, 0, true, g, it, ct);
+					c2_round<MODE, SLOTS>(h, w, mask, 0, true, g, it, ct);
 				w.rng[g] = it.rng;
 				w.hash[g] = it.hash;
 				w.nlive[g] = it.nlive;
@@ -431,7 +455,7 @@ __global__ void k_wl_serial(kma_heap *h, wl_dev w, uint32_t nrounds, int round_m
 		if (w.program == KMA_WL_C2)
 			for (uint64_t g = 0; g < w.items; g++) {
 				wl_item it = {w.rng[g], w.hash[g], w.nlive[g]};
-				c2_drain<MODE>(h, w, mask, 0, true, g, it, ct);
+				c2_drain<MODE, SLOTS>(h, w, mask, 0, true, g, it, ct);
 				w.nlive[g] = it.nlive;
 			}
 	}
@@ -583,25 +607,7 @@ static int wl_launch(kma_wl_t w, uint32_t nrounds, int mode, uint32_t bd, int dr
 	if (bd % 32 || bd > 256)
 		return KMA_EINVAL;
 	kma_device_guard g(w->heap->device);
-	cudaStream_t st = kma_stream(stream);
-	uint32_t nb = wl_blocks(w->d.items, bd);
-	/* persistent grid: no more blocks than stay resident on all SMs */
-	int per_sm = 0, sms = 0;
-	const bool c2 = w->d.program == KMA_WL_C2;
-	const void *fns[4] = {wl_rounds_fn<0>(c2), wl_rounds_fn<1>(c2), wl_rounds_fn<2>(c2), wl_rounds_fn<3>(c2)};
-	KMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns[mode], (int)bd, 0));
-	KMA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, w->heap->device));
-	uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)(sms > 0 ? sms : 1);
-	if (nb > resident)
-		nb = (uint32_t)resident;
-	switch (mode) {
-	case 0: wl_rounds_launch<0>(c2, nb, bd, st, w->heap->dh, w->d, nrounds, drain); break;
-	case 1: wl_rounds_launch<1>(c2, nb, bd, st, w->heap->dh, w->d, nrounds, drain); break;
-	case 2: wl_rounds_launch<2>(c2, nb, bd, st, w->heap->dh, w->d, nrounds, drain); break;
-	default: wl_rounds_launch<3>(c2, nb, bd, st, w->heap->dh, w->d, nrounds, drain); break;
-	}
-	KMA_CUDA(cudaGetLastError());
-	return KMA_OK;
+	return wl_rounds_launch(w->d, w->heap->dh, w->heap->device, nrounds, mode, bd, drain, kma_stream(stream));
 }
 
 extern "C" int kma_wl_rounds(kma_wl_t w, uint32_t nrounds, int mode, uint32_t block_dim, void *stream)
@@ -870,19 +876,9 @@ extern "C" int kma_wl_run_noalloc(kma_heap_t h, int program, uint64_t items, con
 		else
 			k_wl_serial<KMA_MODE_PLAIN><<<1, 1, 0, st>>>(h->dh, d, nrounds, 1);
 	} else {
-		uint32_t nb = wl_blocks(items, 256);
-		int per_sm = 0, sms = 0;
-		const bool c2 = d.program == KMA_WL_C2;
-		const void *fn = mode == KMA_MODE_WARP ? wl_rounds_fn<KMA_MODE_WARP>(c2) : wl_rounds_fn<KMA_MODE_PLAIN>(c2);
-		KMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
-		KMA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-		uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)(sms > 0 ? sms : 1);
-		if (nb > resident)
-			nb = (uint32_t)resident;
-		if (mode == KMA_MODE_WARP)
-			wl_rounds_launch<KMA_MODE_WARP>(c2, nb, 256, st, h->dh, d, nrounds, 1);
-		else
-			wl_rounds_launch<KMA_MODE_PLAIN>(c2, nb, 256, st, h->dh, d, nrounds, 1);
+		rc = wl_rounds_launch(d, h->dh, h->device, nrounds, mode, WL_BLOCK, 1, st);
+		if (rc != KMA_OK)
+			return rc;
 	}
 	k_noalloc_finish<<<1, 1024, 0, st>>>(d.stats, hashes_dev, items, stats_dev);
 	KMA_CUDA(cudaGetLastError());

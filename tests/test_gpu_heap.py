@@ -250,3 +250,22 @@ def test_verify_sees_every_damaged_word(mode):
         wl.drain(mode)
         assert wl.stats()["bad_tags"] == len(hit)
         assert h.error_flags() == 0
+
+
+@pytest.mark.parametrize("items", [1, 33, 148 * 512, 148 * 512 + 1])
+@pytest.mark.parametrize("program", [WL_C1, WL_C2])
+def test_rounds_kernels_agree(program, items):
+    """Both call styles count the same work, on either side of the item count
+    up to which the kernels with 128 registers a thread run."""
+    seen = []
+    for mode in MODES:
+        with Heap(65536, 14) as h, Workload(h, program, items) as wl:
+            wl.begin(0x51 + items)
+            wl.rounds(5, mode)
+            wl.drain(mode)
+            st = wl.stats()
+            assert st["mallocs"] == st["frees"] == items * 5
+            assert st["nulls"] == st["bad_tags"] == 0 and st["fill_bytes"] == st["verify_bytes"] > 0
+            assert ins.check_canonical_empty(h.snapshot(), h.bitmaps()) == []
+            seen.append(st["fill_bytes"])
+    assert seen[0] == seen[1]
