@@ -75,15 +75,13 @@ struct gr_dev {
 	uint32_t *qerr;
 };
 
-/* clGraph_node_ensure (tb_clTree.cl:12-38); NULL when the heap is out of
- * blocks (the reference retries forever there) */
+/* The rest of clGraph_node_ensure (tb_clTree.cl:12-38) for a key that was not
+ * in the tree when looked up; NULL when the heap is out of blocks (the
+ * reference retries forever there) */
 template <class B>
-__device__ gr_node *gr_ensure(const gr_dev<B> &g, uint32_t key, unsigned long long &lost, unsigned long long &nulls)
+__device__ gr_node *gr_insert(const gr_dev<B> &g, uint32_t key, unsigned long long &lost, unsigned long long &nulls)
 {
 	for (int tries = 0; tries < 1 << 20; tries++) {
-		kma_cltree_node *t = kma_cltree_get(g.tree, key);
-		if (t)
-			return gr_of_tree(t);
 		void *b = B::alloc(g.h, gr_layout<B>::node_req);
 		if (!b) {
 			nulls++;
@@ -93,7 +91,6 @@ __device__ gr_node *gr_ensure(const gr_dev<B> &g, uint32_t key, unsigned long lo
 		gr_node *n = reinterpret_cast<gr_node *>(((uintptr_t)b + al) & ~al);
 		n->tree.key = key;
 		kma_clqueue_init(&n->links);
-		__threadfence();
 		if (kma_cltree_add(g.tree, &n->tree) == KMA_TREE_INSERTED) {
 			unsigned long long i = atomicAdd(g.nreg, 1ull);
 			g.reg[i] = n;
@@ -101,9 +98,52 @@ __device__ gr_node *gr_ensure(const gr_dev<B> &g, uint32_t key, unsigned long lo
 		}
 		B::release(g.h, b);
 		lost++;
+		kma_cltree_node *t = kma_cltree_get(g.tree, key);
+		if (t)
+			return gr_of_tree(t);
 	}
 	atomicOr(g.qerr, KMA_ERR_TIMEOUT);
 	return nullptr;
+}
+
+/* An edge's two ends, looked up side by side: a search is one round trip a
+ * level and nothing else, so two cost what the deeper one does. */
+__device__ __forceinline__ void gr_find_both(kma_cltree *tree, uint32_t a, uint32_t b, gr_node **na, gr_node **nb)
+{
+	using namespace kma_detail;
+	const unsigned long long root = ld_relaxed64(&tree->root);
+	unsigned long long *la = &tree->root, *lb = &tree->root;
+	unsigned long long ca = root, cb = root;
+	bool fa = false, fb = false;
+	while ((ca && !fa) || (cb && !fb)) {
+		kma_cltree_node *xa = reinterpret_cast<kma_cltree_node *>(ca), *xb = reinterpret_cast<kma_cltree_node *>(cb);
+		const bool ga = ca && !fa, gb = cb && !fb;
+		/* a search that has ended reads the other's node again */
+		const tree_step sa(ga ? xa : xb), sb(gb ? xb : xa);
+		if (ga) {
+			if (sa.key == a) {
+				fa = true;
+			} else {
+				la = a < sa.key ? &xa->left : &xa->right;
+				ca = a < sa.key ? sa.left : sa.right;
+			}
+		}
+		if (gb) {
+			if (sb.key == b) {
+				fb = true;
+			} else {
+				lb = b < sb.key ? &xb->left : &xb->right;
+				cb = b < sb.key ? sb.left : sb.right;
+			}
+		}
+	}
+	/* as kma_cltree_get: the links again, by acquire loads */
+	if (fa)
+		ld_acquire64(la);
+	if (fb)
+		ld_acquire64(lb);
+	*na = fa ? gr_of_tree(reinterpret_cast<kma_cltree_node *>(ca)) : nullptr;
+	*nb = fb ? gr_of_tree(reinterpret_cast<kma_cltree_node *>(cb)) : nullptr;
 }
 
 /* clTree_test (tb_clTree.cl:40-85) */
@@ -113,8 +153,16 @@ __global__ void k_gr_build(gr_dev<B> g, const uint32_t *edges, uint64_t n)
 	uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
 	unsigned long long lost = 0, nulls = 0;
 	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-		gr_node *src = gr_ensure(g, edges[2 * i], lost, nulls);
-		gr_node *snk = gr_ensure(g, edges[2 * i + 1], lost, nulls);
+		const uint32_t from = edges[2 * i], to = edges[2 * i + 1];
+		gr_node *src, *snk;
+		gr_find_both(g.tree, from, to, &src, &snk);
+		if (!src) {
+			src = gr_insert(g, from, lost, nulls);
+			if (from == to)
+				snk = src;
+		}
+		if (!snk && (src || from != to))
+			snk = gr_insert(g, to, lost, nulls);
 		void *b = src && snk ? B::alloc(g.h, GR_LINK_REQ) : nullptr;
 		if (!b) {
 			nulls += src && snk;
@@ -124,7 +172,7 @@ __global__ void k_gr_build(gr_dev<B> g, const uint32_t *edges, uint64_t n)
 		unsigned char *item = reinterpret_cast<unsigned char *>(((uintptr_t)b + 7) & ~(uintptr_t)7);
 		g.link[i] = (unsigned long long)item;
 		*reinterpret_cast<uint32_t *>(item + 8) = (uint32_t)(((unsigned char *)snk - B::base(g.h)) >> 3);
-		__threadfence();
+		/* (the append's exchange publishes the sink too) */
 		kma_clqueue_enqueue(&src->links, reinterpret_cast<kma_clqueue_item *>(item), g.qerr);
 	}
 	if (lost)
@@ -300,14 +348,19 @@ __global__ void k_gr_walk(gr_dev<B> g, uint64_t nodes, gr_cut c, unsigned long l
 			   });
 		/* a segment of another source's edges is a link on the wrong queue:
 		 * it is not counted, nor is anything behind it */
-		for (uint32_t hops = 0; next != GR_NO_SEG && hops <= nseg && c.seg[next].key == key; hops++) {
+		for (uint32_t hops = 0; next != GR_NO_SEG && hops <= nseg; hops++) {
+			/* the whole record at once: a hop is one round trip */
 			gr_seg &r = c.seg[next];
+			const uint32_t rkey = r.key, len = r.len, behind = r.next;
+			const unsigned long long rx = r.x, rs = r.s;
+			if (rkey != key)
+				break;
 			if (start)
 				r.pos = start[i] + n;
-			n += r.len;
-			x ^= r.x;
-			s += r.s;
-			next = r.next;
+			n += len;
+			x ^= rx;
+			s += rs;
+			next = behind;
 		}
 		if (counts)
 			counts[i] = n;
