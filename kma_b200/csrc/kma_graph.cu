@@ -186,13 +186,13 @@ __global__ void k_gr_build(gr_dev<B> g, const uint32_t *edges, uint64_t n)
  * load per link, and with skewed edges one queue holds a large share of all
  * links: one thread per node took 30 ms for 2^20 Zipf(1.1) edges, all but a
  * little of it on the hottest node.  So the lists are cut (Helman and JaJa's
- * list ranking): every link whose address hashes to 0 mod `spacing` starts a
- * segment, and its thread walks to the next such link or the queue's end;
- * then a node's thread walks to its first segment and goes on from segment to
- * segment.  Both parts are chains of dependent loads, the first of about
- * spacing * ln(segments) links, the second of (links / spacing) segments, and
- * spacing = sqrt(n) / 8 keeps both below a millisecond (1.4 ms in all where
- * it took 30; spacing 128).
+ * list ranking): every link whose address hashes to 0 mod GR_SPACING starts a
+ * segment, and its thread walks to the next such link or the queue's end,
+ * some GR_SPACING * ln(segments) links at most.  Pointer jumping then gives
+ * every segment the totals from itself to the end of its queue (a chain of
+ * the segments, 600 for the hottest node at a spacing of 128, was 1 of the
+ * walk's 1.6 ms; now 0.4 in all), and a node's thread walks to its first
+ * segment and adds those.
  *
  * While the walk runs, a segment's first link holds the segment's number in
  * place of its sink, which the segment keeps.
@@ -201,16 +201,23 @@ struct gr_seg {
 	unsigned long long item; /* its first link */
 	uint32_t sink8;          /* that link's sink, as a link holds it */
 	uint32_t key;            /* the source of that link's edge */
-	uint32_t len, next;      /* links; the segment behind it, or GR_NO_SEG */
+	unsigned long long end;  /* last segment of a queue: where the queue's
+				    sinks end, ~0 when no node leads to it */
+};
+/* From a segment on: over the segments up to `next` (not included), `last`
+ * being the one before; next GR_NO_SEG: to the end of the queue. */
+struct gr_jump {
+	uint32_t next, last, len, pad;
 	unsigned long long x, s; /* edge hashes */
-	unsigned long long pos;  /* where its sinks go, or ~0 when no queue leads to it */
 };
 #define GR_NO_SEG 0xffffffffu
+#define GR_SPACING 32u
 
 struct gr_cut {
 	gr_seg *seg;
+	gr_jump *jump[2];   /* [cap] each; k_gr_jump leaves its result in jump[0] */
 	unsigned int *nseg; /* may count past cap: the links past it stay ordinary */
-	uint32_t cap, mask; /* mask: spacing - 1 */
+	uint32_t cap;
 	uint32_t n;         /* no queue is longer */
 };
 
@@ -219,9 +226,9 @@ __device__ __forceinline__ uint32_t *gr_sink_word(unsigned long long item)
 	return reinterpret_cast<uint32_t *>(item + 8);
 }
 
-__device__ __forceinline__ bool gr_hits(const gr_cut &c, unsigned long long item)
+__device__ __forceinline__ bool gr_hits(unsigned long long item)
 {
-	return ((uint32_t)((item >> 3) * 0x9E3779B97F4A7C15ull >> 32) & c.mask) == 0;
+	return (uint32_t)((item >> 3) * 0x9E3779B97F4A7C15ull >> 32) % GR_SPACING == 0;
 }
 
 /* The segment that starts at `item` (whose sink word is w), or GR_NO_SEG.
@@ -229,7 +236,7 @@ __device__ __forceinline__ bool gr_hits(const gr_cut &c, unsigned long long item
  * in a link that hits but found the records full. */
 __device__ __forceinline__ uint32_t gr_seg_at(const gr_cut &c, uint32_t nseg, unsigned long long item, uint32_t w)
 {
-	return gr_hits(c, item) && w < nseg && c.seg[w].item == item ? w : GR_NO_SEG;
+	return gr_hits(item) && w < nseg && c.seg[w].item == item ? w : GR_NO_SEG;
 }
 __device__ __forceinline__ uint32_t gr_nseg(const gr_cut &c)
 {
@@ -243,7 +250,7 @@ __global__ void k_gr_cut(gr_dev<B> g, const uint32_t *edges, uint64_t n, gr_cut 
 	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
 	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
 		const unsigned long long item = g.link[i];
-		if (!item || !gr_hits(c, item))
+		if (!item || !gr_hits(item))
 			continue;
 		const uint32_t s = atomicAdd(c.nseg, 1u);
 		if (s >= c.cap)
@@ -252,7 +259,7 @@ __global__ void k_gr_cut(gr_dev<B> g, const uint32_t *edges, uint64_t n, gr_cut 
 		r.item = item;
 		r.sink8 = *gr_sink_word(item);
 		r.key = edges[2 * i];
-		r.pos = ~0ull;
+		r.end = ~0ull;
 		*gr_sink_word(item) = s;
 	}
 }
@@ -311,25 +318,46 @@ __global__ void k_gr_walk_segs(gr_dev<B> g, gr_cut c)
 {
 	const uint32_t nseg = gr_nseg(c), stride = gridDim.x * blockDim.x;
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += stride) {
-		gr_seg &r = c.seg[i];
-		unsigned long long x = 0, s = 0;
+		const gr_seg &r = c.seg[i];
+		gr_jump j;
+		j.x = j.s = 0;
 		const uint32_t key = r.key;
-		uint32_t next;
-		const uint32_t len = gr_run(g, c, nseg, r.item, true, r.sink8, &next, [&](uint32_t, uint32_t sk) {
+		j.len = gr_run(g, c, nseg, r.item, true, r.sink8, &j.next, [&](uint32_t, uint32_t sk) {
 			const uint64_t m = gr_mix(key, sk);
-			x ^= m;
-			s += m;
+			j.x ^= m;
+			j.s += m;
 		});
-		r.len = len;
-		r.next = next;
-		r.x = x;
-		r.s = s;
+		/* a segment of another source's edges is a link on the wrong queue:
+		 * it is not counted, nor is anything behind it */
+		if (j.next != GR_NO_SEG && c.seg[j.next].key != key)
+			j.next = GR_NO_SEG;
+		j.last = i;
+		j.pad = 0;
+		c.jump[0][i] = j;
 	}
 }
 
-/* per node: its links in queue order -> count and edge hashes.  start: the
- * node's place among the sinks (second pass of an export), which also goes
- * to its segments. */
+/* one round of pointer jumping */
+__global__ void k_gr_jump(const gr_jump *in, gr_jump *out, gr_cut c)
+{
+	const uint32_t nseg = gr_nseg(c), stride = gridDim.x * blockDim.x;
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += stride) {
+		gr_jump a = in[i];
+		if (a.next != GR_NO_SEG) {
+			const gr_jump b = in[a.next];
+			a.next = b.next;
+			a.last = b.last;
+			a.len += b.len;
+			a.x ^= b.x;
+			a.s += b.s;
+		}
+		out[i] = a;
+	}
+}
+
+/* per node: its links in queue order -> count and edge hashes.  start (second
+ * pass of an export): the node's place among the sinks, whose end goes to
+ * its queue's last segment. */
 template <class B>
 __global__ void k_gr_walk(gr_dev<B> g, uint64_t nodes, gr_cut c, unsigned long long *counts, const uint64_t *start,
 		unsigned long long *sums /* links, xor, sum */)
@@ -346,33 +374,30 @@ __global__ void k_gr_walk(gr_dev<B> g, uint64_t nodes, gr_cut c, unsigned long l
 				   x ^= m;
 				   s += m;
 			   });
-		/* a segment of another source's edges is a link on the wrong queue:
-		 * it is not counted, nor is anything behind it */
-		for (uint32_t hops = 0; next != GR_NO_SEG && hops <= nseg; hops++) {
-			/* the whole record at once: a hop is one round trip */
-			gr_seg &r = c.seg[next];
-			const uint32_t rkey = r.key, len = r.len, behind = r.next;
-			const unsigned long long rx = r.x, rs = r.s;
-			if (rkey != key)
-				break;
+		if (next != GR_NO_SEG && c.seg[next].key == key) {
+			const gr_jump j = c.jump[0][next];
+			n += j.len;
+			x ^= j.x;
+			s += j.s;
 			if (start)
-				r.pos = start[i] + n;
-			n += len;
-			x ^= rx;
-			s += rs;
-			next = behind;
+				c.seg[j.last].end = start[i] + n;
 		}
 		if (counts)
 			counts[i] = n;
 	}
 	if (start)
 		return;
-	if (n)
+	/* a warp's in one: every node's own, on three words, took 0.4 ms */
+	for (int d = 16; d > 0; d >>= 1) {
+		n += __shfl_down_sync(0xffffffffu, n, d);
+		x ^= __shfl_down_sync(0xffffffffu, x, d);
+		s += __shfl_down_sync(0xffffffffu, s, d);
+	}
+	if ((threadIdx.x & 31) == 0 && n) {
 		atomicAdd(&sums[0], n);
-	if (x)
 		atomicXor(&sums[1], x);
-	if (s)
 		atomicAdd(&sums[2], s);
+	}
 }
 
 /* every node's sinks, in queue order: from its head to its first segment,
@@ -385,9 +410,16 @@ __global__ void k_gr_sinks(gr_dev<B> g, uint64_t nodes, gr_cut c, const uint64_t
 	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nodes + nseg; i += stride) {
 		const bool seg = i >= nodes;
 		const gr_seg *r = &c.seg[seg ? i - nodes : 0];
-		const unsigned long long pos = seg ? r->pos : start[i];
-		if (pos == ~0ull)
-			continue;
+		unsigned long long pos;
+		if (seg) {
+			const gr_jump &j = c.jump[0][i - nodes];
+			pos = c.seg[j.last].end;
+			if (pos == ~0ull)
+				continue;
+			pos -= j.len;
+		} else {
+			pos = start[i];
+		}
 		uint32_t next;
 		gr_run(g, c, nseg, seg ? r->item : (unsigned long long)kma_clqueue_first(&g.reg[i]->links), seg,
 		       seg ? r->sink8 : 0u, &next, [&](uint32_t k, uint32_t sk) { sinks[pos + k] = sk; });
@@ -450,17 +482,13 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	kma_device_guard gd(device);
 	memset(st, 0, sizeof(*st));
 	uint64_t cap = 2 * n;
-	/* segments of the walk: a power of two near sqrt(n) / 8 apart, the records
-	 * for twice as many as the hash should give */
-	uint32_t spacing = 1;
-	while ((uint64_t)spacing * spacing * 128 < n)
-		spacing *= 2;
-	const uint32_t segs = (uint32_t)(2 * n / spacing) + 1024;
+	/* segments of the walk: records for twice as many as the hash should give */
+	const uint32_t segs = (uint32_t)(2 * n / GR_SPACING) + 1024;
 	size_t o_tree = 0, o_reg = 256, o_nreg = o_reg + cap * 8, o_acc = o_nreg + 8, o_err = o_acc + 16,
 	       o_sums = (o_err + 8 + 255) & ~(size_t)255, o_nseg = o_sums + 24, o_tc = o_sums + 64, o_cnt = o_tc + 128, o_start = o_cnt + cap * 8,
 	       o_sinks = o_start + (cap + 1) * 8, o_keys = o_sinks + n * 4, o_offs = (o_keys + cap * 4 + 7) & ~(size_t)7,
 	       o_edges = o_offs + cap * 8, o_link = o_edges + n * 8, o_seg = o_link + n * 8,
-	       total = o_seg + (size_t)segs * sizeof(gr_seg);
+	       o_jump = o_seg + (size_t)segs * sizeof(gr_seg), total = o_jump + 2 * (size_t)segs * sizeof(gr_jump);
 	/* the tree check's work list (16 bytes a node, at most cap nodes) lies over
 	 * the export arrays, which are written after it (44 n + 8 bytes, of which
 	 * it needs 16 cap = 32 n behind a 16-byte boundary) */
@@ -479,7 +507,8 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 	g.acc = (unsigned long long *)(m + o_acc);
 	g.qerr = (uint32_t *)(m + o_err);
 	unsigned long long *sums = (unsigned long long *)(m + o_sums);
-	const gr_cut cut = {(gr_seg *)(m + o_seg), (unsigned int *)(m + o_nseg), segs, spacing - 1, (uint32_t)n};
+	gr_jump *jump = (gr_jump *)(m + o_jump);
+	const gr_cut cut = {(gr_seg *)(m + o_seg), {jump, jump + segs}, (unsigned int *)(m + o_nseg), segs, (uint32_t)n};
 	if (cudaMemset(m, 0, o_reg) != cudaSuccess || cudaMemset(m + o_nreg, 0, o_cnt - o_nreg) != cudaSuccess ||
 	    cudaMemcpy(m + o_edges, edges, n * 8, cudaMemcpyHostToDevice) != cudaSuccess)
 		rc = KMA_ECUDA;
@@ -510,6 +539,11 @@ int graph_build(typename B::heap *dh, int device, uint64_t region_bytes, const u
 		unsigned long long *cnt = (unsigned long long *)(m + o_cnt);
 		k_gr_cut<B><<<eb, 256>>>(g, (const uint32_t *)(m + o_edges), n, cut);
 		k_gr_walk_segs<B><<<sb, 256>>>(g, cut);
+		/* an even number of rounds, 2^rounds segments at least */
+		for (uint32_t r = 0; r == 0 || (1ull << r) < segs; r += 2) {
+			k_gr_jump<<<sb, 256>>>(cut.jump[0], cut.jump[1], cut);
+			k_gr_jump<<<sb, 256>>>(cut.jump[1], cut.jump[0], cut);
+		}
 		k_gr_walk<B><<<gb, 256>>>(g, nodes, cut, keys_out ? cnt : NULL, NULL, sums);
 		if (cudaGetLastError() != cudaSuccess)
 			rc = KMA_ECUDA;
