@@ -28,9 +28,10 @@
 #include "kma_wl_common.cuh"
 
 #define WL_CAP 32
-/* Counter words behind wl_dev.stats: [0..5] kma_wl_stats counters, [8] the
- * hash XOR of kma_wl_stats_get, [10..13] phase cycles, [16..23] tallies.
- * Every scratch layout reserves this many. */
+/* Counter words behind wl_dev.stats: [0..5] kma_wl_stats counters, [8] and [9]
+ * the hash XOR and the block count of a kma_wl_stats_get under way (zero
+ * otherwise), [10..13] phase cycles, [16..23] tallies, [24..30] what
+ * kma_wl_stats_get returns.  Every scratch layout reserves this many. */
 #define WL_STATS_WORDS 32
 
 struct wl_dev {
@@ -50,7 +51,6 @@ struct kma_wl_s {
 	wl_dev d;
 	void *scratch;
 	size_t scratch_bytes;
-	unsigned long long *hash_out; /* device u64 for the XOR reduction */
 };
 
 namespace {
@@ -467,9 +467,7 @@ __global__ void k_wl_begin(wl_dev w, uint64_t seed, const uint64_t *seeds)
 {
 	uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (g == 0) {
-		for (int i = 0; i < 6; i++)
-			w.stats[i] = 0;
-		for (int i = 10; i < WL_STATS_WORDS; i++)
+		for (int i = 0; i < WL_STATS_WORDS; i++)
 			w.stats[i] = 0;
 	}
 	for (; g < w.items; g += (uint64_t)gridDim.x * blockDim.x) {
@@ -479,7 +477,11 @@ __global__ void k_wl_begin(wl_dev w, uint64_t seed, const uint64_t *seeds)
 	}
 }
 
-__global__ void k_wl_hash_xor(const uint64_t *hash, uint64_t items, unsigned long long *out)
+/* The counters and the XOR of the items' hashes, as a kma_wl_stats at
+ * stats + 24: written by the last block, which leaves [8] and [9] zero for the
+ * next call (a memset, this kernel and two copies were 20 of the 250 us of a
+ * config 1 run). */
+__global__ void k_wl_stats(const uint64_t *hash, uint64_t items, unsigned long long *stats)
 {
 	uint64_t x = 0;
 	for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < items;
@@ -488,7 +490,23 @@ __global__ void k_wl_hash_xor(const uint64_t *hash, uint64_t items, unsigned lon
 	uint32_t lo = __reduce_xor_sync(0xffffffffu, (uint32_t)x);
 	uint32_t hi = __reduce_xor_sync(0xffffffffu, (uint32_t)(x >> 32));
 	if ((threadIdx.x & 31) == 0 && (lo | hi))
-		atomicXor(out, ((unsigned long long)hi << 32) | lo);
+		atomicXor(&stats[8], ((unsigned long long)hi << 32) | lo);
+	__syncthreads();
+	if (threadIdx.x != 0)
+		return;
+	__threadfence();
+	if (atomicAdd(&stats[9], 1ull) != gridDim.x - 1)
+		return;
+	__threadfence();
+	kma_wl_stats *out = reinterpret_cast<kma_wl_stats *>(stats + 24);
+	out->mallocs = stats[0];
+	out->frees = stats[1];
+	out->nulls = stats[2];
+	out->bad_tags = stats[3];
+	out->offset_hash = atomicExch(&stats[8], 0ull);
+	out->fill_bytes = stats[4];
+	out->verify_bytes = stats[5];
+	stats[9] = 0;
 }
 
 /* atomics microbenchmark: distinct lines or one word */
@@ -558,7 +576,6 @@ extern "C" int kma_wl_create(kma_heap_t h, int program, uint64_t items, kma_wl_t
 	w->d.live_size = (uint32_t *)(b + off_lsize);
 	w->d.stats = (unsigned long long *)(b + off_stats);
 	w->d.seeds = (uint64_t *)(b + off_seeds);
-	w->hash_out = w->d.stats + 8;
 	if (cudaMemset(w->scratch, 0, total) != cudaSuccess) {
 		cudaFree(w->scratch);
 		free(w);
@@ -642,21 +659,11 @@ extern "C" int kma_wl_stats_get(kma_wl_t w, void *stream, kma_wl_stats *out)
 		return KMA_EINVAL;
 	kma_device_guard g(w->heap->device);
 	cudaStream_t st = kma_stream(stream);
-	unsigned long long buf[6], hx = 0;
-	KMA_CUDA(cudaMemsetAsync(w->hash_out, 0, 8, st));
 	uint32_t nb = wl_blocks(w->d.items, 256);
-	k_wl_hash_xor<<<nb < 148 * 4 ? nb : 148 * 4, 256, 0, st>>>(w->d.hash, w->d.items, w->hash_out);
+	k_wl_stats<<<nb < 148 * 4 ? nb : 148 * 4, 256, 0, st>>>(w->d.hash, w->d.items, w->d.stats);
 	KMA_CUDA(cudaGetLastError());
-	KMA_CUDA(cudaMemcpyAsync(buf, w->d.stats, sizeof(buf), cudaMemcpyDeviceToHost, st));
-	KMA_CUDA(cudaMemcpyAsync(&hx, w->hash_out, 8, cudaMemcpyDeviceToHost, st));
+	KMA_CUDA(cudaMemcpyAsync(out, w->d.stats + 24, sizeof(*out), cudaMemcpyDeviceToHost, st));
 	KMA_CUDA(cudaStreamSynchronize(st));
-	out->mallocs = buf[0];
-	out->frees = buf[1];
-	out->nulls = buf[2];
-	out->bad_tags = buf[3];
-	out->offset_hash = hx;
-	out->fill_bytes = buf[4];
-	out->verify_bytes = buf[5];
 	return KMA_OK;
 }
 
