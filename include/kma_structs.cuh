@@ -260,6 +260,7 @@ struct kma_chain_log {
 	uint32_t mask;
 	uint32_t pad;
 	ulonglong2 *notes;       /* [KMA_LOG_NOTES] {item, record number}: see kma_q::clq_dequeue_v */
+	ulonglong2 *lasts;       /* [mask + 1] {last item of a chain, its record number} */
 
 	/* a record's slot; its entries are read with ld (relaxed) */
 	__device__ __forceinline__ const unsigned long long *clq_record(uint32_t recno) const
@@ -279,23 +280,51 @@ struct kma_chain_log {
 	{
 		return raw(p) & kma_q::PTR_MASK;
 	}
-	/* one of the notes per item (by hash), overwritten freely: a queue needs
-	 * one at a time, its head's */
-	__device__ __forceinline__ ulonglong2 *note_of(unsigned long long item) const
+	/* {item, record number} pairs by the item's hash, overwritten freely: a
+	 * queue needs one note at a time, its head's, and of the chains' last
+	 * items those whose successors are being appended */
+	static __device__ __forceinline__ unsigned long long hash(unsigned long long item)
 	{
-		return &notes[((item >> 3) * 0x9E3779B97F4A7C15ull) >> (64 - KMA_LOG_NOTES_LOG2)];
+		return (item >> 3) * 0x9E3779B97F4A7C15ull;
 	}
-	__device__ __forceinline__ bool resume(unsigned long long item, uint32_t *recno) const
+	static __device__ __forceinline__ bool pair_ld(const ulonglong2 *p, unsigned long long item, uint32_t *recno)
 	{
 		unsigned long long i, r;
-		asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(i), "=l"(r) : "l"(note_of(item)) : "memory");
+		asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(i), "=l"(r) : "l"(p) : "memory");
 		*recno = (uint32_t)r;
 		return i == item;
 	}
-	__device__ __forceinline__ void note(unsigned long long item, uint32_t recno) const
+	static __device__ __forceinline__ void pair_st(ulonglong2 *p, unsigned long long item, uint32_t recno)
 	{
 		asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};"
-			     ::"l"(note_of(item)), "l"(item), "l"((unsigned long long)recno) : "memory");
+			     ::"l"(p), "l"(item), "l"((unsigned long long)recno) : "memory");
+	}
+	__device__ __forceinline__ ulonglong2 *note_of(unsigned long long item) const
+	{
+		return &notes[hash(item) >> (64 - KMA_LOG_NOTES_LOG2)];
+	}
+	__device__ __forceinline__ bool resume(unsigned long long item, uint32_t *recno) const
+	{
+		return pair_ld(note_of(item), item, recno);
+	}
+	__device__ __forceinline__ void note(unsigned long long item, uint32_t recno) const
+	{
+		pair_st(note_of(item), item, recno);
+	}
+	__device__ __forceinline__ ulonglong2 *last_of(unsigned long long item) const
+	{
+		return &lasts[(uint32_t)(hash(item) >> 32) & mask];
+	}
+	__device__ __forceinline__ void last(unsigned long long item, uint32_t recno) { pair_st(last_of(item), item, recno); }
+	__device__ __forceinline__ bool lookup(unsigned long long item, uint32_t *recno) const
+	{
+		return pair_ld(last_of(item), item, recno);
+	}
+	/* (the upper 16 bits of entry 1 alone: little endian) */
+	__device__ __forceinline__ void behind(uint32_t recno, uint32_t bits)
+	{
+		unsigned short *p = reinterpret_cast<unsigned short *>(clq_slot(recno) + 1) + 3;
+		asm volatile("st.relaxed.gpu.global.u16 [%0], %1;" ::"l"(p), "h"((unsigned short)bits) : "memory");
 	}
 	static __device__ __forceinline__ uint32_t ld(const uint32_t *p) { return kma_detail::ld_relaxed(p); }
 	__device__ __forceinline__ uint32_t take() { return atomicAdd(next, 1u) & kma_q::LOG_RECNO_MASK; }
@@ -504,6 +533,8 @@ __device__ inline int kma_clqueue_enqueue_warp(kma_clqueue *q, kma_clqueue_item 
 			link |= gp.rank == 0 ? kma_q::clq_mark_first(recno, gp.size)
 					     : (gp.rank == 1 ? kma_q::clq_mark_second(recno) : 0ull);
 		}
+		if (logged && gp.next == lane)
+			log->last(ip, recno);
 		st_relaxed64(clq_link_head::at(ip), link);
 		/* every lane's link and record entry is visible before the first
 		 * lane's exchange publishes the chain */
@@ -512,10 +543,13 @@ __device__ inline int kma_clqueue_enqueue_warp(kma_clqueue *q, kma_clqueue_item 
 	__syncwarp(active);
 	int r = 0;
 	if (ok && lane == gp.first) {
+		unsigned long long prev = 0;
 		r = kma_q::clq_append<gpu_ops_group, clq_link_head>(&q->head, &q->tail, ip, lip, spin_limit,
-								       logged ? kma_q::clq_mark_into(recno) : 0ull);
+								       logged ? kma_q::clq_mark_into(recno) : 0ull, &prev);
 		if (!r)
 			flag_err(err, KMA_ERR_TIMEOUT);
+		else if (logged)
+			kma_q::clq_log_behind(log, prev, recno);
 	}
 	r = __shfl_sync(active, r, gp.first);
 	return ok ? r : 0;

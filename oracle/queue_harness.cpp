@@ -146,6 +146,23 @@ struct HostLog {
 		note_item[i].store(item, std::memory_order_relaxed);
 		note_rec[i].store(recno, std::memory_order_relaxed);
 	}
+	/* the chains' last items, in the same way */
+	std::atomic<u64> last_item[NOTES] = {}, last_rec[NOTES] = {};
+	void last(u64 item, uint32_t recno)
+	{
+		last_item[note_of(item)].store(item, std::memory_order_relaxed);
+		last_rec[note_of(item)].store(recno, std::memory_order_relaxed);
+	}
+	bool lookup(u64 item, uint32_t *recno)
+	{
+		*recno = (uint32_t)last_rec[note_of(item)].load(std::memory_order_relaxed);
+		return last_item[note_of(item)].load(std::memory_order_relaxed) == item;
+	}
+	void behind(uint32_t recno, uint32_t bits)
+	{
+		uint16_t *p = reinterpret_cast<uint16_t *>(&clq[(size_t)(recno & mask) * 32 + 1]) + 3;
+		__atomic_store_n(p, (uint16_t)bits, __ATOMIC_RELAXED);
+	}
 	const u64 *clq_record(uint32_t recno) const { return &clq[(size_t)(recno & mask) * 32]; }
 	const uint32_t *iq_record(uint32_t recno) const { return &iq[(size_t)(recno & mask) * 32]; }
 	static u64 raw(const u64 *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
@@ -291,9 +308,14 @@ void run_clq(int threads, int chains, int maxc, int batch, double recycle, uint6
 			}
 			__atomic_store_n(&v[j]->next, link, __ATOMIC_RELAXED);
 		}
+		u64 prev = 0;
+		if (logged)
+			g_log.last((u64)v[len - 1], recno);
 		if (!kma_q::clq_append<HostOps, LinkAtItem>(&q[0], &q[1], (u64)v[0], (u64)v[len - 1], LIMIT,
-							     logged ? kma_q::clq_mark_into(recno) : 0ull))
+							     logged ? kma_q::clq_mark_into(recno) : 0ull, &prev))
 			bk.tmo++;
+		else if (logged)
+			kma_q::clq_log_behind(&g_log, prev, recno);
 		bk.enq += len;
 	};
 	auto producer = [&](int p) {

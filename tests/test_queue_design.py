@@ -217,3 +217,16 @@ def test_warp_text_takes_chains_from_the_log(harness, batch):
     rc, st = run(harness, "clq", f"8 5000 -32 -{batch} 0 15 4 0 65536 1 1")
     assert rc == 0 and st.get("ok"), st
     assert st["log_chains"] / st["dequeue_calls"] > 6
+
+
+# records that name the chain behind them: logs that keep every record, that
+# lose some and that lose nearly all (a name may then be another chain's), and
+# batches that end on and inside the chains they name
+@pytest.mark.parametrize("lanes", [1, 2])
+@pytest.mark.parametrize("cfg", ["8 5000 -32 -256 0.02 21 4 0 65536 1", "8 5000 -3 -250 0.02 22 4 0 1024 1",
+                                 "8 5000 -4 -64 0.02 23 4 0.5 2 0", "8 5000 32 256 0.02 24 4 0.5 16 0"])
+def test_named_records_conserve_and_keep_order(harness, cfg, lanes):
+    rc, st = run(harness, "clq", f"{cfg} {lanes}")
+    assert rc == 0 and st.get("ok"), st
+    assert st["taken"] + st["left"] >= st["appended"] > 0
+    assert st["conservation_faults"] == 0 and st["order_faults"] == 0 and st["timeouts"] == 0
