@@ -151,3 +151,20 @@ def test_gpu_serve_degrees_and_blocks(deg_max, gamma, block_dim):
                 assert r["status"] == "ok" and r["nulls"] == 0 and r["mallocs"] == r["frees"] >= n
                 assert (r["checksum"], r["edges"]) == expected_result(sd, n, deg_max, gamma)
         _empty(h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("deg_max,gamma", [(2, 1.05), (4095, 1.05), (65535, 1.05), (65535, 8.0)])
+def test_gpu_serve_degree_steps(deg_max, gamma):
+    """Laws whose steps are wide (two degrees, or all but one so rare that
+    their thresholds are equal) and narrow (65535 degrees, most of them in
+    the last few steps of the table)."""
+    from kma_b200 import Heap
+    from kma_b200.serve import Server
+    nv, seeds = [1, 777, 3000], [deg_max + 1, deg_max + 2, deg_max + 3]
+    with Heap(65536, 14) as h, Server(h, slots=1, max_vertices=3000, deg_max=deg_max, gamma=gamma) as s:
+        res, _ = s.run(nv, seeds)
+        for r, n, sd in zip(res, nv, seeds):
+            assert r["status"] == "ok" and r["nulls"] == 0
+            assert (r["checksum"], r["edges"]) == expected_result(sd, n, deg_max, gamma)
+        _empty(h)
