@@ -168,3 +168,20 @@ def test_gpu_serve_degree_steps(deg_max, gamma):
             assert r["status"] == "ok" and r["nulls"] == 0
             assert (r["checksum"], r["edges"]) == expected_result(sd, n, deg_max, gamma)
         _empty(h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("block_dim", [32, 256, 1024])
+def test_gpu_serve_requests_around_the_gpu_size(block_dim):
+    """Requests that fill the GPU at 32 warps an SM and one vertex more."""
+    import torch
+    from kma_b200 import Heap
+    from kma_b200.serve import Server
+    full = torch.cuda.get_device_properties(0).multi_processor_count * 1024
+    nv, seeds = [full, full + 1], [32, 33]
+    with Heap(65536, 14) as h, Server(h, slots=2, max_vertices=full + 1, block_dim=block_dim) as s:
+        res, _ = s.run(nv, seeds)
+        for r, n, sd in zip(res, nv, seeds):
+            assert r["status"] == "ok" and r["nulls"] == 0 and r["mallocs"] == r["frees"] >= n
+            assert (r["checksum"], r["edges"]) == expected_result(sd, n)
+        _empty(h)
