@@ -915,7 +915,8 @@ __device__ inline void kma_free(kma_heap *h, void *p)
 /* needs a whole superblock takes a fresh one without touching the      */
 /* class table), then claims the bitmap bits one word at a time with    */
 /* one atomicOr per word; the claimed (superblock, word, mask) is       */
-/* broadcast with __shfl_sync and each lane picks its bit by rank.  One */
+/* broadcast with __shfl_sync and each lane picks its bit by rank.  All  */
+/* leaders take these steps side by side, one of each per iteration.  One */
 /* atomic per warp per superblock (and per bitmap word) reaches L2      */
 /* instead of two or three per lane.  A single calling lane follows     */
 /* exactly the plain path's choices.                                    */

@@ -10,13 +10,13 @@
  *
  * Request (seed, N): a random graph on N vertices whose degrees follow a
  * power law P(d) ~ d^-gamma on 1..deg_max (gamma = 2.1) with uint32
- * neighbour ids drawn uniformly from [0, N).  Its three kernels, on the
+ * neighbour ids drawn uniformly from [0, N).  Its two kernels, on the
  * request's slot stream:
  *   build   every vertex grows its own clArrayList of neighbour ids in
  *           pages of 8, 16, 32, ... objects (one heap block per page);
- *   verify  every vertex walks its pages, checks each id against the
- *           seed's draw, and folds its list into the request checksum;
- *   free    every vertex clears its list (all blocks back to the heap).
+ *   finish  every vertex walks its pages, checks each id against the
+ *           seed's draw, folds its list into the request checksum and
+ *           clears the list (all blocks back to the heap).
  * The checksum depends only on (seed, N), never on where the blocks
  * landed, so a request gives the same result alone and in any mix.
  */
@@ -50,7 +50,7 @@ typedef struct kma_serve_req {
 
 #define KMA_SERVE_OK 0
 #define KMA_SERVE_NOMEM 1    /* a page malloc returned NULL (heap exhausted) */
-#define KMA_SERVE_MISMATCH 2 /* verify found a neighbour id that differs */
+#define KMA_SERVE_MISMATCH 2 /* the check found a neighbour id that differs */
 #define KMA_SERVE_TOO_BIG 3  /* N above max_vertices, or larger than the heap */
 
 typedef struct kma_serve_result {
