@@ -836,26 +836,27 @@ __device__ __forceinline__ bool block_locate(const kma_heap *h, const void *p, u
  * free list unless a reservation gets in first: kma.cl:350-367.  The lanes
  * of `active` that have one do it together; every lane of it calls.
  *
- * The home shard of this incarnation was stored before its class slot, and
- * so before any block of it was handed out; a gpu-scope relaxed load issued
- * after the count that made it full is served at L2, where that store
- * already was.  A plain load may be served from this SM's L1, where a line
- * of sb_home read during an earlier incarnation can still sit: the slot of
- * the old home would be cleared and the current one left naming a superblock
- * on the free list. */
+ * The CAS that takes the count away detaches s: from then on, until it is on
+ * the free list, nobody else can reserve from it, recycle it or give it another
+ * home.  So the home is read after that CAS has returned.  Before it, s may be
+ * recycled, formatted for the same class under another shard and freed again,
+ * which the CAS cannot tell from nothing having happened: the old home's slot
+ * would be cleared and the current one left naming a superblock on the free
+ * list.  The home was stored before the state (sb_format), and a gpu-scope
+ * relaxed load is served at L2, where that store already was; a plain one may
+ * be served from this SM's L1, where a line of sb_home read during an earlier
+ * incarnation can still sit. */
 __device__ __forceinline__ void sb_recycle(kma_heap *h, uint32_t active, bool all_free, uint32_t s, uint32_t c,
 		uint32_t full)
 {
-	uint32_t home = 0, seen = 0, old = 0;
-	if (all_free) {
-		home = ld_relaxed16(&h->sb_home[s]);
-		seen = cas_relaxed(&h->sb_state[s], full, st_make(c, st_slots(full), 0));
-	}
-	const bool mine = all_free && seen == full;
+	uint32_t old = 0;
+	bool mine = false;
+	if (all_free)
+		mine = cas_relaxed(&h->sb_state[s], full, st_make(c, st_slots(full), 0)) == full;
 	if (!__any_sync(active, mine))
 		return;
 	if (mine)
-		old = cas_relaxed(cls_word(h, c, home), s + KMA_CLS_BASE, 0);
+		old = cas_relaxed(cls_word(h, c, ld_relaxed16(&h->sb_home[s])), s + KMA_CLS_BASE, 0);
 	if (h->flags & KMA_HEAP_RING)
 		ring_enqueue_lanes(h, active, mine, s, old);
 	else if (mine)

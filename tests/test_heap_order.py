@@ -80,6 +80,53 @@ int main(int, char **argv)
 }
 """
 
+RECYCLE = COMMON + r"""
+#define KMA_HEAP_RING 1u
+#define KMA_CLS_BASE 2u
+struct kma_heap { uint32_t flags; uint16_t sb_home[4]; uint32_t sb_state[4], cls[8]; };
+static kma_heap h;
+static int listed, acts_before;
+static void step() { if (acts_before-- == 0) other(); }
+static uint32_t ld_relaxed16(const uint16_t *p) { step(); return *p; }
+static uint32_t cas_relaxed(uint32_t *p, uint32_t c, uint32_t v)
+{
+	step();
+	uint32_t old = *p;
+	if (old == c)
+		*p = v;
+	return old;
+}
+static uint32_t *cls_word(kma_heap *, uint32_t, uint32_t shard) { return &h.cls[shard]; }
+static bool __any_sync(uint32_t, bool b) { return b; }
+static void ring_enqueue_lanes(kma_heap *, uint32_t, bool want, uint32_t, uint32_t) { listed += want; }
+static void msq_enqueue(kma_heap *, uint32_t) { listed++; }
+%s
+int main(int, char **argv)
+{
+	const uint32_t full = st_make(CLS, 7, 7);
+	h.flags = atoi(argv[2]);
+	h.sb_state[1] = full;
+	h.sb_home[1] = 4;
+	h.cls[4] = 1 + KMA_CLS_BASE;
+	acts_before = atoi(argv[1]); /* accesses before the other thread acts */
+	/* the other thread recycles the superblock, unless it is detached; it is
+	 * formatted again for the same class, under shard 5, and freed again */
+	other = [&] {
+		if (h.sb_state[1] != full)
+			return;
+		h.cls[4] = 0;
+		h.sb_home[1] = 5;
+		h.cls[5] = 1 + KMA_CLS_BASE;
+	};
+	sb_recycle(&h, 1, true, 1, CLS, full);
+	bool bad = listed != 1 || h.sb_state[1] != st_make(CLS, 7, 0);
+	for (uint32_t w : h.cls)
+		bad |= w == 1 + KMA_CLS_BASE; /* no slot names a superblock on the free list */
+	printf("%%s\n", bad ? "bad" : "ok");
+	return bad;
+}
+"""
+
 
 def function(name: str) -> str:
     """The text of the function `name` of kma_device.cuh."""
@@ -105,3 +152,13 @@ def test_a_superblock_is_reserved_from_only_after_its_bitmap(tmp_path):
     for slots, pre_lo in [(1, 0), (2, 1), (31, 30), (32, 1), (33, 32), (64, 40), (509, 477), (2000, 1)]:
         r = subprocess.run([binary, str(slots), str(pre_lo)], capture_output=True, text=True, timeout=60)
         assert r.returncode == 0, (slots, pre_lo, r.stdout)
+
+
+@pytest.mark.parametrize("ring", [0, 1])
+def test_a_recycled_superblock_leaves_its_current_home(tmp_path, ring):
+    """Whenever another thread gets in between: a superblock on the free list
+    is in nobody's class slot."""
+    binary = build(tmp_path, RECYCLE % function("sb_recycle"))
+    for before in range(5):
+        r = subprocess.run([binary, str(before), str(ring)], capture_output=True, text=True, timeout=60)
+        assert r.returncode == 0, (before, r.stdout)
