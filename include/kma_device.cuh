@@ -1086,8 +1086,10 @@ __device__ __forceinline__ sweep_got warp_sweep(kma_heap *h, uint32_t s, uint32_
  * superblock they last reserved from.  Its state is loaded together with the
  * class word on the next call, and if it still serves the request it is
  * reserved from, current or not (hint_serves): the class slot does not get
- * back a detached superblock whose blocks are freed one by one.  Any earlier
- * content is safe, as a reservation's CAS checks class and count. */
+ * back a detached superblock whose blocks are freed one by one.  (Not for a
+ * single calling lane, which follows the reference's choices.)  Words an
+ * earlier call left are safe whatever has become of their superblocks, as a
+ * reservation's CAS checks class and count. */
 template <bool SWEEP>
 __device__ __forceinline__ void *kma_malloc_warp_t(kma_heap *h, size_t size, kma_tally *tl, uint32_t *hint)
 {
@@ -1142,7 +1144,7 @@ __device__ __forceinline__ void *kma_malloc_warp_t(kma_heap *h, size_t size, kma
 				cur = ld_relaxed(cls_word(h, c, shard));
 				if (guess)
 					st = ld_relaxed(&h->sb_state[guess - KMA_CLS_BASE]);
-				if (guess && hint_serves(h, c, slots, want, st)) {
+				if (guess && hint_serves(h, c, slots, want, st) && (active & (active - 1u))) {
 					kind = KMA_R_TAKE;
 					known = true;
 					cur = guess;
