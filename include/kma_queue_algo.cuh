@@ -102,10 +102,13 @@ struct no_log {
 KQ_FN u64 qp_ptr(u64 w) { return w & PTR_MASK; }
 KQ_FN u64 qp_next(u64 w, u64 ptr) { return (((w >> PTR_BITS) + 1ull) << PTR_BITS) | ptr; }
 
-/* A logged chain (at least 3 items) marks the top 16 bits of its first
- * two links: first = CLQ_LOG | (length - 1) << 10 | record number bits
- * 14..23, second = record number bits 0..13 (its top two bits stay clear,
- * so it never reads as a first or into mark).  The append that links the
+/* A logged chain (at least 3 items) marks the top 16 bits of its links, so
+ * that any two that follow one another give its record number: the first and
+ * every second one after it CLQ_LOG | (length - 1) << 10 | record number bits
+ * 14..23 (length - 1: 0 in all but the first), the others record number bits
+ * 0..13 (their top two bits stay clear, so they never read as a first or into
+ * mark).  The last item's link is not the chain's to mark, and a CLQ_LOG mark
+ * whose other half would stand there is left out (clq_mark).  The append that links the
  * chain after the previous tail item marks that link too (the link INTO
  * the chain): CLQ_INTO | record number bits 0..13, so that a dequeuer that
  * reaches the chain over that link has its whole record number without
@@ -118,6 +121,26 @@ KQ_FN u64 clq_mark_first(uint32_t recno, uint32_t len)
 	return CLQ_LOG | ((u64)(((len - 1u) << 10) | ((recno >> 14) & 0x3FFu)) << PTR_BITS);
 }
 KQ_FN u64 clq_mark_second(uint32_t recno) { return (u64)(recno & 0x3FFFu) << PTR_BITS; }
+/* the mark of item i's link in a logged chain of len items */
+KQ_FN u64 clq_mark(uint32_t recno, uint32_t i, uint32_t len)
+{
+	if (i & 1u)
+		return i + 1 < len ? clq_mark_second(recno) : 0ull;
+	return i + 2 < len ? clq_mark_first(recno, i ? 1u : len) : 0ull;
+}
+/* Whether link a and the link b of the item that a names give the number of
+ * one logged chain that both items are in. */
+KQ_FN bool clq_number(u64 a, u64 b, uint32_t *recno)
+{
+	const bool first = (a & CLQ_LOG) != 0;
+	const u64 hi = first ? a : b, lo = first ? b : a;
+	if (!(hi & CLQ_LOG) || (lo & (CLQ_LOG | CLQ_INTO)) || qp_ptr(a) <= POISON || qp_ptr(b) <= POISON)
+		return false;
+	if (!first && ((hi >> (PTR_BITS + 10)) & 31u)) /* b starts the next chain */
+		return false;
+	*recno = (((uint32_t)(hi >> PTR_BITS) & 0x3FFu) << 14) | ((uint32_t)(lo >> PTR_BITS) & 0x3FFFu);
+	return true;
+}
 KQ_FN u64 clq_mark_into(uint32_t recno) { return CLQ_INTO | ((u64)(recno & 0x3FFFu) << PTR_BITS); }
 
 /* Up to k items [hp, ...] of the logged chain that starts at hp (its link
@@ -366,29 +389,40 @@ KQ_FN uint32_t clq_dequeue_n(u64 *headw, u64 *tailw, u64 *out, uint32_t k, uint3
  * bounds a hot queue is the hold, a chain of dependent round trips, so the
  * point is to have fewer of them:
  *   - a record's entries are one load per lane, and so are the links that
- *     prove them, so a chain costs two round trips (its record; its links,
- *     the last of which says where the next chain's record is), or one (see
- *     below), however long it is.  A chain's length stands in its record
- *     (bits 48.. of entry 0), its number's low 14 bits in the link into it;
- *     the bits above are those of the chain before, or one more or less:
- *     chains are appended about in the order of their numbers, and a wrong
- *     guess fails the check;
+ *     prove them, so a chain costs two round trips (its record; its links),
+ *     or one (see below), however long it is.  A chain's length stands in
+ *     every entry of its record (bits 48..), and it writes all 32 of them, 0
+ *     behind its own;
  *   - the hold before leaves a note in the log (`resume`): the record in
- *     which the new head is.  It is read with the head's link, and the
- *     record with the recheck of the head, so that neither costs a round
- *     trip.  The note also finds the place in the middle of a chain, where a
- *     batch that is no multiple of the chains leaves the head for good: no
- *     link there is marked, and a walk is one round trip per item;
- *   - the record of a chain names the one behind it (bits 48.. of entry 1,
- *     written by the append of that one: clq_log_behind), so that the next
+ *     which the new head is.  It is read with the head's link, the record
+ *     with the exchange that takes the head, and the link of the item behind
+ *     the head with the recheck, so that none of them costs a round trip.
+ *     The note also finds the place in the middle of a chain, where a
+ *     batch that is no multiple of the chains leaves the head;
+ *   - the record of a chain has a name: the number of the chain behind it,
+ *     written by the append of that one (clq_log_behind), so that the next
  *     record is on its way while this chain's links are: one round trip a
- *     chain, not two (2^22 items in batches of 256: 190 -> 164 ms).  Like
- *     the record it is only a hint, compared with the link that decides;
+ *     chain, not two (2^22 items in batches of 256: 190 -> 164 ms);
  *   - taken items get their POISON after the head is released: nobody else
  *     writes or reads the link of an item behind a held head that has a
  *     successor, and the caller has the items only when this returns.
- * A walk goes on only to the next marked link.  As everywhere, records and
- * notes are hints, believed only where the queue's links say the same.
+ *
+ * A record's entries are followed before the queue's links can have vouched
+ * for each of them, so it must be certain that they are items of this queue,
+ * behind its held head, and not what the log kept of items that have left
+ * their queue and whose memory may be gone.  It is, when the number of the
+ * record is known to be that of the chain the next item is in, and the record
+ * was read after that chain was appended: its slot then holds what that chain
+ * wrote, or what a later one did, and names the next item only in the first
+ * case.  The number is known
+ *   - from two links of the chain that follow one another (clq_number), which
+ *     the queue's own items carry.  A note is taken for true only so;
+ *   - from the name of the record before, which has both chains' numbers.  It
+ *     was written by an append that found the number of the chain before by
+ *     the item its exchange of the tail gave it (`last`, `lookup`), and a tail
+ *     value is given to one append only: no other chain can follow that one.
+ * Numbers have 24 bits: a chain that stays queued while 2^24 others are
+ * appended through the same log is not told from a later one.
  *
  * Vector policy `V` (32 lanes; on the host, arrays of 32):
  *   reg<T>        one T per lane; x[j] is lane j's (on the GPU: the caller's)
@@ -399,36 +433,35 @@ KQ_FN uint32_t clq_dequeue_n(u64 *headw, u64 *tailw, u64 *out, uint32_t k, uint3
  * Log policy, besides the above:
  *   raw(p)        relaxed load of an entry of clq_record with its length bits
  *   taken_chains(n)        n chains were taken from records (a count)
- *   resume(item, &recno)   whether there is a note for item
+ *   resume(item, &recno)   whether there is a note for item (a hint)
  *   note(item, recno)      leave one
- *   last(item, recno), lookup(item, &recno)   the same for a chain's last item, by its append
- *   behind(recno, low)     record recno is followed by one with these low bits
+ *   last(item, recno), lookup(item, &recno)   the same for a chain's last item, by its append; a
+ *                          pair is written and read in one piece
+ *   name(recno)            the name of record recno (0: none; cleared when the record is written)
+ *   set_name(recno, name)  write it
  * Output `OUT`: run(at, items, first, n) puts items[first .. first+n) at
  * at.., one(at, item) puts one; each_taken(r, f) calls f(item) for those at
  * 1 .. r-1.
  */
-const uint32_t LOG_LOW_BITS = 14;
-const uint32_t LOG_LOW_MASK = (1u << LOG_LOW_BITS) - 1u;
 const int LOG_LEN_SHIFT = PTR_BITS;
 
-/* the number with the low bits `low` that is nearest to ref (mod 2^24) */
-KQ_FN uint32_t log_near(uint32_t ref, uint32_t low)
+/* the name of record recno: chain `behind` follows its chain */
+const u64 LOG_NAMED = 1ull << 63;
+KQ_FN u64 log_name(uint32_t recno, uint32_t behind) { return LOG_NAMED | ((u64)recno << 24) | behind; }
+KQ_FN bool log_named(u64 name, uint32_t recno, uint32_t *behind)
 {
-	const uint32_t half = 1u << (LOG_LOW_BITS - 1);
-	const uint32_t up = (low - ref) & LOG_LOW_MASK; /* steps up from ref */
-	return (up < half ? ref + up : ref + up - (LOG_LOW_MASK + 1u)) & LOG_RECNO_MASK;
+	*behind = (uint32_t)name & LOG_RECNO_MASK;
+	return (name >> 24) == ((LOG_NAMED >> 24) | recno);
 }
 
-const u64 LOG_BEHIND = 1ull << 63;
-
-/* After an append of logged chain recno: tell the record of the chain before
- * it (whose last item is prev), if the log still knows which that is. */
+/* After an append of logged chain recno: name it in the record of the chain
+ * before it (whose last item is prev), if the log still knows which that is. */
 template <class LG>
 KQ_FN void clq_log_behind(LG *log, u64 prev, uint32_t recno)
 {
 	uint32_t r = 0;
 	if (prev && log->lookup(prev, &r))
-		log->behind(r, (uint32_t)(LOG_BEHIND >> PTR_BITS) | (recno & LOG_LOW_MASK));
+		log->set_name(r, log_name(r, recno));
 }
 
 template <class O, class L, class V, class OUT, class LG>
@@ -462,20 +495,46 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 			O::pause(it++);
 			continue;
 		}
+		/* the record of the note, if there is one, beside the exchange */
+		noted = V::one([&] { return noted; });
+		recno = V::one([&] { return recno; });
+		vec raw, item, name; /* (name: the same in every lane; no wait for it here) */
+		typename V::template reg<bool> hit;
+		auto load_record = [&](vec &rec_of, vec &name_of, uint32_t no) {
+			const u64 *rec = log->clq_record(no);
+			V::each([&](uint32_t j) {
+				rec_of[j] = LG::raw(rec + j);
+				name_of[j] = log->name(no);
+			});
+		};
+		if (noted)
+			load_record(raw, name, recno);
 		const u64 nx = V::one([&] { return O::xchg(hl, POISON); });
 		if (nx == POISON) {
 			O::pause(it++);
 			continue;
 		}
-		noted = V::one([&] { return noted; });
-		recno = V::one([&] { return recno; });
-		/* the record of the note, if there is one, beside the recheck */
-		vec raw;
+		/* the link of the item behind the head, where the record agrees on
+		 * what item that is, beside the recheck */
+		u64 second = 0, l1 = 0;
 		if (noted) {
-			const u64 *rec = log->clq_record(recno);
-			V::each([&](uint32_t j) { raw[j] = LG::raw(rec + j); });
+			V::each([&](uint32_t j) {
+				item[j] = qp_ptr(raw[j]);
+				hit[j] = item[j] == hp;
+			});
+			const uint32_t at = V::ballot(hit);
+			const vec next = V::above(item);
+			uint32_t p = 0;
+			while (at && !((at >> p) & 1u))
+				p++;
+			const u64 n = V::get(next, p);
+			second = at && p < LOG_CHAIN_MAX - 1u && n > POISON && n == qp_ptr(nx) ? n : 0ull;
 		}
-		if (V::one([&] { return O::ld(headw); }) != h) {
+		if (V::one([&] {
+			    if (second)
+				    l1 = O::ld_rlx(L::at(second));
+			    return O::ld(headw);
+		    }) != h) {
 			V::one([&] {
 				O::st(hl, nx);
 				return 0u;
@@ -483,36 +542,37 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 			O::pause(it++);
 			continue;
 		}
+		if (noted) {
+			uint32_t no = 0;
+			l1 = V::one([&] { return l1; });
+			noted = second && clq_number(nx, l1, &no) && no == recno;
+		}
 		/* held: cur is the next item to take, curl its link where known */
 		uint32_t r = 0, chains = 0;
-		u64 cur = hp, curl = nx, untried = ~0ull;
-		bool have = noted, end = nx == 0;
+		u64 cur = hp, curl = nx, into = 0, untried = ~0ull;
+		bool have = noted, end = nx == 0; /* have: raw is cur's chain's record, of number recno */
 		while (r < k && !end) {
 			if (have) {
-				const uint32_t len = (uint32_t)(V::get(raw, 0) >> LOG_LEN_SHIFT);
-				vec item, link;
-				typename V::template reg<bool> hit, bad;
 				V::each([&](uint32_t j) {
 					item[j] = qp_ptr(raw[j]);
-					hit[j] = j < len && item[j] == cur;
+					hit[j] = item[j] == cur;
 				});
 				const uint32_t at = V::ballot(hit);
 				uint32_t p = 0;
 				while (at && !((at >> p) & 1u))
 					p++;
-				const uint32_t n = at ? (len < LOG_CHAIN_MAX ? len : LOG_CHAIN_MAX) - p : 0u;
+				const uint32_t len = (uint32_t)(V::get(raw, p) >> LOG_LEN_SHIFT);
+				const uint32_t n = at && p < len && len <= LOG_CHAIN_MAX ? len - p : 0u;
 				uint32_t m = n < k - r ? n : k - r;
 				/* the record behind, beside the links, where more is wanted */
-				const u64 hint = V::get(raw, 1);
-				const bool ahead = at && n < k - r && (hint & LOG_BEHIND);
-				const uint32_t rahead = log_near(recno, (uint32_t)(hint >> PTR_BITS) & LOG_LOW_MASK);
-				vec rawn;
-				if (ahead) {
-					const u64 *rec = log->clq_record(rahead);
-					V::each([&](uint32_t j) { rawn[j] = LG::raw(rec + j); });
-				}
+				uint32_t rahead = 0;
+				const bool named = log_named(V::get(name, 0), recno, &rahead), ahead = named && n < k - r;
+				vec rawn, namen, link;
+				if (ahead)
+					load_record(rawn, namen, rahead);
 				/* the links of the items to take; an entry that is no item
 				 * pointer is not followed */
+				typename V::template reg<bool> bad;
 				V::each([&](uint32_t j) {
 					const bool mine = j >= p && j < p + m;
 					bad[j] = mine && item[j] <= POISON;
@@ -543,13 +603,12 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 						cur = nh;
 						curl = 0;
 						if (whole && !end) {
-							have = (ll & CLQ_INTO) && !(ll & CLQ_LOG);
-							recno = log_near(recno, (uint32_t)(ll >> PTR_BITS) & LOG_LOW_MASK);
-							if (have && ahead && recno == rahead) {
+							into = ll;
+							have = named; /* and read, unless this was the last */
+							recno = named ? rahead : recno;
+							if (ahead) {
 								raw = rawn;
-							} else if (have && r < k) {
-								const u64 *rec = log->clq_record(recno);
-								V::each([&](uint32_t j) { raw[j] = LG::raw(rec + j); });
+								name = namen;
 							}
 						}
 						continue;
@@ -564,18 +623,23 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 			if (curl == 0 || curl == POISON)
 				break; /* cur is the last linked item: it stays, as the head */
 			if ((curl & CLQ_LOG) && log && cur != untried) {
+				/* its chain's number: the other half stands in the link into the
+				 * chain, or in the next link */
 				untried = cur;
-				const u64 second = qp_ptr(curl);
-				const uint32_t lo = V::one([&] {
-					return (uint32_t)(O::ld_rlx(L::at(second)) >> PTR_BITS) & LOG_LOW_MASK;
-				});
-				recno = (((uint32_t)(curl >> PTR_BITS) & 0x3FFu) << LOG_LOW_BITS) | lo;
-				const u64 *rec = log->clq_record(recno);
-				V::each([&](uint32_t j) { raw[j] = LG::raw(rec + j); });
-				have = true;
-				continue;
+				const bool first = ((curl >> (PTR_BITS + 10)) & 31u) != 0;
+				u64 lo = POISON;
+				if (first && (into & CLQ_INTO) && !(into & CLQ_LOG))
+					lo = (into & ~(CLQ_INTO | PTR_MASK)) | qp_ptr(curl);
+				else if (qp_ptr(curl) > POISON)
+					lo = V::one([&] { return O::ld_rlx(L::at(qp_ptr(curl))); });
+				have = clq_number(curl, lo, &recno);
+				if (have) {
+					load_record(raw, name, recno);
+					continue;
+				}
 			}
 			out.one(r++, cur);
+			into = curl;
 			cur = qp_ptr(curl);
 			curl = 0;
 		}

@@ -242,14 +242,15 @@ __device__ __forceinline__ bool lanes_share(uint32_t active, unsigned long long 
  * A log of `mask + 1` records (a power of two), reused round robin.  A
  * warp that appends a chain of its items (kma_clqueue_enqueue_warp: 3 or
  * more items; kma_iqueue_enqueue_warp_shard: 2 or more) writes the items
- * into the next record and marks the chain's first link(s) with the
+ * into the next record and marks the chain's links with the
  * record's number; a warp dequeue that finds a marked chain at the head
  * checks the record against the queue's links with independent loads and
  * takes the chain at once instead of walking it link by link (the
  * algorithm and its checks: kma_queue_algo.cuh).  Records are only hints:
  * a stale or overwritten one fails the check and the dequeue walks.  One
- * log may serve any number of queues of one kind.  No counterpart in the
- * reference.
+ * log may serve any number of queues of one kind, one after the other too:
+ * what it keeps of items that are gone is not followed.  No counterpart in
+ * the reference.
  */
 #define KMA_LOG_NOTES_LOG2 10
 #define KMA_LOG_NOTES (1u << KMA_LOG_NOTES_LOG2)
@@ -261,6 +262,7 @@ struct kma_chain_log {
 	uint32_t pad;
 	ulonglong2 *notes;       /* [KMA_LOG_NOTES] {item, record number}: see kma_q::clq_dequeue_v */
 	ulonglong2 *lasts;       /* [mask + 1] {last item of a chain, its record number} */
+	unsigned long long *names; /* [mask + 1] kma_q::log_name of the records of pointer chains */
 
 	/* a record's slot; its entries are read with ld (relaxed) */
 	__device__ __forceinline__ const unsigned long long *clq_record(uint32_t recno) const
@@ -271,7 +273,7 @@ struct kma_chain_log {
 	{
 		return reinterpret_cast<const uint32_t *>(&rec[(size_t)(recno & mask) * 32]);
 	}
-	/* (entry 0 of a pointer record has the chain's length above the pointer) */
+	/* (an entry of a pointer record has the chain's length above the pointer) */
 	static __device__ __forceinline__ unsigned long long raw(const unsigned long long *p)
 	{
 		return kma_detail::ld_relaxed64(p);
@@ -287,16 +289,19 @@ struct kma_chain_log {
 	{
 		return (item >> 3) * 0x9E3779B97F4A7C15ull;
 	}
+	/* (a 128-bit access is one piece, two 64-bit elements need not be: an item
+	 * of one pair with the number of another would name a wrong chain) */
 	static __device__ __forceinline__ bool pair_ld(const ulonglong2 *p, unsigned long long item, uint32_t *recno)
 	{
 		unsigned long long i, r;
-		asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(i), "=l"(r) : "l"(p) : "memory");
+		asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+			     : "=l"(i), "=l"(r) : "l"(p) : "memory");
 		*recno = (uint32_t)r;
 		return i == item;
 	}
 	static __device__ __forceinline__ void pair_st(ulonglong2 *p, unsigned long long item, uint32_t recno)
 	{
-		asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};"
+		asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
 			     ::"l"(p), "l"(item), "l"((unsigned long long)recno) : "memory");
 	}
 	__device__ __forceinline__ ulonglong2 *note_of(unsigned long long item) const
@@ -320,11 +325,25 @@ struct kma_chain_log {
 	{
 		return pair_ld(last_of(item), item, recno);
 	}
-	/* (the upper 16 bits of entry 1 alone: little endian) */
-	__device__ __forceinline__ void behind(uint32_t recno, uint32_t bits)
+	__device__ __forceinline__ unsigned long long name(uint32_t recno) const
 	{
-		unsigned short *p = reinterpret_cast<unsigned short *>(clq_slot(recno) + 1) + 3;
-		asm volatile("st.relaxed.gpu.global.u16 [%0], %1;" ::"l"(p), "h"((unsigned short)bits) : "memory");
+		return kma_detail::ld_relaxed64(&names[recno & mask]);
+	}
+	__device__ __forceinline__ void set_name(uint32_t recno, unsigned long long v)
+	{
+		kma_detail::st_relaxed64(&names[recno & mask], v);
+	}
+	/* item i's part (of len) in recording a pointer chain, before its append */
+	__device__ __forceinline__ void write(uint32_t recno, uint32_t i, uint32_t len, unsigned long long item)
+	{
+		unsigned long long *rec = clq_slot(recno);
+		rec[i] = item | (unsigned long long)len << kma_q::LOG_LEN_SHIFT;
+		for (uint32_t j = i + len; j < kma_q::LOG_CHAIN_MAX; j += len)
+			rec[j] = 0;
+		if (i == 0)
+			set_name(recno, 0);
+		if (i == len - 1)
+			last(item, recno);
 	}
 	static __device__ __forceinline__ uint32_t ld(const uint32_t *p) { return kma_detail::ld_relaxed(p); }
 	__device__ __forceinline__ uint32_t take() { return atomicAdd(next, 1u) & kma_q::LOG_RECNO_MASK; }
@@ -528,13 +547,9 @@ __device__ inline int kma_clqueue_enqueue_warp(kma_clqueue *q, kma_clqueue_item 
 	if (ok) {
 		unsigned long long link = gp.next != lane ? nip : 0ull;
 		if (logged) {
-			log->clq_slot(recno)[gp.rank] =
-				gp.rank == 0 ? ip | (unsigned long long)gp.size << kma_q::LOG_LEN_SHIFT : ip;
-			link |= gp.rank == 0 ? kma_q::clq_mark_first(recno, gp.size)
-					     : (gp.rank == 1 ? kma_q::clq_mark_second(recno) : 0ull);
+			log->write(recno, gp.rank, gp.size, ip);
+			link |= kma_q::clq_mark(recno, gp.rank, gp.size);
 		}
-		if (logged && gp.next == lane)
-			log->last(ip, recno);
 		st_relaxed64(clq_link_head::at(ip), link);
 		/* every lane's link and record entry is visible before the first
 		 * lane's exchange publishes the chain */

@@ -161,7 +161,7 @@ int kma_clarraylist_group_host(kma_heap_t kma, kma_pma_t pma, uint32_t obj_size,
 /* A log of `records` (a power of two, at most 2^24) chain records for the
  * warp forms of the queues: warp enqueues record each chain's items, warp
  * dequeues take a recorded chain at the head in one step instead of
- * walking it.  272 bytes per record; records are reused round robin and
+ * walking it.  280 bytes per record; records are reused round robin and
  * are only hints (checked against the queue before use), so any size is
  * correct and a size at least the number of chains queued at once is
  * fastest.  No counterpart in the reference. */

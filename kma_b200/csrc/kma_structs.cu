@@ -650,11 +650,11 @@ extern "C" int kma_iqueue_replay_host(uint32_t n_items, uint32_t stride_l2, cons
 
 namespace {
 /* A chain log in device memory `mem`: header line, counter line, the records,
- * the last items and the notes, all zero (an entry is 0 until a chain fills
- * it). */
+ * the last items, the notes and the names, all zero (an entry is 0 until a
+ * chain fills it). */
 size_t chain_log_bytes(uint32_t records)
 {
-	return 256 + (size_t)records * (256 + sizeof(ulonglong2)) + KMA_LOG_NOTES * sizeof(ulonglong2);
+	return 256 + (size_t)records * (256 + sizeof(ulonglong2) + 8) + KMA_LOG_NOTES * sizeof(ulonglong2);
 }
 int chain_log_setup(void *mem, uint32_t records, cudaStream_t st)
 {
@@ -666,6 +666,7 @@ int chain_log_setup(void *mem, uint32_t records, cudaStream_t st)
 	hl.mask = records - 1;
 	hl.lasts = (ulonglong2 *)(m + 256 + (size_t)records * 256);
 	hl.notes = hl.lasts + records;
+	hl.names = (unsigned long long *)(hl.notes + KMA_LOG_NOTES);
 	KMA_CUDA(cudaMemsetAsync(mem, 0, chain_log_bytes(records), st));
 	KMA_CUDA(cudaMemcpyAsync(mem, &hl, sizeof(hl), cudaMemcpyHostToDevice, st));
 	return KMA_OK;

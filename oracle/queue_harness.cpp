@@ -33,6 +33,7 @@
  *   queue_harness clq|iq THREADS CHAINS MAX_CHAIN DEQ_BATCH DELAY_PROB SEED
  *                 [PRODUCERS [RECYCLE [LOG_RECORDS [PHASED [LANES]]]]]
  *   queue_harness stuck
+ *   queue_harness reuse SEED LOG_RECORDS LIVES   (see run_reuse)
  *
  * PRODUCERS of the threads (default half) append CHAINS fresh chains of
  * 1..MAX_CHAIN items each; the rest take batches of 1..DEQ_BATCH until
@@ -114,8 +115,25 @@ struct Item {
 	u64 next;
 	Stamp st;
 };
+/* Items whose memory there is, where a run says so: any other address that is
+ * followed is counted. */
+const std::vector<char> *g_there = nullptr;
+const Item *g_first = nullptr;
+uint64_t g_strays = 0;
 struct LinkAtItem {
-	static u64 *at(u64 p) { return reinterpret_cast<u64 *>(p); }
+	static u64 *at(u64 p)
+	{
+		static u64 nowhere;
+		if (g_there) {
+			const u64 i = (p - (u64)g_first) / sizeof(Item);
+			if (p < (u64)g_first || i >= g_there->size() || !(*g_there)[i]) {
+				g_strays++;
+				nowhere = kma_q::POISON;
+				return &nowhere;
+			}
+		}
+		return reinterpret_cast<u64 *>(p);
+	}
 };
 
 /* host waits: long enough for any sleeping appender, short enough that a
@@ -146,22 +164,60 @@ struct HostLog {
 		note_item[i].store(item, std::memory_order_relaxed);
 		note_rec[i].store(recno, std::memory_order_relaxed);
 	}
-	/* the chains' last items, in the same way */
-	std::atomic<u64> last_item[NOTES] = {}, last_rec[NOTES] = {};
+	/* the chains' last items, in the same way, a pair in one piece */
+	struct Pair {
+		std::atomic_flag busy = ATOMIC_FLAG_INIT;
+		u64 item = 0;
+		uint32_t rec = 0;
+		template <class F>
+		void locked(F f)
+		{
+			while (busy.test_and_set(std::memory_order_acquire))
+				;
+			f();
+			busy.clear(std::memory_order_release);
+		}
+	};
+	Pair lasts[NOTES];
 	void last(u64 item, uint32_t recno)
 	{
-		last_item[note_of(item)].store(item, std::memory_order_relaxed);
-		last_rec[note_of(item)].store(recno, std::memory_order_relaxed);
+		Pair &p = lasts[note_of(item)];
+		p.locked([&] {
+			p.item = item;
+			p.rec = recno;
+		});
 	}
 	bool lookup(u64 item, uint32_t *recno)
 	{
-		*recno = (uint32_t)last_rec[note_of(item)].load(std::memory_order_relaxed);
-		return last_item[note_of(item)].load(std::memory_order_relaxed) == item;
+		Pair &p = lasts[note_of(item)];
+		bool is = false;
+		p.locked([&] {
+			is = p.item == item;
+			*recno = p.rec;
+		});
+		return is;
 	}
-	void behind(uint32_t recno, uint32_t bits)
+	std::vector<u64> names;
+	u64 name(uint32_t recno) const { return __atomic_load_n(&names[recno & mask], __ATOMIC_RELAXED); }
+	void set_name(uint32_t recno, u64 v) { __atomic_store_n(&names[recno & mask], v, __ATOMIC_RELAXED); }
+	/* record chain recno, before it is appended: entry j of len */
+	void write(uint32_t recno, uint32_t j, uint32_t len, u64 item)
 	{
-		uint16_t *p = reinterpret_cast<uint16_t *>(&clq[(size_t)(recno & mask) * 32 + 1]) + 3;
-		__atomic_store_n(p, (uint16_t)bits, __ATOMIC_RELAXED);
+		u64 *rec = &clq[(size_t)(recno & mask) * 32];
+		__atomic_store_n(rec + j, item | (u64)len << kma_q::LOG_LEN_SHIFT, __ATOMIC_RELAXED);
+		for (uint32_t i = j + len; i < 32; i += len)
+			__atomic_store_n(rec + i, 0ull, __ATOMIC_RELAXED);
+		if (j == 0)
+			set_name(recno, 0);
+		if (j == len - 1)
+			last(item, recno);
+	}
+	void resize(uint32_t records)
+	{
+		mask = records - 1;
+		clq.assign((size_t)records * 32, 0);
+		iq.assign((size_t)records * 32, 0);
+		names.assign(records, 0);
 	}
 	const u64 *clq_record(uint32_t recno) const { return &clq[(size_t)(recno & mask) * 32]; }
 	const uint32_t *iq_record(uint32_t recno) const { return &iq[(size_t)(recno & mask) * 32]; }
@@ -301,16 +357,12 @@ void run_clq(int threads, int chains, int maxc, int batch, double recycle, uint6
 			__atomic_fetch_add(&bk.appends[(size_t)(v[j] - items.data())], 1, __ATOMIC_RELAXED);
 			u64 link = j + 1 < len ? (u64)v[j + 1] : 0ull;
 			if (logged) {
-				__atomic_store_n(&g_log.clq[(size_t)(recno & g_log.mask) * 32 + j],
-						 (u64)v[j] | (j == 0 ? (u64)len << kma_q::LOG_LEN_SHIFT : 0ull), __ATOMIC_RELAXED);
-				link |= j == 0 ? kma_q::clq_mark_first(recno, (uint32_t)len)
-					       : (j == 1 ? kma_q::clq_mark_second(recno) : 0ull);
+				g_log.write(recno, (uint32_t)j, (uint32_t)len, (u64)v[j]);
+				link |= kma_q::clq_mark(recno, (uint32_t)j, (uint32_t)len);
 			}
 			__atomic_store_n(&v[j]->next, link, __ATOMIC_RELAXED);
 		}
 		u64 prev = 0;
-		if (logged)
-			g_log.last((u64)v[len - 1], recno);
 		if (!kma_q::clq_append<HostOps, LinkAtItem>(&q[0], &q[1], (u64)v[0], (u64)v[len - 1], LIMIT,
 							     logged ? kma_q::clq_mark_into(recno) : 0ull, &prev))
 			bk.tmo++;
@@ -591,8 +643,86 @@ int run_stuck()
 	return ok ? 0 : 1;
 }
 
+/* One log over many lives of one item array.  In each life a part of the
+ * items is there (the memory of the others is gone), in an order of its own;
+ * a queue takes them in chains, some of them logged, and batches of all forms
+ * empty it.  The items must come in the order appended, and whatever the log
+ * kept from earlier lives, no item that is not there may be followed. */
+int run_reuse(uint64_t seed, uint32_t records, int lives)
+{
+	t_rng = seed * 0x9E3779B97F4A7C15ull + 0x5000u;
+	g_log.resize(records);
+	const size_t n = 400;
+	std::vector<Item> items(n);
+	std::vector<char> there(n);
+	std::vector<Item *> order;
+	uint64_t order_bad = 0, batches = 0;
+	g_first = items.data();
+	for (int life = 0; life < lives; life++) {
+		g_there = nullptr;
+		const double part = 0.1 + 0.9 * unit();
+		order.clear();
+		for (size_t i = 0; i < n; i++)
+			if ((there[i] = unit() < part))
+				order.push_back(&items[i]);
+		/* mostly in place, so that chains of two lives begin alike */
+		for (size_t i = 1; i < order.size(); i++)
+			if (unit() < 0.1)
+				std::swap(order[i], order[rnd() % (i + 1)]);
+		g_there = &there;
+		u64 q[2] = {0, 0};
+		size_t put = 0, got = 0;
+		const double log_some = unit() < 0.5 ? 1.0 : unit();
+		std::vector<u64> out(300);
+		while (got < order.size()) {
+			while (put < order.size() && (put == got || unit() < 0.7)) {
+				const uint32_t len = (uint32_t)std::min<size_t>(1 + rnd() % 32, order.size() - put);
+				const bool logged = len >= 3 && unit() < log_some;
+				const uint32_t recno = logged ? g_log.take() : 0;
+				for (uint32_t j = 0; j < len; j++) {
+					Item *it = order[put + j];
+					if (logged)
+						g_log.write(recno, j, len, (u64)it);
+					it->next = (j + 1 < len ? (u64)order[put + j + 1] : 0ull) |
+						   (logged ? kma_q::clq_mark(recno, j, len) : 0ull);
+				}
+				u64 prev = 0;
+				if (kma_q::clq_append<HostOps, LinkAtItem>(&q[0], &q[1], (u64)order[put], (u64)order[put + len - 1],
+									    LIMIT, logged ? kma_q::clq_mark_into(recno) : 0ull,
+									    &prev) &&
+				    logged)
+					kma_q::clq_log_behind(&g_log, prev, recno);
+				put += len;
+			}
+			const uint32_t k = 1 + (uint32_t)(rnd() % (unit() < 0.5 ? 300 : 20));
+			bool to = false;
+			HostOut ho = {out.data()};
+			const uint32_t r = unit() < 0.8 ? kma_q::clq_dequeue_v<HostOps, LinkAtItem, HostLanes>(
+								  &q[0], &q[1], ho, k, 1000, &to, log_ptr())
+							 : kma_q::clq_dequeue_n<HostOps, LinkAtItem>(
+								   &q[0], &q[1], out.data(), k, 1000, &to,
+								   unit() < 0.5 ? log_ptr() : (const HostLog *)nullptr);
+			batches++;
+			if (!r || to || got + r > put) {
+				order_bad++;
+				break;
+			}
+			for (uint32_t i = 0; i < r; i++)
+				order_bad += out[i] != (u64)order[got + i];
+			got += r;
+		}
+	}
+	g_there = nullptr;
+	printf("{\"batches\": %llu, \"log_chains\": %llu, \"order_faults\": %llu, \"strays\": %llu}\n",
+	       (unsigned long long)batches, (unsigned long long)g_log.chains.load(), (unsigned long long)order_bad,
+	       (unsigned long long)g_strays);
+	return order_bad || g_strays;
+}
+
 int main(int argc, char **argv)
 {
+	if (argc == 5 && strcmp(argv[1], "reuse") == 0)
+		return run_reuse(strtoull(argv[2], NULL, 0), (uint32_t)strtoul(argv[3], NULL, 0), atoi(argv[4]));
 	if (argc == 2 && strcmp(argv[1], "stuck") == 0)
 		return run_stuck();
 	if (argc < 8 || argc > 13) {
@@ -622,9 +752,7 @@ int main(int argc, char **argv)
 	if (log_records) {
 		if (log_records & (log_records - 1))
 			return 2; /* a power of two */
-		g_log.mask = log_records - 1;
-		g_log.clq.assign((size_t)log_records * 32, 0);
-		g_log.iq.assign((size_t)log_records * 32, 0);
+		g_log.resize(log_records);
 	}
 	if (threads < 1 || chains < 1 || maxc < 1 || batch < 1)
 		return 2;

@@ -230,3 +230,41 @@ def test_named_records_conserve_and_keep_order(harness, cfg, lanes):
     assert rc == 0 and st.get("ok"), st
     assert st["taken"] + st["left"] >= st["appended"] > 0
     assert st["conservation_faults"] == 0 and st["order_faults"] == 0 and st["timeouts"] == 0
+
+
+# one log over many lives of one item array: a log that keeps hardly anything,
+# some, all of a life, and more chains than the low half of a record number counts
+REUSE = ["1 1 400", "2 8 400", "3 64 400", "4 1024 400", "5 65536 3000"]
+
+
+@pytest.mark.parametrize("args", REUSE)
+def test_a_log_outlives_the_items_it_has_recorded(harness, args):
+    """Notes and records of items that have left their queues, and whose
+    memory is gone, are never followed, even where the next queue holds some
+    of the same items; its chains still come from their records."""
+    r = subprocess.run([harness, "reuse", *args.split()], capture_output=True, text=True, timeout=120)
+    st = json.loads(r.stdout)
+    assert r.returncode == 0 and st["strays"] == 0 and st["order_faults"] == 0, st
+    if args.split()[1] != "1":
+        assert st["log_chains"] > 8 * int(args.split()[2])
+
+
+REUSE_MUTANTS = {
+    # believe a note because the record has the head in it
+    "note_unproven": ("noted = second && clq_number(nx, l1, &no) && no == recno;", "noted = second != 0;"),
+    # believe a name whoever it was given to
+    "name_of_any_record": ("return (name >> 24) == ((LOG_NAMED >> 24) | recno);", "return (name & LOG_NAMED) != 0;"),
+}
+
+
+@pytest.mark.parametrize("name", sorted(REUSE_MUTANTS))
+def test_reuse_run_detects_planted_mistakes(harness, tmp_path, name):
+    old, new = REUSE_MUTANTS[name]
+    src = open(ALGO).read()
+    assert src.count(old) == 1
+    (tmp_path / "kma_queue_algo.cuh").write_text(src.replace(old, new))
+    binary = str(tmp_path / "h")
+    subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-pthread", f"-I{tmp_path}", "-o", binary,
+                    os.path.join(ORACLE, "queue_harness.cpp")], check=True)
+    assert any(subprocess.run([binary, "reuse", *args.split()], capture_output=True, timeout=120).returncode
+               for args in REUSE)
