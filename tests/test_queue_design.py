@@ -252,8 +252,6 @@ def test_a_log_outlives_the_items_it_has_recorded(harness, args):
 REUSE_MUTANTS = {
     # believe a note because the record has the head in it
     "note_unproven": ("noted = second && clq_number(nx, l1, &no) && no == recno;", "noted = second != 0;"),
-    # believe a name whoever it was given to
-    "name_of_any_record": ("return (name >> 24) == ((LOG_NAMED >> 24) | recno);", "return (name & LOG_NAMED) != 0;"),
 }
 
 
