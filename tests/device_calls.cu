@@ -24,7 +24,57 @@ __global__ void k_replay_hint(kma_heap *h, const long long *ops, long long n, lo
 		}
 	}
 }
+
+/* One warp: lane 0 puts n items on each of nq queues, the head of each then
+ * held for good if `stuck`; every lane takes one from queue lane % nq, with an
+ * error word of its own and a limit that `step` makes differ.  out: the item's
+ * number in its queue, -1 for none. */
+__global__ void k_lanes_dequeue(kma_clqueue *q, unsigned long long *items, int nq, int n, int stuck, uint32_t step,
+		int *out, uint32_t *err)
+{
+	const int lane = threadIdx.x;
+	if (lane == 0)
+		for (int k = 0; k < nq; k++) {
+			kma_clqueue_init(&q[k]);
+			for (int i = 0; i < n; i++)
+				kma_clqueue_enqueue(&q[k], reinterpret_cast<kma_clqueue_item *>(&items[2 * (k * n + i)]));
+			if (stuck)
+				items[2 * k * n] = kma_q::POISON;
+		}
+	__syncwarp();
+	unsigned long long *it = reinterpret_cast<unsigned long long *>(
+		kma_clqueue_dequeue(&q[lane % nq], &err[lane], 1024u + step * (lane % 3)));
+	out[lane] = it ? (int)((it - items) / 2) - (lane % nq) * n : -1;
+}
+
+/* a user's kernels of one per-thread dequeue each, without launch bounds */
+__global__ void k_user_clqueue(kma_clqueue *q, unsigned long long *sum)
+{
+	kma_clqueue_item *it = kma_clqueue_dequeue(q + threadIdx.x % 7);
+	if (it)
+		atomicAdd(sum, reinterpret_cast<unsigned long long *>(it)[1]);
+}
+__global__ void k_user_iqueue(kma_iqueue *q, unsigned long long *sum)
+{
+	void *it = kma_iqueue_dequeue(q);
+	if (it)
+		atomicAdd(sum, reinterpret_cast<unsigned long long *>(it)[1]);
+}
 } /* namespace */
+
+extern "C" int t_lanes_dequeue(void *q, unsigned long long *items, int nq, int n, int stuck, uint32_t step, int *out,
+		uint32_t *err)
+{
+	k_lanes_dequeue<<<1, 32>>>((kma_clqueue *)q, items, nq, n, stuck, step, out, err);
+	const cudaError_t e = cudaGetLastError();
+	return e != cudaSuccess ? e : cudaDeviceSynchronize();
+}
+
+extern "C" void t_user_kernels(kma_clqueue *q, kma_iqueue *iq, unsigned long long *sum)
+{
+	k_user_clqueue<<<1, 1024>>>(q, sum);
+	k_user_iqueue<<<1, 1024>>>(iq, sum);
+}
 
 /* one lane replays ops through the warp calls, with hints */
 extern "C" int t_replay_hint(kma_heap *h, const long long *ops, long long n, long long *out)

@@ -2,6 +2,8 @@
 library's entry points do not reach (tests/device_calls.cu, built here)."""
 import ctypes
 import os
+import re
+import shutil
 import subprocess
 
 import numpy as np
@@ -40,3 +42,56 @@ def test_one_lane_with_hints_replays_as_the_reference(calls, seed):
         assert rc == 0
         np.testing.assert_array_equal(out.cpu().numpy(), want)
         assert h.error_flags() == 0
+
+
+def test_per_thread_dequeues_fit_a_block_of_1024_threads(tmp_path):
+    """They are header code in the user's kernel: with more than 64 registers
+    a thread, or arrays in local memory, a kernel of one such call would not
+    launch with 1024 threads, or would pay for what its lanes never use."""
+    if shutil.which(kbuild.nvcc()) is None:
+        pytest.skip("no nvcc")
+    r = subprocess.run([kbuild.nvcc(), *kbuild.ARCH, "-O3", "-std=c++17", "-Xptxas", "-v", "-I", kbuild.INCLUDE, "-c",
+                        "-o", str(tmp_path / "o.o"), os.path.join(HERE, "device_calls.cu")],
+                       check=True, capture_output=True, text=True)
+    found = re.findall(r"Compiling entry function '\w*(k_user_\w+?queue)\w*'.*?(\d+) bytes stack frame.*?Used (\d+) registers",
+                       r.stderr, re.S)
+    assert {f[0] for f in found} == {"k_user_clqueue", "k_user_iqueue"}
+    for name, stack, regs in found:
+        assert int(stack) == 0 and int(regs) <= 64, (name, stack, regs)
+
+
+def _lanes(calls, nq, n, stuck, step):
+    import torch
+    q = torch.zeros(2 * nq, dtype=torch.int64, device="cuda")
+    items = torch.zeros(2 * nq * n, dtype=torch.int64, device="cuda")
+    out = torch.full((32,), -7, dtype=torch.int32, device="cuda")
+    err = torch.zeros(32, dtype=torch.int32, device="cuda")
+    rc = calls.t_lanes_dequeue(ctypes.c_void_p(q.data_ptr()), ctypes.c_void_p(items.data_ptr()), nq, n, stuck, step,
+                               ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(err.data_ptr()))
+    assert rc == 0
+    return out.cpu().numpy(), err.cpu().numpy()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("step", [0, 5])
+@pytest.mark.parametrize("nq,n", [(1, 1), (1, 20), (1, 32), (1, 40), (2, 9), (2, 16), (3, 20)])
+def test_lanes_of_a_warp_dequeue_each_its_own(calls, nq, n, step):
+    """On one queue or several, with one limit or several: the first items
+    come out, each to one lane, and nobody's wait is reported as expired."""
+    out, err = _lanes(calls, nq, n, 0, step)
+    assert not err.any()
+    for k in range(nq):
+        mine = out[k::nq]
+        assert sorted(mine[mine >= 0]) == list(range(min(n, len(mine))))
+        assert (mine >= -1).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("step", [0, 5])
+@pytest.mark.parametrize("nq", [1, 2])
+def test_every_lane_learns_of_its_expired_wait(calls, nq, step):
+    """A head that is never given back: each lane gets NULL, and the timeout
+    in the error word that it passed."""
+    from kma_b200 import KMA_FLAG_TIMEOUT
+    out, err = _lanes(calls, nq, 3, 1, step)
+    assert (out == -1).all() and ((err & KMA_FLAG_TIMEOUT) != 0).all()

@@ -266,3 +266,15 @@ def test_reuse_run_detects_planted_mistakes(harness, tmp_path, name):
                     os.path.join(ORACLE, "queue_harness.cpp")], check=True)
     assert any(subprocess.run([binary, "reuse", *args.split()], capture_output=True, timeout=120).returncode
                for args in REUSE)
+
+
+# the text of lanes that call a per-thread dequeue together, always (3) or mixed with the others (4)
+@pytest.mark.parametrize("lanes", [3, 4])
+@pytest.mark.parametrize("kind", ["clq", "iq"])
+@pytest.mark.parametrize("cfg", ["8 20000 1 1 0.01 1 1 0.5 64 0", "8 5000 32 32 0.02 7 4 0.5 1024 0",
+                                 "3 20000 8 8 0.01 6 1 0.5 0 0", "8 5000 -32 -32 0.02 15 4 0.5 0 1"])
+def test_text_of_lanes_conserves_and_keeps_order(harness, cfg, kind, lanes):
+    rc, st = run(harness, kind, f"{cfg} {lanes}")
+    assert rc == 0 and st.get("ok"), st
+    assert st["taken"] + st["left"] >= st["appended"] > 0
+    assert st["conservation_faults"] == 0 and st["order_faults"] == 0 and st["timeouts"] == 0
