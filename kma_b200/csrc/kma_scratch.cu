@@ -19,22 +19,57 @@ std::mutex g_mu;
 std::vector<kept> g_kept; /* oldest first */
 size_t g_bytes = 0;
 
-/* A number of the current context that no later one has (0: unknown, and
- * then nothing is kept). */
-unsigned long long context_id()
-{
-	typedef CUresult (*get_id_t)(CUcontext, unsigned long long *);
-	static get_id_t get_id = []() -> get_id_t {
-		void *f = NULL;
+/* The driver's context calls. */
+struct driver {
+	CUresult (*get_id)(CUcontext, unsigned long long *);
+	CUresult (*get)(CUcontext *);
+	CUresult (*set)(CUcontext);
+	CUresult (*retain)(CUcontext *, CUdevice);
+	CUresult (*release)(CUdevice);
+	CUresult (*state)(CUdevice, unsigned int *, int *);
+	bool ok;
+
+	driver() : ok(true)
+	{
+		find("cuCtxGetId", (void **)&get_id);
+		find("cuCtxGetCurrent", (void **)&get);
+		find("cuCtxSetCurrent", (void **)&set);
+		find("cuDevicePrimaryCtxRetain", (void **)&retain);
+		find("cuDevicePrimaryCtxRelease", (void **)&release);
+		find("cuDevicePrimaryCtxGetState", (void **)&state);
+	}
+	void find(const char *name, void **f)
+	{
 		cudaDriverEntryPointQueryResult r;
-		if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &r) != cudaSuccess) {
+		*f = NULL;
+		if (cudaGetDriverEntryPoint(name, f, cudaEnableDefault, &r) != cudaSuccess)
 			cudaGetLastError();
-			return NULL;
-		}
-		return r == cudaDriverEntryPointSuccess ? (get_id_t)f : NULL;
-	}();
+		else if (r != cudaDriverEntryPointSuccess)
+			*f = NULL;
+		ok = ok && *f;
+	}
+};
+const driver &drv()
+{
+	static const driver d;
+	return d;
+}
+
+/* A number of device dev's primary context, which no later one has, if that
+ * is the current context; else 0, and then nothing is kept: another context
+ * may end at any time, and its memory with it, without a sign. */
+unsigned long long context_id(int dev)
+{
+	const driver &d = drv();
+	CUcontext now = NULL, primary = NULL;
 	unsigned long long id = 0;
-	return get_id && get_id(NULL, &id) == CUDA_SUCCESS ? id : 0;
+	unsigned int flags;
+	int active = 0;
+	if (!d.ok || d.get(&now) != CUDA_SUCCESS || d.state(dev, &flags, &active) != CUDA_SUCCESS || !active ||
+	    d.retain(&primary, dev) != CUDA_SUCCESS)
+		return 0;
+	d.release(dev);
+	return now == primary && d.get_id(now, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 void drop(size_t i)
@@ -55,13 +90,19 @@ void kma_scratch_trim(void)
 	}
 	if (all.empty())
 		return;
-	int prev = 0;
-	if (cudaGetDevice(&prev) != cudaSuccess)
+	const driver &d = drv();
+	CUcontext now = NULL;
+	if (d.get(&now) != CUDA_SUCCESS)
 		return;
-	for (const kept &k : all)
-		if (cudaSetDevice(k.device) == cudaSuccess && context_id() == k.ctx)
+	for (const kept &k : all) {
+		/* (the memory of a context that was reset went with it) */
+		unsigned int flags;
+		int active = 0;
+		if (d.state(k.device, &flags, &active) == CUDA_SUCCESS && active && cudaSetDevice(k.device) == cudaSuccess &&
+		    context_id(k.device) == k.ctx)
 			cudaFree(k.p);
-	cudaSetDevice(prev);
+	}
+	d.set(now);
 	cudaGetLastError();
 }
 
@@ -87,7 +128,7 @@ void *kma_dev_bufs::take(size_t bytes)
 		cudaGetLastError();
 		return NULL;
 	}
-	const unsigned long long ctx = context_id();
+	const unsigned long long ctx = context_id(dev);
 	{
 		std::lock_guard<std::mutex> lk(g_mu);
 		/* the smallest that fits */
@@ -117,7 +158,7 @@ kma_dev_bufs::~kma_dev_bufs()
 	int dev = 0;
 	/* nothing may still use them; after an error they are not kept */
 	const bool idle = cudaDeviceSynchronize() == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess;
-	const unsigned long long ctx = idle ? context_id() : 0;
+	const unsigned long long ctx = idle ? context_id(dev) : 0;
 	std::vector<void *> gone;
 	{
 		std::lock_guard<std::mutex> lk(g_mu);
@@ -126,8 +167,9 @@ kma_dev_bufs::~kma_dev_bufs()
 				gone.push_back(b.p);
 				continue;
 			}
-			/* make room: the oldest of this context leave, those of a
-			 * context that is gone are forgotten with their memory */
+			/* make room: the oldest of this context leave; others of the
+			 * device are of primary contexts that were reset, and are
+			 * forgotten as their memory is gone */
 			for (size_t i = 0; i < g_kept.size() && g_bytes + b.bytes > KMA_SCRATCH_KEEP;) {
 				if (g_kept[i].device == dev && g_kept[i].ctx != ctx) {
 					drop(i);

@@ -16,8 +16,9 @@
  *   - a buffer belongs to one call at a time (the list is behind a mutex) and
  *     returns to the list only when the device is idle, as cudaFree would
  *     have waited, so no stream of any caller can still use it;
- *   - a list entry is used only in the context that it came from (the
- *     device's primary context may be reset in between).
+ *   - only buffers of a device's primary context are kept, and used only in
+ *     that one (it may be reset in between); calls that a program makes in a
+ *     context of its own allocate and free.
  */
 #ifndef KMA_SCRATCH_H
 #define KMA_SCRATCH_H
