@@ -156,8 +156,10 @@ kma_dev_bufs::~kma_dev_bufs()
 	if (v_.empty())
 		return;
 	int dev = 0;
-	/* nothing may still use them; after an error they are not kept */
-	const bool idle = cudaDeviceSynchronize() == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess;
+	/* nothing may still use them; after an error they are not kept.  (The
+	 * calls work on the default stream: a wait for the whole device would
+	 * break any capture that another thread has under way on it.) */
+	const bool idle = cudaStreamSynchronize(NULL) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess;
 	const unsigned long long ctx = idle ? context_id(dev) : 0;
 	std::vector<void *> gone;
 	{

@@ -14,8 +14,8 @@
  *     allocation of the library fails (kma_device_malloc empties the list and
  *     tries again);
  *   - a buffer belongs to one call at a time (the list is behind a mutex) and
- *     returns to the list only when the device is idle, as cudaFree would
- *     have waited, so no stream of any caller can still use it;
+ *     returns to the list only when the default stream, on which all of these
+ *     calls work, is idle, so nothing can still use it;
  *   - only buffers of a device's primary context are kept, and used only in
  *     that one (it may be reset in between); calls that a program makes in a
  *     context of its own allocate and free.
@@ -35,7 +35,7 @@ cudaError_t kma_device_malloc(void **p, size_t bytes);
 void kma_scratch_trim(void);
 
 /* The buffers of one host call on the current device, all returned when it
- * goes out of scope. */
+ * goes out of scope.  For use on the default stream only. */
 class kma_dev_bufs {
 public:
 	kma_dev_bufs() {}

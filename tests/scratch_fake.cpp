@@ -210,6 +210,15 @@ static void two_devices()
 	kma_scratch_trim();
 	CHECK(current == primary[0] && live(primary[0]) == 0 && live(primary[1]) == 0);
 }
+/* another thread captures a graph on the device meanwhile */
+static void capture()
+{
+	cudaSetDevice(0);
+	capturing = true;
+	void *p = call(7000, 100);
+	CHECK(call(7000, 100) == p);
+	CHECK(!capture_broken);
+}
 static void bounded()
 {
 	cudaSetDevice(0);
@@ -230,7 +239,7 @@ int main(int argc, char **argv)
 	static const struct {
 		const char *name;
 		void (*run)();
-	} all[] = {{"contexts", contexts}, {"reset", reset}, {"two_devices", two_devices}, {"bounded", bounded}};
+	} all[] = {{"contexts", contexts}, {"reset", reset}, {"two_devices", two_devices}, {"capture", capture}, {"bounded", bounded}};
 	for (auto &s : all)
 		if (argc == 2 && !strcmp(argv[1], s.name)) {
 			s.run();
