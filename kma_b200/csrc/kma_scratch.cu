@@ -16,8 +16,10 @@ struct kept {
 };
 
 std::mutex g_mu;
-std::vector<kept> g_kept; /* oldest first */
-size_t g_bytes = 0;
+/* oldest first.  (Arrays: these calls are made from C, which no exception of a
+ * container may reach.) */
+kept g_kept[KMA_SCRATCH_LIST];
+size_t g_n = 0, g_bytes = 0;
 
 /* The driver's context calls. */
 struct driver {
@@ -75,26 +77,32 @@ unsigned long long context_id(int dev)
 void drop(size_t i)
 {
 	g_bytes -= g_kept[i].bytes;
-	g_kept.erase(g_kept.begin() + (ptrdiff_t)i);
+	for (g_n--; i < g_n; i++)
+		g_kept[i] = g_kept[i + 1];
 }
+bool full(size_t bytes) { return g_n == KMA_SCRATCH_LIST || g_bytes + bytes > KMA_SCRATCH_KEEP; }
 
 } /* namespace */
 
 void kma_scratch_trim(void)
 {
-	std::vector<kept> all;
+	kept all[KMA_SCRATCH_LIST];
+	size_t n;
 	{
 		std::lock_guard<std::mutex> lk(g_mu);
-		all.swap(g_kept);
-		g_bytes = 0;
+		for (size_t i = 0; i < g_n; i++)
+			all[i] = g_kept[i];
+		n = g_n;
+		g_n = g_bytes = 0;
 	}
-	if (all.empty())
+	if (!n)
 		return;
 	const driver &d = drv();
 	CUcontext now = NULL;
 	if (d.get(&now) != CUDA_SUCCESS)
 		return;
-	for (const kept &k : all) {
+	for (size_t i = 0; i < n; i++) {
+		const kept &k = all[i];
 		/* (the memory of a context that was reset went with it) */
 		unsigned int flags;
 		int active = 0;
@@ -120,7 +128,7 @@ cudaError_t kma_device_malloc(void **p, size_t bytes)
 void *kma_dev_bufs::take(size_t bytes)
 {
 	int dev = 0;
-	if (cudaGetDevice(&dev) != cudaSuccess)
+	if (n_ == KMA_SCRATCH_PER_CALL || cudaGetDevice(&dev) != cudaSuccess)
 		return NULL;
 	/* also brings the device's context up, where it is not */
 	void *p = NULL;
@@ -132,12 +140,12 @@ void *kma_dev_bufs::take(size_t bytes)
 	{
 		std::lock_guard<std::mutex> lk(g_mu);
 		/* the smallest that fits */
-		size_t best = g_kept.size();
-		for (size_t i = 0; i < g_kept.size(); i++)
+		size_t best = g_n;
+		for (size_t i = 0; i < g_n; i++)
 			if (ctx && g_kept[i].device == dev && g_kept[i].ctx == ctx && g_kept[i].bytes >= bytes &&
-			    (best == g_kept.size() || g_kept[i].bytes < g_kept[best].bytes))
+			    (best == g_n || g_kept[i].bytes < g_kept[best].bytes))
 				best = i;
-		if (best < g_kept.size()) {
+		if (best < g_n) {
 			p = g_kept[best].p;
 			bytes = g_kept[best].bytes;
 			drop(best);
@@ -147,13 +155,13 @@ void *kma_dev_bufs::take(size_t bytes)
 		cudaGetLastError();
 		return NULL;
 	}
-	v_.push_back({p, bytes});
+	v_[n_++] = {p, bytes};
 	return p;
 }
 
 kma_dev_bufs::~kma_dev_bufs()
 {
-	if (v_.empty())
+	if (!n_)
 		return;
 	int dev = 0;
 	/* nothing may still use them; after an error they are not kept.  (The
@@ -161,35 +169,35 @@ kma_dev_bufs::~kma_dev_bufs()
 	 * break any capture that another thread has under way on it.) */
 	const bool idle = cudaStreamSynchronize(NULL) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess;
 	const unsigned long long ctx = idle ? context_id(dev) : 0;
-	std::vector<void *> gone;
-	{
-		std::lock_guard<std::mutex> lk(g_mu);
-		for (const buf &b : v_) {
-			if (!ctx || b.bytes > KMA_SCRATCH_KEEP) {
-				gone.push_back(b.p);
-				continue;
-			}
+	for (unsigned j = 0; j < n_; j++) {
+		const buf &b = v_[j];
+		void *gone[KMA_SCRATCH_LIST + 1];
+		size_t ngone = 0;
+		if (!ctx || b.bytes > KMA_SCRATCH_KEEP) {
+			gone[ngone++] = b.p;
+		} else {
+			std::lock_guard<std::mutex> lk(g_mu);
 			/* make room: the oldest of this context leave; others of the
 			 * device are of primary contexts that were reset, and are
 			 * forgotten as their memory is gone */
-			for (size_t i = 0; i < g_kept.size() && g_bytes + b.bytes > KMA_SCRATCH_KEEP;) {
+			for (size_t i = 0; i < g_n && full(b.bytes);) {
 				if (g_kept[i].device == dev && g_kept[i].ctx != ctx) {
 					drop(i);
 				} else if (g_kept[i].device == dev) {
-					gone.push_back(g_kept[i].p);
+					gone[ngone++] = g_kept[i].p;
 					drop(i);
 				} else {
 					i++;
 				}
 			}
-			if (g_bytes + b.bytes > KMA_SCRATCH_KEEP) {
-				gone.push_back(b.p);
-				continue;
+			if (full(b.bytes)) {
+				gone[ngone++] = b.p;
+			} else {
+				g_kept[g_n++] = {b.p, b.bytes, dev, ctx};
+				g_bytes += b.bytes;
 			}
-			g_kept.push_back({b.p, b.bytes, dev, ctx});
-			g_bytes += b.bytes;
 		}
+		for (size_t i = 0; i < ngone; i++)
+			cudaFree(gone[i]);
 	}
-	for (void *p : gone)
-		cudaFree(p);
 }

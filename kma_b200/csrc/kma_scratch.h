@@ -8,8 +8,9 @@
  * 28 ms of a 2^21-operation tree run.  dev_bufs takes its buffers from a list
  * of ones that earlier calls returned.
  *
- *   - bounded: at most KMA_SCRATCH_KEEP bytes per process stay on the list,
- *     the oldest leave first; a larger buffer is never kept;
+ *   - bounded: at most KMA_SCRATCH_KEEP bytes per process, in at most
+ *     KMA_SCRATCH_LIST buffers, stay on the list, the oldest leave first; a
+ *     larger buffer is never kept;
  *   - given back: when a heap or a PMA heap is destroyed, and whenever an
  *     allocation of the library fails (kma_device_malloc empties the list and
  *     tries again);
@@ -25,9 +26,10 @@
 
 #include <cuda_runtime.h>
 #include <stddef.h>
-#include <vector>
 
 #define KMA_SCRATCH_KEEP ((size_t)1 << 30)
+#define KMA_SCRATCH_LIST 64     /* buffers on the list, at most */
+#define KMA_SCRATCH_PER_CALL 8  /* buffers of one call, at most */
 
 /* cudaMalloc on the current device; on failure once more with an empty list. */
 cudaError_t kma_device_malloc(void **p, size_t bytes);
@@ -42,7 +44,7 @@ public:
 	~kma_dev_bufs();
 	kma_dev_bufs(const kma_dev_bufs &) = delete;
 	kma_dev_bufs &operator=(const kma_dev_bufs &) = delete;
-	/* NULL when out of memory; contents undefined */
+	/* NULL when out of memory, or past KMA_SCRATCH_PER_CALL; contents undefined */
 	template <typename T>
 	T *alloc(size_t bytes)
 	{
@@ -55,7 +57,8 @@ private:
 		size_t bytes;
 	};
 	void *take(size_t bytes);
-	std::vector<buf> v_;
+	buf v_[KMA_SCRATCH_PER_CALL];
+	unsigned n_ = 0;
 };
 
 #endif

@@ -219,6 +219,27 @@ static void capture()
 	CHECK(call(7000, 100) == p);
 	CHECK(!capture_broken);
 }
+/* the host is out of memory: no exception leaves a call, nothing is lost */
+static void no_host_memory()
+{
+	cudaSetDevice(0);
+	for (int n = 0; n < 12; n++)
+		for (int before = 0; before < 2; before++) {
+			if (before)
+				call(1 << 20, 100);
+			{
+				kma_dev_bufs bufs;
+				fail_new = n;
+				char *p = bufs.alloc<char>(1 << 20);
+				char *q = p ? bufs.alloc<char>((1 << 20) + n) : nullptr;
+				CHECK(!p || live(primary[0]) >= 1);
+				(void)q;
+			}
+			fail_new = -1;
+			kma_scratch_trim();
+			CHECK(live(primary[0]) == 0);
+		}
+}
 static void bounded()
 {
 	cudaSetDevice(0);
@@ -239,7 +260,8 @@ int main(int argc, char **argv)
 	static const struct {
 		const char *name;
 		void (*run)();
-	} all[] = {{"contexts", contexts}, {"reset", reset}, {"two_devices", two_devices}, {"capture", capture}, {"bounded", bounded}};
+	} all[] = {{"contexts", contexts}, {"reset", reset}, {"two_devices", two_devices}, {"capture", capture},
+		 {"no_host_memory", no_host_memory}, {"bounded", bounded}};
 	for (auto &s : all)
 		if (argc == 2 && !strcmp(argv[1], s.name)) {
 			s.run();

@@ -9,7 +9,7 @@ import pytest
 from kma_b200 import build as kbuild
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SCENARIOS = ["contexts", "reset", "two_devices", "capture", "bounded"]
+SCENARIOS = ["contexts", "reset", "two_devices", "capture", "no_host_memory", "bounded"]
 
 
 @pytest.fixture(scope="module")
