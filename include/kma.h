@@ -97,6 +97,12 @@ int kma_create_ex(const kma_config *cfg, void *stream, kma_heap_t *out);
 /* Frees the heap's device memory (the reference's clReleaseMemObject,
  * test/tb_kma.c:316; the reference has no kma_destroy). */
 int kma_destroy(kma_heap_t h);
+/* Gives device memory that the library keeps between host calls (at most 1 GiB
+ * of scratch of the replays, the structure runs and the graph build) back to
+ * CUDA, on all devices.  Destroying a heap does so too, and the library itself
+ * does when it is out of memory; a program that allocates by other means calls
+ * this.  May be called at any time. */
+int kma_trim_scratch(void);
 /* Re-initialise in place, stream-ordered: the state clheap_init
  * (kma.cl:27-52) leaves, written by parallel bulk stores. */
 int kma_reset(kma_heap_t h, void *stream);

@@ -7,8 +7,8 @@ is its host-side mirror: ``Heap`` (kma_create/kma_destroy), ``Workload``
 """
 from ._lib import (KMA_FLAG_BADFREE, KMA_FLAG_TIMEOUT, MODE_PLAIN, MODE_WARP, WL_C1, WL_C2,
                    KmaError, lib)
-from .heap import Heap, Workload, bench_atomics, sbid_by_size, size_by_sbid, slots_by_size
+from .heap import Heap, Workload, bench_atomics, sbid_by_size, size_by_sbid, slots_by_size, trim_scratch
 
 __all__ = ["Heap", "Workload", "KmaError", "lib", "bench_atomics", "size_by_sbid",
-           "slots_by_size", "sbid_by_size", "MODE_PLAIN", "MODE_WARP", "WL_C1", "WL_C2",
+           "slots_by_size", "sbid_by_size", "trim_scratch", "MODE_PLAIN", "MODE_WARP", "WL_C1", "WL_C2",
            "KMA_FLAG_TIMEOUT", "KMA_FLAG_BADFREE"]

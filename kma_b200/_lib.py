@@ -124,6 +124,7 @@ SIGNATURES = [
     ("kma_create", c_void_p, [c_int, c_void_p, c_uint]),
     ("kma_create_ex", c_int, [POINTER(KmaConfig), c_void_p, POINTER(c_void_p)]),
     ("kma_destroy", c_int, [c_void_p]),
+    ("kma_trim_scratch", c_int, []),
     ("kma_reset", c_int, [c_void_p, c_void_p]),
     ("kma_heap_device_ptr", c_void_p, [c_void_p]),
     ("kma_get_info", c_int, [c_void_p, POINTER(KmaInfo)]),

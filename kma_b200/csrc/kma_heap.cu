@@ -386,6 +386,12 @@ extern "C" const char *kma_strerror(int err)
 	}
 }
 
+extern "C" int kma_trim_scratch(void)
+{
+	kma_scratch_trim();
+	return KMA_OK;
+}
+
 extern "C" const char *kma_version(void) { return "kma_b200 1.1 sm_100a"; }
 
 extern "C" int kma_snapshot(kma_heap_t h, void *stream, uint32_t *cls, uint32_t *state,

@@ -11,9 +11,9 @@
  *   - bounded: at most KMA_SCRATCH_KEEP bytes per process, in at most
  *     KMA_SCRATCH_LIST buffers, stay on the list, the oldest leave first; a
  *     larger buffer is never kept;
- *   - given back: when a heap or a PMA heap is destroyed, and whenever an
- *     allocation of the library fails (kma_device_malloc empties the list and
- *     tries again);
+ *   - given back: when a heap or a PMA heap is destroyed, when the program asks
+ *     for it (kma_trim_scratch), and whenever an allocation of the library
+ *     fails (kma_device_malloc empties the list and tries again);
  *   - a buffer belongs to one call at a time (the list is behind a mutex) and
  *     returns to the list only when the default stream, on which all of these
  *     calls work, is idle, so nothing can still use it;

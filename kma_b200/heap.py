@@ -293,6 +293,11 @@ class Workload:
         return nlive, off, size
 
 
+def trim_scratch() -> None:
+    """Give the device memory that host calls keep between them back to CUDA."""
+    check(lib().kma_trim_scratch(), "kma_trim_scratch")
+
+
 def bench_atomics(distinct: bool, threads: int, iters: int, stride_words: int = 32,
                   stream=None) -> float:
     """Milliseconds for threads*iters returning 32-bit atomicAdds."""

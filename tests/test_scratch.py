@@ -61,3 +61,15 @@ def test_kept_scratch_is_bounded_and_given_back(threads, per, kept):
     with Heap(64, 12):
         pass
     assert before - _free() < 64 << 20
+
+
+def test_a_program_gets_the_scratch_back():
+    """For an allocation that is not the library's: no heap is destroyed."""
+    import kma_b200
+    from kma_b200 import structs
+    kma_b200.trim_scratch()
+    before = _free()
+    structs.c3_queue(structs.C3_CLQUEUE, 1 << 17, 64, 4096)  # 16 bytes a payload
+    assert before - _free() >= (1 << 23) * 16
+    kma_b200.trim_scratch()
+    assert before - _free() < 64 << 20
