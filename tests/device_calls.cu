@@ -25,6 +25,18 @@ __global__ void k_replay_hint(kma_heap *h, const long long *ops, long long n, lo
 	}
 }
 
+/* One thread, lane `lane` of warp `warp` of the grid, mallocs up to `count`
+ * blocks of n bytes, until it is refused one. */
+__global__ void k_malloc_at(kma_heap *h, unsigned warp, unsigned lane, unsigned n, unsigned count, unsigned *got)
+{
+	if (blockIdx.x != warp || threadIdx.x != lane)
+		return;
+	unsigned k = 0;
+	while (k < count && kma_malloc(h, n))
+		k++;
+	*got = k;
+}
+
 /* One warp: lane 0 puts n items on each of nq queues, the head of each then
  * held for good if `stuck`; every lane takes one from queue lane % nq, with an
  * error word of its own and a limit that `step` makes differ.  out: the item's
@@ -61,6 +73,13 @@ __global__ void k_user_iqueue(kma_iqueue *q, unsigned long long *sum)
 		atomicAdd(sum, reinterpret_cast<unsigned long long *>(it)[1]);
 }
 } /* namespace */
+
+extern "C" int t_malloc_at(kma_heap *h, unsigned warp, unsigned lane, unsigned n, unsigned count, unsigned *got)
+{
+	k_malloc_at<<<warp + 1, 32>>>(h, warp, lane, n, count, got);
+	const cudaError_t e = cudaGetLastError();
+	return e != cudaSuccess ? e : cudaDeviceSynchronize();
+}
 
 extern "C" int t_lanes_dequeue(void *q, unsigned long long *items, int nq, int n, int stuck, uint32_t step, int *out,
 		uint32_t *err)

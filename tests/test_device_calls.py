@@ -95,3 +95,30 @@ def test_every_lane_learns_of_its_expired_wait(calls, nq, step):
     from kma_b200 import KMA_FLAG_TIMEOUT
     out, err = _lanes(calls, nq, 3, 1, step)
     assert (out == -1).all() and ((err & KMA_FLAG_TIMEOUT) != 0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shards,at,other", [(2, 0, 1), (9, 0, 8), (9, 3, 2), (66, 0, 1), (66, 0, 7), (66, 0, 8), (66, 0, 9),
+                                             (66, 0, 63), (66, 0, 64), (66, 0, 65), (66, 40, 9), (66, 65, 0)])
+def test_an_exhausted_heap_serves_from_the_next_64_shards(calls, shards, at, other):
+    """The free list is empty and shard `other` has a superblock with slots
+    left: per-thread calls of shard `at` get all of them, if it is near enough."""
+    import torch
+    from kma_b200 import Heap, slots_by_size
+    n = 32
+    with Heap(shards * 32 + 1, 12, shards=shards) as h:
+        got = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+        def malloc_at(shard, size, count):
+            rc = calls.t_malloc_at(ctypes.c_void_p(h.device_ptr), shard // 8, shard % 8, size, count,
+                                   ctypes.c_void_p(got.data_ptr()))
+            assert rc == 0
+            return int(got[0])
+
+        assert malloc_at(other, n, 1) == 1
+        full = malloc_at(at, 4000, 1 << 20)  # one block to a superblock: the free list runs empty
+        assert 0 < full < 1 << 20
+        near = 1 <= (other - at) % shards <= 64
+        assert malloc_at(at, n, 1 << 20) == (slots_by_size(12, n) - 1 if near else 0)
+        assert malloc_at(at, n, 1) == 0
+        assert h.error_flags() == 0
