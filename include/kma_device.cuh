@@ -87,6 +87,7 @@
 #define KMA_ERR_AT_RING_DEQ (1u << 11)  /* ring: slot not yet filled */
 #define KMA_ERR_AT_CLAIM (1u << 12)     /* plain malloc: bitmap claim */
 #define KMA_ERR_AT_MALLOC (1u << 13)    /* plain malloc: reservation */
+#define KMA_ERR_AT_FREE (1u << 14)      /* plain free: no wait of its own any more, never set */
 #define KMA_ERR_AT_RESERVE (1u << 15)   /* warp malloc: reservation (POISON / stale waits) */
 #define KMA_ERR_AT_WARP (1u << 16)      /* warp malloc: leader turns */
 
@@ -502,11 +503,6 @@ __device__ __forceinline__ int ring_put(kma_heap *h, unsigned long long pos, uin
 	}
 	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RING_ENQ);
 	return 0;
-}
-__device__ __forceinline__ void ring_enqueue(kma_heap *h, uint32_t s, uint32_t detached)
-{
-	if (ring_put(h, add64_relaxed(&h->free_tail.v, 1ull), s, detached))
-		atomicAdd(&h->ring_avail.v, 1u);
 }
 /* The calling lanes (`active`) that `want` to put theirs take tickets
  * together.  Every lane of `active` calls. */
@@ -955,10 +951,6 @@ __device__ inline void kma_free(kma_heap *h, void *p)
 /* instead of two or three per lane.  A single calling lane follows     */
 /* exactly the plain path's choices.                                    */
 /* ------------------------------------------------------------------ */
-namespace kma_detail {
-
-} /* namespace kma_detail */
-
 /* Optional event counts of the warp-collaborative calls (diagnostics):
  * pass a pointer to a per-thread tally to kma_malloc_warp/kma_free_warp;
  * with the default null pointer the counting compiles away. */

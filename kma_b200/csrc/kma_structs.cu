@@ -150,9 +150,6 @@ extern "C" int kma_pma_head(kma_pma_t p, void *stream, uint64_t *head)
 	return KMA_OK;
 }
 
-namespace {
-} /* namespace */
-
 /* run a one-thread replay kernel over host op/out arrays */
 template <typename F>
 static int replay_host(int64_t n, const int64_t *ops, int64_t *out, F launch)

@@ -32,10 +32,9 @@
 #define KMA_TC_UNSORTED 3 /* nodes outside their interval */
 #define KMA_TC_OVERFLOW 4 /* more nodes reachable than the list holds */
 #define KMA_TC_COUNT 5    /* [3] entries pushed by a level, by level number mod 3 */
-#define KMA_TC_BEGIN 8    /* the level block 0 stopped at: first entry, */
-#define KMA_TC_END 9      /* end, */
-#define KMA_TC_LEVEL 10   /* and number */
-#define KMA_TC_WORDS 12
+#define KMA_TC_BEGIN 8    /* the level block 0 stopped at: first entry */
+#define KMA_TC_END 9      /* and end */
+#define KMA_TC_WORDS 10
 
 namespace {
 
