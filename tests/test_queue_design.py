@@ -278,3 +278,53 @@ def test_text_of_lanes_conserves_and_keeps_order(harness, cfg, kind, lanes):
     assert rc == 0 and st.get("ok"), st
     assert st["taken"] + st["left"] >= st["appended"] > 0
     assert st["conservation_faults"] == 0 and st["order_faults"] == 0 and st["timeouts"] == 0
+
+
+# the texts of the warp and of lanes without a log, and the single-item one:
+# (kind, configuration with its LANES, old, new)
+LANES_MUTANTS = {
+    "v_no_head_recheck": ("clq", "8 20000 4 4 0.01 2 2 0.5 64 0 1",
+                          "\t\t    }) != h) {\n\t\t\tV::one([&] {\n\t\t\t\tO::st(hl, nx);",
+                          "\t\t    }) == ~0ull) {\n\t\t\tV::one([&] {\n\t\t\t\tO::st(hl, nx);"),
+    "v_last_item_no_tail_cas": ("clq", "8 20000 1 1 0.01 1 1 0.5 64 0 1",
+                                "if (V::one([&] { return O::cas(tailw, hp, 0ull); }) == hp) {",
+                                "if (V::one([&] { O::st(tailw, 0ull); return hp; }) == hp) {"),
+    # the item that stays as the head, one too early
+    "v_wrong_new_head": ("clq", "8 5000 -32 -250 0.02 15 4 0 65536 1 1",
+                         "m--;\n\t\t\t\t\t\tnh = V::get(item, (p + m) & 31u);",
+                         "nh = V::get(item, (p + m - 1u) & 31u);"),
+    "walk_no_head_recheck": ("clq", "8 20000 4 4 0.01 2 2 0.5 0 0 3",
+                             "if (v.one([&] { return O::ld(headw); }) != h) {", "if (false) {"),
+    "walk_last_item_no_tail_cas": ("clq", "8 20000 1 1 0.01 1 1 0.5 0 0 3",
+                                   "if (v.one([&] { return O::cas(tailw, cur, 0ull); }) == cur) {",
+                                   "if (v.one([&] { O::st(tailw, 0ull); return cur; }) == cur) {"),
+    "iq_walk_hold_store": ("iq", "8 20000 4 4 0.01 2 2 0.5 0 0 3",
+                           "if (v.one([&] { return O::cas(headw, hd, tw_make(tw_tag(hd) + 1u, cur)); }) != hd) {",
+                           "if (v.one([&] { O::st(headw, tw_make(tw_tag(hd) + 1u, cur)); return hd; }) != hd) {"),
+    "iq_single_uncounted": ("iq", "8 20000 1 1 0.01 1 1 0.5 0 0 1",
+                            "O::cas(headw, hd, tw_make(tw_tag(hd) + 2u, next));",
+                            "O::cas(headw, hd, tw_make(tw_tag(hd), next));"),
+    "iq_single_store": ("iq", "8 20000 4 4 0.01 2 2 0.5 0 0 1",
+                        "const u64 now = O::cas(headw, hd, tw_make(tw_tag(hd) + 2u, next));",
+                        "O::st(headw, tw_make(tw_tag(hd) + 2u, next));\n\t\tconst u64 now = hd;"),
+}
+
+
+@pytest.mark.parametrize("name", sorted(LANES_MUTANTS))
+def test_harness_detects_mistakes_in_the_lanes_texts(harness, tmp_path, name):
+    kind, cfg, old, new = LANES_MUTANTS[name]
+    src = open(ALGO).read()
+    assert src.count(old) == 1, f"mutation site of {name} not found once"
+    (tmp_path / "kma_queue_algo.cuh").write_text(src.replace(old, new))
+    binary = str(tmp_path / "h")
+    subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-pthread", "-w", f"-I{tmp_path}", "-o", binary,
+                    os.path.join(ORACLE, "queue_harness.cpp")], check=True)
+    for seed in range(4):
+        args = cfg.split()
+        args[5] = str(int(args[5]) + 100 * seed)
+        try:
+            if run(binary, kind, " ".join(args), timeout=120)[0] != 0:
+                return
+        except subprocess.TimeoutExpired:
+            return  # a wait that never ends is a detection too
+    raise AssertionError(f"mutant {name} passed unnoticed")
