@@ -417,6 +417,9 @@ KQ_FN uint32_t clq_dequeue_n(u64 *headw, u64 *tailw, u64 *out, uint32_t k, uint3
  * case.  The number is known
  *   - from two links of the chain that follow one another (clq_number), which
  *     the queue's own items carry.  A note is taken for true only so;
+ *     Where a name is missing, the link into the next chain gives half of its
+ *     number, and the record that is probably its is read beside the first
+ *     link of the chain, which gives the other half;
  *   - from the name of the record before, which has both chains' numbers.  It
  *     was written by an append that found the number of the chain before by
  *     the item its exchange of the tail gave it (`last`, `lookup`), and a tail
@@ -454,6 +457,14 @@ KQ_FN bool log_named(u64 name, uint32_t recno, uint32_t *behind)
 	return (name >> 24) == ((LOG_NAMED >> 24) | recno);
 }
 
+/* the number with the low bits that an into mark has, nearest to ref (mod 2^24):
+ * chains are appended about in the order of their numbers */
+KQ_FN uint32_t log_near(uint32_t ref, u64 into)
+{
+	const uint32_t up = ((uint32_t)(into >> PTR_BITS) - ref) & 0x3FFFu; /* steps up from ref */
+	return (up < 0x2000u ? ref + up : ref + up - 0x4000u) & LOG_RECNO_MASK;
+}
+
 /* After an append of logged chain recno: name it in the record of the chain
  * before it (whose last item is prev), if the log still knows which that is. */
 template <class LG>
@@ -484,20 +495,20 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 		if (hp == 0)
 			return 0;
 		u64 *hl = L::at(hp);
-		uint32_t recno = 0;
-		bool noted = false;
-		const u64 seen = V::one([&] {
+		/* the head's link (POISON: held) and its note, if there is one */
+		const u64 note = V::one([&] {
+			uint32_t no = 0;
 			const u64 l = O::ld_rlx(hl);
-			noted = log && log->resume(hp, &recno);
-			return l;
+			const bool is = log && log->resume(hp, &no);
+			return l == POISON ? POISON : is ? LOG_NAMED | no : 0ull;
 		});
-		if (seen == POISON) {
+		if (note == POISON) {
 			O::pause(it++);
 			continue;
 		}
-		/* the record of the note, if there is one, beside the exchange */
-		noted = V::one([&] { return noted; });
-		recno = V::one([&] { return recno; });
+		bool noted = note != 0;
+		uint32_t recno = (uint32_t)note;
+		/* its record beside the exchange */
 		vec raw, item, name; /* (name: the same in every lane; no wait for it here) */
 		typename V::template reg<bool> hit;
 		auto load_record = [&](vec &rec_of, vec &name_of, uint32_t no) {
@@ -514,27 +525,24 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 			O::pause(it++);
 			continue;
 		}
-		/* the link of the item behind the head, where the record agrees on
-		 * what item that is, beside the recheck */
-		u64 second = 0, l1 = 0;
+		/* beside the recheck, where the record agrees on what item is behind
+		 * the head, that item's link, which proves the note */
+		const u64 second = qp_ptr(nx);
 		if (noted) {
+			typename V::template reg<bool> behind;
 			V::each([&](uint32_t j) {
 				item[j] = qp_ptr(raw[j]);
 				hit[j] = item[j] == hp;
+				behind[j] = item[j] == second;
 			});
-			const uint32_t at = V::ballot(hit);
-			const vec next = V::above(item);
-			uint32_t p = 0;
-			while (at && !((at >> p) & 1u))
-				p++;
-			const u64 n = V::get(next, p);
-			second = at && p < LOG_CHAIN_MAX - 1u && n > POISON && n == qp_ptr(nx) ? n : 0ull;
+			noted = second > POISON && ((V::ballot(hit) << 1) & V::ballot(behind));
 		}
-		if (V::one([&] {
-			    if (second)
-				    l1 = O::ld_rlx(L::at(second));
-			    return O::ld(headw);
-		    }) != h) {
+		const uint32_t held = V::one([&] {
+			uint32_t no = 0;
+			const u64 l1 = noted ? O::ld_rlx(L::at(second)) : 0ull;
+			return O::ld(headw) != h ? 0u : noted && clq_number(nx, l1, &no) && no == recno ? 2u : 1u;
+		});
+		if (!held) {
 			V::one([&] {
 				O::st(hl, nx);
 				return 0u;
@@ -542,15 +550,13 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 			O::pause(it++);
 			continue;
 		}
-		if (noted) {
-			uint32_t no = 0;
-			l1 = V::one([&] { return l1; });
-			noted = second && clq_number(nx, l1, &no) && no == recno;
-		}
+		noted = held == 2u;
 		/* held: cur is the next item to take, curl its link where known */
 		uint32_t r = 0, chains = 0;
 		u64 cur = hp, curl = nx, into = 0, untried = ~0ull;
-		bool have = noted, end = nx == 0; /* have: raw is cur's chain's record, of number recno */
+		/* have: raw is the record of cur's chain, of number recno; guessed: recno
+		 * is probably that number */
+		bool have = noted, guessed = false, end = nx == 0;
 		while (r < k && !end) {
 			if (have) {
 				V::each([&](uint32_t j) {
@@ -605,7 +611,8 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 						if (whole && !end) {
 							into = ll;
 							have = named; /* and read, unless this was the last */
-							recno = named ? rahead : recno;
+							guessed = !named && (ll & CLQ_INTO) && !(ll & CLQ_LOG);
+							recno = named ? rahead : guessed ? log_near(recno, ll) : recno;
 							if (ahead) {
 								raw = rawn;
 								name = namen;
@@ -615,9 +622,12 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 					}
 					end = false;
 				}
-				have = false;
+				have = guessed = false;
 			}
-			/* no record that fits: one link */
+			/* no record that fits: one link, and beside it the record that is
+			 * probably the one */
+			if (guessed)
+				load_record(raw, name, recno);
 			if (!curl)
 				curl = V::one([&] { return O::ld(L::at(cur)); });
 			if (curl == 0 || curl == POISON)
@@ -632,12 +642,17 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 					lo = (into & ~(CLQ_INTO | PTR_MASK)) | qp_ptr(curl);
 				else if (qp_ptr(curl) > POISON)
 					lo = V::one([&] { return O::ld_rlx(L::at(qp_ptr(curl))); });
-				have = clq_number(curl, lo, &recno);
+				uint32_t no = 0;
+				have = clq_number(curl, lo, &no);
 				if (have) {
-					load_record(raw, name, recno);
+					if (!guessed || no != recno)
+						load_record(raw, name, no);
+					recno = no;
+					guessed = false;
 					continue;
 				}
 			}
+			guessed = false;
 			out.one(r++, cur);
 			into = curl;
 			cur = qp_ptr(curl);
@@ -645,7 +660,7 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 		}
 		if (r) {
 			V::one([&] {
-				if (have)
+				if (have || guessed)
 					log->note(cur, recno);
 				O::st(headw, qp_next(h, cur));
 				return 0u;

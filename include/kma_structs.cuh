@@ -702,9 +702,9 @@ __device__ inline uint32_t block_rank(bool want, unsigned int *cnt, uint32_t *to
  * without one (a walk, one item at a time) or in a block of less than a
  * warp its first thread, in turns of one hold of the head each.  A hold
  * takes several logged chains in a row, and is a chain of round trips
- * whatever the load: 4 to take the head, 1 or 2 a chain (26 M items/s in
+ * whatever the load: 4 to take the head, 1 or 2 a chain (27 M items/s in
  * batches of 256; 12.2 with one thread and 3 a chain), also where the chains
- * do not fill the batches (2^18 + 77 threads: 25.7; one thread, which walks
+ * do not fill the batches (2^18 + 77 threads: 26; one thread, which walks
  * from a head in the middle of a chain: 4).  smem: blockDim + 1 words of
  * shared memory the call may use.
  * Items go to the wanting threads in the order block_rank numbers them;

@@ -251,7 +251,7 @@ def test_a_log_outlives_the_items_it_has_recorded(harness, args):
 
 REUSE_MUTANTS = {
     # believe a note because the record has the head in it
-    "note_unproven": ("noted = second && clq_number(nx, l1, &no) && no == recno;", "noted = second != 0;"),
+    "note_unproven": ("noted && clq_number(nx, l1, &no) && no == recno ? 2u : 1u", "noted ? 2u : 1u"),
 }
 
 
@@ -284,8 +284,7 @@ def test_text_of_lanes_conserves_and_keeps_order(harness, cfg, kind, lanes):
 # (kind, configuration with its LANES, old, new)
 LANES_MUTANTS = {
     "v_no_head_recheck": ("clq", "8 20000 4 4 0.01 2 2 0.5 64 0 1",
-                          "\t\t    }) != h) {\n\t\t\tV::one([&] {\n\t\t\t\tO::st(hl, nx);",
-                          "\t\t    }) == ~0ull) {\n\t\t\tV::one([&] {\n\t\t\t\tO::st(hl, nx);"),
+                          "return O::ld(headw) != h ? 0u : noted", "return noted"),
     "v_last_item_no_tail_cas": ("clq", "8 20000 1 1 0.01 1 1 0.5 64 0 1",
                                 "if (V::one([&] { return O::cas(tailw, hp, 0ull); }) == hp) {",
                                 "if (V::one([&] { O::st(tailw, 0ull); return hp; }) == hp) {"),
