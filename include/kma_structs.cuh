@@ -222,9 +222,6 @@ struct lanes_out_regs {
 typedef gpu_ops_t<KMA_QUEUE_PAUSE_MAX_NS> gpu_ops;
 /* the warp and block forms */
 typedef gpu_ops_t<KMA_QUEUE_GROUP_PAUSE_MAX_NS> gpu_ops_group;
-/* single items of an indexed queue, which wait only while a group holds the
- * head, and hold nothing up themselves */
-typedef gpu_ops_t<256u> gpu_ops_one;
 /* Lanes that call a per-thread dequeue together (active, two at least), as the
  * queue algorithms' clq_walk_v and iq_walk_v take them: */
 struct gpu_some_lanes {
@@ -919,7 +916,7 @@ __device__ inline void *kma_iqueue_dequeue_shard(kma_iqueue *q, uint32_t shard)
 	for (uint32_t k = 0; k < 2; k++) {
 		uint32_t idx = 0;
 		bool timed_out = false;
-		if (!kma_q::iq_dequeue_1<gpu_ops_one>(L, &q->ends[2 * shard].v, &idx, q->spin_limit, &timed_out)) {
+		if (!kma_q::iq_dequeue_1<gpu_ops>(L, &q->ends[2 * shard].v, &idx, q->spin_limit, &timed_out)) {
 			if (timed_out)
 				atomicOr(&q->err, KMA_ERR_TIMEOUT);
 			return nullptr;
