@@ -14,9 +14,10 @@
  * serial execution of both yields identical offsets.
  *
  * Concurrent execution: a persistent grid walks the items round by round
- * (k_wl_rounds).  Each lane tags and verifies its own block with 16-byte
- * accesses unrolled by four, so a warp keeps many independent requests in
- * flight (the verify pass is bound by memory latency, not by bandwidth).
+ * (k_wl_rounds).  Lanes tag and verify their own small blocks, the whole warp
+ * the larger ones, with several 16-byte accesses of each lane in flight
+ * (coop_fill, coop_verify: the verify pass is bound by memory latency, not by
+ * bandwidth).
  * The per-item state (PRNG, ordered malloc hash, live table) lives in
  * device scratch owned by the kma_wl handle.
  */
@@ -329,7 +330,7 @@ __device__ __forceinline__ void flush_counters(const wl_dev &w, uint32_t mask, u
  * their rounds and pin their last live blocks while later waves start,
  * which fragments the heap far beyond what concurrent items do.) */
 /* PER_SM: blocks an SM must hold, 4 (64 registers a thread) or, when half the
- * GPU's threads hold every item, 2 (wl_per_sm). */
+ * GPU's threads hold every item, 2 (wl_rounds_launch). */
 template <int MODE, bool C2, int PER_SM>
 __global__ void __launch_bounds__(WL_BLOCK, PER_SM) k_wl_rounds(kma_heap *h, wl_dev w, uint32_t nrounds, int drain)
 {
@@ -394,8 +395,8 @@ wl_rounds_fn wl_rounds_of(bool c2, bool wide)
  * When there are no more items than 2 blocks an SM hold, the instantiation
  * with 128 registers a thread runs them: nothing spills, and six vectors are
  * in flight in the verify instead of three (50021 items, per thread / warp
- * calls: 1.10 and 0.87 ms a launch instead of 1.17 and 0.90).  With more, the missing warps cost more (config 2
- * with 24 warps an SM: +9%). */
+ * calls: 1.10 and 0.87 ms a launch instead of 1.17 and 0.90).  With more, the
+ * missing warps cost more (config 2 with 24 warps an SM: +9%). */
 int wl_rounds_launch(const wl_dev &d, kma_heap *h, int device, uint32_t nrounds, int mode, uint32_t bd, int drain,
 		cudaStream_t st)
 {
