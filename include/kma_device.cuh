@@ -728,11 +728,13 @@ __device__ __forceinline__ void *sb_get_block(kma_heap *h, uint32_t s, uint32_t 
  *
  * A refusal pays for the look, so KMA_STEAL_ROW class words are read at a time:
  * a refused call by one thread takes 6.7 us (18 a word at a time, 1.0 without
- * the look), by 148 x 256 threads on 16 MiB / 224 MiB of heap 766 / 105 us
- * (943 / 141; 454 / 155), by 592 x 512 6.2 / 1.3 ms (7.9 / 1.4; 47 / 1.3).
- * Rows of 16 and 32 take 64 and 96 registers for the same. */
+ * the look), by 148 x 256 threads on 16 MiB / 224 MiB of heap 713 / 109 us
+ * (943 / 141; 454 / 155), by 592 x 512 7.7 / 1.3 ms (7.9 / 1.4; 47 / 1.3).
+ * Longer rows are no faster, and their registers are the caller's: with the
+ * words of 8 at hand until they are tried, the graph build had 72 instead of
+ * 64, and 22% more time. */
 #define KMA_STEAL_SHARDS 64u
-#define KMA_STEAL_ROW 8u
+#define KMA_STEAL_ROW 4u
 /* (below 2 n) */
 __device__ __forceinline__ uint32_t *steal_word(kma_heap *h, uint32_t c, uint32_t shard, uint32_t n)
 {
@@ -742,22 +744,17 @@ static __device__ __noinline__ void *steal_block(kma_heap *h, uint32_t c, uint32
 {
 	const uint32_t n = h->cls_nsh[c], most = n - 1 < KMA_STEAL_SHARDS ? n - 1 : KMA_STEAL_SHARDS;
 	for (uint32_t base = 1; base <= most; base += KMA_STEAL_ROW) {
-		uint32_t cur[KMA_STEAL_ROW];
+		uint32_t named = 0; /* those that name a superblock */
 #pragma unroll
 		for (uint32_t i = 0; i < KMA_STEAL_ROW; i++)
-			cur[i] = base + i <= most ? ld_relaxed(steal_word(h, c, shard + base + i, n)) : 0u;
-		/* the first that names a superblock and is not tried yet */
-		for (uint32_t from = 0;;) {
-			uint32_t at = KMA_STEAL_ROW, s = 0;
-#pragma unroll
-			for (uint32_t i = KMA_STEAL_ROW; i-- > 0;)
-				if (i >= from && cur[i] >= KMA_CLS_BASE) {
-					at = i;
-					s = cur[i] - KMA_CLS_BASE;
-				}
-			if (at == KMA_STEAL_ROW)
-				break;
-			from = at + 1;
+			if (base + i <= most)
+				named |= (uint32_t)(ld_relaxed(steal_word(h, c, shard + base + i, n)) >= KMA_CLS_BASE) << i;
+		for (; named; named &= named - 1) {
+			uint32_t *clsw = steal_word(h, c, shard + base + (__ffs(named) - 1), n);
+			const uint32_t cur = ld_relaxed(clsw);
+			if (cur < KMA_CLS_BASE)
+				continue;
+			const uint32_t s = cur - KMA_CLS_BASE;
 			for (uint32_t tries = 0; tries < 4; tries++) {
 				const uint32_t st = ld_relaxed(&h->sb_state[s]);
 				if (st_class(st) != c || st_free(st) == 0)
@@ -767,7 +764,7 @@ static __device__ __noinline__ void *steal_block(kma_heap *h, uint32_t c, uint32
 				if (cas_relaxed(&h->sb_state[s], st, st - 1) != st)
 					continue;
 				if (fr == 0)
-					cas_relaxed(steal_word(h, c, shard + base + at, n), s + KMA_CLS_BASE, 0);
+					cas_relaxed(clsw, cur, 0);
 				return sb_get_block(h, s, c, fr, v);
 			}
 		}

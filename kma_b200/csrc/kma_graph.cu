@@ -146,9 +146,12 @@ __device__ __forceinline__ void gr_find_both(kma_cltree *tree, uint32_t a, uint3
 	*nb = fb ? gr_of_tree(reinterpret_cast<kma_cltree_node *>(cb)) : nullptr;
 }
 
-/* clTree_test (tb_clTree.cl:40-85) */
+/* clTree_test (tb_clTree.cl:40-85).  At most 64 registers a thread: a search
+ * is bound by its round trips, so the more warps an SM holds the better (2^22
+ * uniform edges by 1024 threads an SM: 7.2 ms, 8.9 at 72 registers, where a
+ * quarter of them waits for the others to end). */
 template <class B>
-__global__ void k_gr_build(gr_dev<B> g, const uint32_t *edges, uint64_t n)
+__global__ void __launch_bounds__(256, 4) k_gr_build(gr_dev<B> g, const uint32_t *edges, uint64_t n)
 {
 	uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
 	unsigned long long lost = 0, nulls = 0;
