@@ -504,6 +504,11 @@ __device__ __forceinline__ int ring_put(kma_heap *h, unsigned long long pos, uin
 	set_err(h, KMA_ERR_TIMEOUT | KMA_ERR_AT_RING_ENQ);
 	return 0;
 }
+__device__ __forceinline__ void ring_enqueue(kma_heap *h, uint32_t s, uint32_t detached)
+{
+	if (ring_put(h, add64_relaxed(&h->free_tail.v, 1ull), s, detached))
+		atomicAdd(&h->ring_avail.v, 1u);
+}
 /* The calling lanes (`active`) that `want` to put theirs take tickets
  * together.  Every lane of `active` calls. */
 __device__ __forceinline__ void ring_enqueue_lanes(kma_heap *h, uint32_t active, bool want, uint32_t s,
@@ -849,9 +854,9 @@ __device__ __forceinline__ bool block_locate(const kma_heap *h, const void *p, u
 	return slot < h->cls_slots[c];
 }
 
-/* Return superblock s (class c, state word `full`: every slot free) to the
- * free list unless a reservation gets in first: kma.cl:350-367.  The lanes
- * of `active` that have one do it together; every lane of it calls.
+/* Detach superblock s (class c, state word `full`: every slot free) from its
+ * class, unless a reservation gets in first: kma.cl:350-367.  True: it is the
+ * caller's to put on the free list; *seen: what its class slot held.
  *
  * The CAS that takes the count away detaches s: from then on, until it is on
  * the free list, nobody else can reserve from it, recycle it or give it another
@@ -863,19 +868,35 @@ __device__ __forceinline__ bool block_locate(const kma_heap *h, const void *p, u
  * relaxed load is served at L2, where that store already was; a plain one may
  * be served from this SM's L1, where a line of sb_home read during an earlier
  * incarnation can still sit. */
-__device__ __forceinline__ void sb_recycle(kma_heap *h, uint32_t active, bool all_free, uint32_t s, uint32_t c,
+__device__ __forceinline__ bool sb_detach(kma_heap *h, uint32_t s, uint32_t c, uint32_t full, uint32_t *seen)
+{
+	if (cas_relaxed(&h->sb_state[s], full, st_make(c, st_slots(full), 0)) != full)
+		return false;
+	*seen = cas_relaxed(cls_word(h, c, ld_relaxed16(&h->sb_home[s])), s + KMA_CLS_BASE, 0);
+	return true;
+}
+/* Recycle it, by one thread. */
+__device__ __forceinline__ void sb_recycle(kma_heap *h, uint32_t s, uint32_t c, uint32_t full)
+{
+	uint32_t seen = 0;
+	if (!sb_detach(h, s, c, full, &seen))
+		return;
+	if (h->flags & KMA_HEAP_RING)
+		ring_enqueue(h, s, seen);
+	else
+		msq_enqueue(h, s);
+}
+/* The lanes of `active` that have one (all_free) recycle theirs together;
+ * every lane of it calls. */
+__device__ __forceinline__ void sb_recycle_lanes(kma_heap *h, uint32_t active, bool all_free, uint32_t s, uint32_t c,
 		uint32_t full)
 {
-	uint32_t old = 0;
-	bool mine = false;
-	if (all_free)
-		mine = cas_relaxed(&h->sb_state[s], full, st_make(c, st_slots(full), 0)) == full;
+	uint32_t seen = 0;
+	const bool mine = all_free && sb_detach(h, s, c, full, &seen);
 	if (!__any_sync(active, mine))
 		return;
-	if (mine)
-		old = cas_relaxed(cls_word(h, c, ld_relaxed16(&h->sb_home[s])), s + KMA_CLS_BASE, 0);
 	if (h->flags & KMA_HEAP_RING)
-		ring_enqueue_lanes(h, active, mine, s, old);
+		ring_enqueue_lanes(h, active, mine, s, seen);
 	else if (mine)
 		msq_enqueue(h, s);
 }
@@ -928,9 +949,12 @@ __device__ inline void kma_free(kma_heap *h, void *p)
 	/* kma.cl:343-367 re-reads and CASes the count until it fits; an add
 	 * cannot miss, and lanes that free into one superblock need not queue */
 	const uint32_t full = atomicAdd(&h->sb_state[s], 1u) + 1u;
-	const bool all_free = st_free(full) == st_slots(full);
-	const uint32_t active = __activemask();
-	sb_recycle(h, active, all_free, s, c, full);
+	/* by itself: a per-thread call stands in whatever divergent code its caller
+	 * has, where the lanes that seem to run with it need not take part in a
+	 * vote or a shuffle with it (recycling together, threads of the graph build
+	 * got tickets that nobody had drawn) */
+	if (st_free(full) == st_slots(full))
+		sb_recycle(h, s, c, full);
 }
 
 /* ------------------------------------------------------------------ */
@@ -1444,7 +1468,7 @@ __device__ inline void kma_free_warp(kma_heap *h, void *p)
 	}
 	/* 3) kma.cl:350-367: all free -- recycle */
 	if (__any_sync(active, all_free))
-		sb_recycle(h, active, all_free, s, c, full);
+		sb_recycle_lanes(h, active, all_free, s, c, full);
 }
 
 #endif /* KMA_DEVICE_CUH */

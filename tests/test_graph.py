@@ -106,3 +106,20 @@ def test_gpu_graph_long_queue(n, threads):
             np.testing.assert_array_equal(*((got, want) if threads == 1 else (np.sort(got), np.sort(want))))
         assert ins.check_canonical_empty(h.snapshot(), h.bitmaps()) == []
         assert h.error_flags() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("edges,vertices,threads", [(2188, 547, 4096), (14928, 3732, 151552)])
+def test_gpu_losers_of_inserts_give_their_blocks_back(edges, vertices, threads):
+    """Small graphs by many threads: most inserts are lost, and the losers'
+    per-thread frees, in divergent code, empty superblocks all the time.  No
+    wait of the heap expires, and every superblock comes back."""
+    from kma_b200 import Heap, graph
+    from kma_b200 import inspect as ins
+    e = graph.synth_edges(edges, edges, vertices)
+    with Heap((1 << 30) >> 14, 14) as h:
+        for _ in range(40):
+            st, _ = graph.build(h, e, threads=threads, free_after=True)
+            assert st["err"] == 0 and st["nulls"] == 0 and st["links"] == edges
+            assert h.error_flags() == 0
+        assert ins.check_canonical_empty(h.snapshot(), h.bitmaps()) == []

@@ -97,8 +97,7 @@ static uint32_t cas_relaxed(uint32_t *p, uint32_t c, uint32_t v)
 	return old;
 }
 static uint32_t *cls_word(kma_heap *, uint32_t, uint32_t shard) { return &h.cls[shard]; }
-static bool __any_sync(uint32_t, bool b) { return b; }
-static void ring_enqueue_lanes(kma_heap *, uint32_t, bool want, uint32_t, uint32_t) { listed += want; }
+static void ring_enqueue(kma_heap *, uint32_t, uint32_t) { listed++; }
 static void msq_enqueue(kma_heap *, uint32_t) { listed++; }
 %s
 int main(int, char **argv)
@@ -118,7 +117,7 @@ int main(int, char **argv)
 		h.sb_home[1] = 5;
 		h.cls[5] = 1 + KMA_CLS_BASE;
 	};
-	sb_recycle(&h, 1, true, 1, CLS, full);
+	sb_recycle(&h, 1, CLS, full);
 	bool bad = listed != 1 || h.sb_state[1] != st_make(CLS, 7, 0);
 	for (uint32_t w : h.cls)
 		bad |= w == 1 + KMA_CLS_BASE; /* no slot names a superblock on the free list */
@@ -128,10 +127,10 @@ int main(int, char **argv)
 """
 
 
-def function(name: str) -> str:
+def function(name: str, returns: str = "void") -> str:
     """The text of the function `name` of kma_device.cuh."""
     src = open(DEVICE).read()
-    at = src.index(f"__device__ __forceinline__ void {name}(")
+    at = src.index(f"__device__ __forceinline__ {returns} {name}(")
     return src[at:src.index("\n}\n", at) + 3]
 
 
@@ -158,7 +157,7 @@ def test_a_superblock_is_reserved_from_only_after_its_bitmap(tmp_path):
 def test_a_recycled_superblock_leaves_its_current_home(tmp_path, ring):
     """Whenever another thread gets in between: a superblock on the free list
     is in nobody's class slot."""
-    binary = build(tmp_path, RECYCLE % function("sb_recycle"))
+    binary = build(tmp_path, RECYCLE % (function("sb_detach", "bool") + function("sb_recycle")))
     for before in range(5):
         r = subprocess.run([binary, str(before), str(ring)], capture_output=True, text=True, timeout=60)
         assert r.returncode == 0, (before, r.stdout)
