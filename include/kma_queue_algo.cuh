@@ -698,95 +698,6 @@ KQ_FN uint32_t clq_dequeue_v(u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint3
 	return 0;
 }
 
-/* clq_dequeue_n without a log, by lanes that each want one item: one of them
- * does what it does, and an item goes to its lane as it is met.  (As an array
- * of 32, handed out at the end, the items are 256 bytes of local memory, and
- * with the log's text beside it the caller's kernel took 128 registers.)  The
- * links behind a held head are read relaxed, one from the other; the fence
- * that makes the items' contents visible comes once, after the hold.
- * v.one(f): f() on one of the lanes, its result on all of them; v.fence(): as
- * V::fence() above; k: how many lanes there are, at most. */
-template <class O, class L, class V, class OUT>
-KQ_FN uint32_t clq_walk_v(const V &v, u64 *headw, u64 *tailw, OUT &out, uint32_t k, uint32_t limit, bool *timed_out)
-{
-	*timed_out = false;
-	uint32_t it = 0, idle = 0;
-	u64 last = ~0ull;
-	for (;;) {
-		const u64 h = v.one([&] { return O::ld_rlx(headw); });
-		if (h != last) {
-			last = h;
-			idle = 0;
-		} else if (++idle >= limit) {
-			break;
-		}
-		u64 cur = qp_ptr(h);
-		if (cur == 0)
-			return 0;
-		u64 *hl = L::at(cur);
-		u64 next = v.one([&] {
-			const u64 seen = O::ld_rlx(hl);
-			return seen == POISON ? POISON : O::xchg(hl, POISON);
-		});
-		if (next == POISON) {
-			O::pause(it++);
-			continue;
-		}
-		if (v.one([&] { return O::ld(headw); }) != h) {
-			v.one([&] {
-				O::st(hl, next);
-				return 0u;
-			});
-			O::pause(it++);
-			continue;
-		}
-		/* held: next is cur's link, and cur has its POISON */
-		uint32_t r = 0;
-		while (next != 0) {
-			out.one(r++, cur);
-			cur = qp_ptr(next);
-			if (r == k)
-				break;
-			/* cur is the last linked item, and stays as the head, unless it
-			 * has a successor */
-			next = v.one([&] {
-				const u64 n = O::ld_rlx(L::at(cur));
-				if (n == 0 || n == POISON)
-					return 0ull;
-				O::st_rlx(L::at(cur), POISON);
-				return n;
-			});
-		}
-		if (r) {
-			v.one([&] {
-				O::st(headw, qp_next(h, cur));
-				return 0u;
-			});
-			v.fence();
-			return r;
-		}
-		/* cur is the last linked item: see clq_dequeue_n */
-		if (v.one([&] { return O::cas(tailw, cur, 0ull); }) == cur) {
-			v.one([&] {
-				O::st(headw, qp_next(h, 0ull));
-				return 0u;
-			});
-			out.one(0, cur);
-			return 1;
-		}
-		v.one([&] {
-			O::st(hl, 0ull);
-			return 0u;
-		});
-		while (idle < limit && v.one([&] { return O::ld(hl); }) == 0ull && v.one([&] { return O::ld(headw); }) == h) {
-			O::pause(it++);
-			idle++;
-		}
-	}
-	*timed_out = true;
-	return 0;
-}
-
 /* ------------------------------------------------------------------ */
 /* indexed queue (clIndexedQueue)                                      */
 /* ------------------------------------------------------------------ */
@@ -983,56 +894,6 @@ KQ_FN uint32_t iq_dequeue_n(const Q &q, u64 *headw, uint32_t *out, uint32_t k, u
 			}
 		}
 		O::st(headw, tw_make(tw_tag(hd) + 2u, cur));
-		return r;
-	}
-	*timed_out = true;
-	return 0;
-}
-
-/* iq_dequeue_n without a log, by lanes that each want one item (see
- * clq_walk_v). */
-template <class O, class Q, class V, class OUT>
-KQ_FN uint32_t iq_walk_v(const V &v, const Q &q, u64 *headw, OUT &out, uint32_t k, uint32_t limit, bool *timed_out)
-{
-	*timed_out = false;
-	uint32_t idle = 0;
-	u64 last = ~0ull;
-	for (uint32_t it = 0;; it++) {
-		const u64 hd = v.one([&] { return O::ld_rlx(headw); });
-		if (hd != last) {
-			last = hd;
-			idle = 0;
-		} else if (++idle >= limit) {
-			break;
-		}
-		if (iq_head_held(hd)) {
-			O::pause(it);
-			continue;
-		}
-		uint32_t cur = tw_idx(hd), r = 0;
-		if (tw_idx(v.one([&] { return O::ld_rlx(q.link(cur)); })) == 0) {
-			/* only the dummy: empty, if the head is still this one */
-			if (v.one([&] { return O::ld_rlx(headw); }) == hd)
-				return 0;
-			continue;
-		}
-		if (v.one([&] { return O::cas(headw, hd, tw_make(tw_tag(hd) + 1u, cur)); }) != hd) {
-			O::pause(it);
-			continue;
-		}
-		/* held: the items behind the head cannot leave the queue */
-		while (r < k) {
-			const uint32_t nx = tw_idx(v.one([&] { return O::ld_rlx(q.link(cur)); }));
-			if (nx == 0)
-				break;
-			out.one(r++, cur);
-			cur = nx;
-		}
-		v.one([&] {
-			O::st(headw, tw_make(tw_tag(hd) + 2u, cur));
-			return 0u;
-		});
-		v.fence();
 		return r;
 	}
 	*timed_out = true;

@@ -222,42 +222,6 @@ struct lanes_out_regs {
 typedef gpu_ops_t<KMA_QUEUE_PAUSE_MAX_NS> gpu_ops;
 /* the warp and block forms */
 typedef gpu_ops_t<KMA_QUEUE_GROUP_PAUSE_MAX_NS> gpu_ops_group;
-/* Lanes that call a per-thread dequeue together (active, two at least), as the
- * queue algorithms' clq_walk_v and iq_walk_v take them: */
-struct gpu_some_lanes {
-	uint32_t active;
-	/* whether all of them have the same key */
-	template <class T>
-	__device__ __forceinline__ bool share(T key) const
-	{
-		return __all_sync(active, __shfl_sync(active, key, __ffs(active) - 1) == key);
-	}
-	template <class F>
-	__device__ __forceinline__ auto one(F f) const -> decltype(f())
-	{
-		decltype(f()) r = 0;
-		if (lane_id() == (uint32_t)__ffs(active) - 1)
-			r = f();
-		return __shfl_sync(active, r, __ffs(active) - 1);
-	}
-	__device__ __forceinline__ void fence() const { fence_acqrel(); }
-	__device__ __forceinline__ uint32_t rank() const { return __popc(active & lanemask_lt()); }
-	__device__ __forceinline__ uint32_t size() const { return __popc(active); }
-};
-/* What they take: the lane of rank base + at gets item `at` of a hold.  Items
- * above `most` (an indexed queue's internal dummies) are nobody's. */
-template <class T>
-struct lanes_out_rank {
-	T mine, most;
-	uint32_t rank, base;
-	__device__ __forceinline__ void one(uint32_t at, T item)
-	{
-		if (item > most)
-			base--;
-		else if (rank == base + at)
-			mine = item;
-	}
-};
 
 } /* namespace kma_detail */
 
@@ -529,30 +493,14 @@ __device__ __forceinline__ int kma_clqueue_enqueue(kma_clqueue *q, kma_clqueue_i
 }
 
 /* dequeue (clQueue.cl:82-118): the oldest item, NULL when empty or on
- * spin-limit expiry (which also flags *err).  Lanes that call it together on
- * one queue (with one spin limit) take their items under one hold, as the
- * warp form does: each for itself they wait for one another's holds (2^16
- * payloads on one queue by 4096 threads: 24.6 ms, 142 each for itself; indexed
- * queue 22.5 and 73). */
+ * spin-limit expiry (which also flags *err).  Each thread takes its item by
+ * itself, also where lanes of a warp call it on one queue: a per-thread call
+ * may stand in divergent code, where no lane can count on another.  Many
+ * threads on one queue are served by the warp form (2^16 payloads by 4096
+ * threads: 7 ms, 142 with this one). */
 __device__ __forceinline__ kma_clqueue_item *kma_clqueue_dequeue(kma_clqueue *q, uint32_t *err = nullptr,
 		uint32_t spin_limit = KMA_STRUCT_SPIN)
 {
-	using namespace kma_detail;
-	const gpu_some_lanes v = {__activemask()};
-	if (v.size() > 1 && v.share((unsigned long long)q) && v.share(spin_limit)) {
-		lanes_out_rank<unsigned long long> o = {0ull, ~0ull, v.rank(), 0u};
-		bool timed_out = false;
-		for (uint32_t turn = 0; o.base < v.size() && turn < 32; turn++) {
-			const uint32_t r = kma_q::clq_walk_v<gpu_ops_group, clq_link_head>(v, &q->head, &q->tail, o,
-										   v.size() - o.base, spin_limit, &timed_out);
-			if (r == 0)
-				break;
-			o.base += r;
-		}
-		if (timed_out && !o.mine)
-			flag_err(err, KMA_ERR_TIMEOUT);
-		return reinterpret_cast<kma_clqueue_item *>(o.mine);
-	}
 	return reinterpret_cast<kma_clqueue_item *>(
 		kma_detail::clq_dequeue<kma_detail::clq_link_head>(q, err, spin_limit));
 }
@@ -892,27 +840,11 @@ __device__ inline int kma_iqueue_enqueue_shard(kma_iqueue *q, void *item, uint32
 
 /* idxd_dequeue (clIndexedQueue.cl:203-247) on one shard: the old dummy
  * (an item pointer), NULL when only the dummy is left or on spin-limit
- * expiry.  An internal dummy leaving the shard is skipped.  Lanes that call
- * it together on one shard take theirs together (see kma_clqueue_dequeue). */
+ * expiry.  An internal dummy leaving the shard is skipped. */
 __device__ inline void *kma_iqueue_dequeue_shard(kma_iqueue *q, uint32_t shard)
 {
 	using namespace kma_detail;
 	const iq_links L(q);
-	const gpu_some_lanes v = {__activemask()};
-	if (v.size() > 1 && v.share(shard) && v.share((unsigned long long)q)) {
-		lanes_out_rank<uint32_t> o = {0u, L.capacity, v.rank(), 0u};
-		for (uint32_t turn = 0; o.base < v.size() && turn < 33; turn++) {
-			bool timed_out = false;
-			const uint32_t r = kma_q::iq_walk_v<gpu_ops_group>(v, L, &q->ends[2 * shard].v, o, v.size() - o.base,
-									   q->spin_limit, &timed_out);
-			if (timed_out)
-				atomicOr(&q->err, KMA_ERR_TIMEOUT);
-			if (r == 0)
-				break;
-			o.base += r; /* (less the internal dummies it has met) */
-		}
-		return o.mine ? kma_iqueue_item(q, o.mine) : nullptr;
-	}
 	for (uint32_t k = 0; k < 2; k++) {
 		uint32_t idx = 0;
 		bool timed_out = false;

@@ -45,9 +45,7 @@
  * batches meet whole logged chains and take several per hold; LANES 1
  * dequeues with the warp's text (clq_dequeue_v), its 32 lanes as arrays:
  * LANES 2 every other batch, so that both texts meet on one queue.  (Indexed
- * queue: LANES takes one item at a time, with iq_dequeue_1.)  LANES 3: with
- * the text of lanes that call a per-thread dequeue together (clq_walk_v,
- * iq_walk_v), LANES 4 every third batch, beside the other two.  Prints one
+ * queue: LANES takes one item at a time, with iq_dequeue_1.)  Prints one
  * JSON line (with the chains taken from records and the dequeue calls
  * that took items); exits 0 when every check passed.  The reference's own
  * queues are the parity oracle (serial replays against tests/golden);
@@ -288,23 +286,8 @@ struct HostOut {
 			f(a[i]);
 	}
 };
-struct HostIdx {
-	uint32_t *a;
-	void one(uint32_t at, uint32_t item) { a[at] = item; }
-};
-/* the text of the dequeues (LANES): of this batch, 0 one thread's, 1 the
- * warp's, 2 that of lanes without a log */
+/* dequeue with the warp's text: 0 never, 1 always, 2 every other batch */
 int g_lanes = 0;
-int text_of_batch()
-{
-	switch (g_lanes) {
-	case 0: return 0;
-	case 1: return 1;
-	case 2: return (int)(rnd() & 1);
-	case 3: return 2;
-	default: return (int)(rnd() % 3);
-	}
-}
 
 HostLog g_log;
 const HostLog *log_ptr() { return g_log.mask || !g_log.clq.empty() || !g_log.iq.empty() ? &g_log : nullptr; }
@@ -414,11 +397,8 @@ void run_clq(int threads, int chains, int maxc, int batch, double recycle, uint6
 			bool to = false;
 			uint32_t k = g_fixed_batch ? (uint32_t)batch : 1 + (uint32_t)(rnd() % batch);
 			HostOut ho = {out.data()};
-			const int text = text_of_batch();
-			uint32_t r = text == 1
+			uint32_t r = g_lanes == 1 || (g_lanes == 2 && (rnd() & 1))
 				? kma_q::clq_dequeue_v<HostOps, LinkAtItem, HostLanes>(&q[0], &q[1], ho, k, LIMIT, &to, log_ptr())
-				: text == 2
-				? kma_q::clq_walk_v<HostOps, LinkAtItem>(HostLanes{}, &q[0], &q[1], ho, k, LIMIT, &to)
 				: kma_q::clq_dequeue_n<HostOps, LinkAtItem>(&q[0], &q[1], out.data(), k, LIMIT, &to, log_ptr());
 			if (to)
 				bk.tmo++;
@@ -540,12 +520,8 @@ void run_iq(int threads, int chains, int maxc, int batch, double recycle, uint64
 			bool done = producing.load() == 0;
 			bool to = false;
 			uint32_t k = g_fixed_batch ? (uint32_t)batch : 1 + (uint32_t)(rnd() % batch);
-			const int text = text_of_batch();
-			HostIdx ho = {out.data()};
-			uint32_t r = text == 1
+			uint32_t r = g_lanes == 1 || (g_lanes == 2 && (rnd() & 1))
 				? kma_q::iq_dequeue_1<HostOps>(q, &ends[0], out.data(), LIMIT, &to)
-				: text == 2
-				? kma_q::iq_walk_v<HostOps>(HostLanes{}, q, &ends[0], ho, k, LIMIT, &to)
 				: kma_q::iq_dequeue_n<HostOps>(q, &ends[0], out.data(), k, LIMIT, &to, log_ptr());
 			if (to)
 				bk.tmo++;
@@ -662,27 +638,6 @@ int run_stuck()
 		uint32_t out[1];
 		bool to = false;
 		ok &= kma_q::iq_dequeue_1<HostOps>(iq, &ends[0], out, limit, &to) == 0 && to && ends[0] == kma_q::tw_make(1, 1);
-	}
-	for (int state = 0; state < 2; state++) { /* and with that of lanes without a log */
-		Item a{}, b{};
-		u64 q[2] = {(u64)&a, (u64)&b};
-		a.next = state == 0 ? kma_q::POISON : 0ull;
-		u64 buf[4];
-		HostOut out = {buf};
-		bool to = false;
-		uint32_t r = kma_q::clq_walk_v<HostOps, LinkAtItem>(HostLanes{}, &q[0], &q[1], out, 4, limit, &to);
-		ok &= r == 0 && to && a.next == (state == 0 ? kma_q::POISON : 0ull) && q[0] == (u64)&a;
-	}
-	{
-		std::vector<u64> links(4, 0);
-		IdxQ iq{&links};
-		links[1] = kma_q::tw_make(0, 2);
-		u64 ends[2] = {kma_q::tw_make(1, 1), kma_q::tw_make(0, 2)};
-		uint32_t buf[4];
-		HostIdx out = {buf};
-		bool to = false;
-		ok &= kma_q::iq_walk_v<HostOps>(HostLanes{}, iq, &ends[0], out, 4, limit, &to) == 0 && to &&
-		      ends[0] == kma_q::tw_make(1, 1);
 	}
 	printf("{\"stuck_ok\": %s}\n", ok ? "true" : "false");
 	return ok ? 0 : 1;
