@@ -459,9 +459,17 @@ __global__ void k_gr_export(gr_dev<B> g, uint64_t nodes, uint32_t *keys, long lo
 template <class B>
 __global__ void k_gr_free(gr_dev<B> g, uint64_t nodes, uint64_t n)
 {
-	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-	for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n + nodes; i += stride)
-		B::release_warp(g.h, i < n ? reinterpret_cast<void *>(g.link[i]) : g.reg[i - n]);
+	if constexpr (B::id == KMA_BACKEND_ID_KMA) {
+		const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+		/* all lanes of a warp call every time, together */
+		for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n + nodes; base += stride) {
+			const uint64_t i = base + threadIdx.x;
+			void *b = B::block(g.h, i < n ? reinterpret_cast<void *>(g.link[i])
+						      : i < n + nodes ? g.reg[i - n] : nullptr);
+			__syncwarp();
+			B::free_block_warp(g.h, b);
+		}
+	}
 }
 
 } /* namespace */
